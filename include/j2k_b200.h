@@ -76,18 +76,18 @@ enum {
                                  levels; 2, 3, 4, 5: from the first level with at most 96, 32, 96, 320
                                  tiles per plane, one thread-block cluster of 16, 16, 8, 16 CTAs per
                                  plane with the cluster barrier between levels.  0 (default): off */
-    J2K_TUNE_T1D_LANES = 10,  /* tier-1 decoder: code-blocks decoded side by side in one warp, one per lane
-                                 (2, 4 default, 8, 16, 32); 0: one warp per block, lane 0 decoding */
+    J2K_TUNE_T1D_LANES = 10,  /* tier-1 decoder: code-blocks decoded side by side in one warp, one per lane:
+                                 0 (one), 2, 4, 8, 16; 3, 6 and 32 run as 4, 8 and 16.  Left alone, it is 1,
+                                 2 or 4 by the number of blocks */
     J2K_TUNE_T1D_STEPS = 11,  /* 1: with 8, 16 or 32 lanes, unstyled blocks are decoded in a loop of one
-                                 symbol per step (one MQ decoding site); 0 (default): in the pass /
-                                 stripe / column loops */
+                                 symbol per step over 64-bit row masks; 0 (default): stripe by stripe */
     J2K_TUNE_PLANAR = 12,     /* interleaved-to-planar split of contiguous images: 0: 16 pixels per thread;
                                  1 (default) / 2: 4 pixels per thread and step, a warp's stores contiguous,
                                  4 / 8 steps per thread with all their loads issued first */
     J2K_TUNE_DWT97_ROWS = 13, /* differentiable 9/7 (j2k_dwt97_*): 1 (default) runs every level whose width is
                                  a power of two in 64..1024 as bands of 16 full rows (a warp per row in
                                  registers, no halo columns); 0: the 248 x 16 strip kernels */
-    J2K_TUNE_T1D_ORDER = 14,  /* tier-1 decoder with blocks side by side in a warp: 1 (default) gives the
+    J2K_TUNE_T1D_ORDER = 14,  /* tier-1 decoder: 1 (default) gives the
                                  warps their blocks sorted by codeword length, longest first (the blocks
                                  of a warp then take about as long); 0: list order */
     J2K_TUNE_DWT_PX = 15,     /* encoder of interleaved 8-bit pixels (j2k_encoder_run_interleaved), 1 or 3

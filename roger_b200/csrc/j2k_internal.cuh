@@ -59,7 +59,7 @@ enum : uint32_t {
     J2K_DEVERR_SEG_CAPACITY = 6,  // a coding-pass segment outgrew its slot (code-block styles)
 };
 
-constexpr int J2K_SCRATCH_SLOTS = 15;
+constexpr int J2K_SCRATCH_SLOTS = 16;
 
 constexpr int J2K_MQ_TIERS = 4;
 
@@ -86,7 +86,7 @@ struct j2k_ctx {
     int dwt_tma = 0;             // fast forward DWT: strips staged by TMA tensor copies (persistent CTAs)
     int t1a_ctas = 2;            // tier-1 phase A: resident CTAs per SM its registers are cut for (2 or 3)
     int dwt_tail = 0;            // forward DWT: deep levels in one launch (1 cooperative, 2..5 clusters)
-    int t1d_lanes = 4;           // tier-1 decoder: code-blocks per warp (2, 4, 8, 16, 32), 0 = one warp per block
+    int t1d_lanes = -1;          // tier-1 decoder: code-blocks per warp (0: one), -1: by the number of blocks
     int t1d_steps = 0;           // tier-1 decoder: unstyled blocks by the one-symbol-per-step loop
     int planar_form = 1;         // planar split: 0 16 pixels per thread; 1 / 2: 4 pixels per thread and step
     int dwt97_rows = 1;          // differentiable 9/7: levels 64..1024 wide (powers of two) as full-row bands
@@ -97,7 +97,7 @@ struct j2k_ctx {
 // scratch slot ids
 enum { SCR_LL0 = 0, SCR_LL1 = 1, SCR_JOBS = 2, SCR_SYMS = 3, SCR_T1STATE = 4, SCR_MISC = 5,
        SCR_PLANES = 6, SCR_MISC2 = 7, SCR_RES = 8, SCR_UNITS = 9, SCR_SEGS = 10, SCR_BARRIER = 11,
-       SCR_PLANE = 12, SCR_DECORD = 13, SCR_LLPX = 14 };
+       SCR_PLANE = 12, SCR_DECORD = 13, SCR_LLPX = 14, SCR_DECQ = 15 };
 
 j2k_status j2k_fail(j2k_ctx* ctx, j2k_status s, const std::string& msg);
 j2k_status j2k_cuda_check(j2k_ctx* ctx, cudaError_t e, const char* what);

@@ -2,15 +2,15 @@
 //
 // The reference has no decoder for this stage (src/OCLDecoder.cpp:35-38 runs only the "reverse"
 // DWT).  Decoding is serial per code-block: every context depends on the bits decoded before it.
-// The default kernel runs one code-block per LANE: a warp decodes 8, 16 or 32 blocks side by side,
-// each lane with its own MQ registers and its own 64-bit row masks of significance / sign /
-// refined / visited in shared memory (interleaved by lane, so that the warp's accesses to any rows
-// fall in distinct banks).  Lanes that take the same branch of the pass / stripe / column loops
-// issue together; the decoder is bound by the latency of each decision's dependent chain, not by
-// instruction issue, so a warp instruction that serves many blocks is what makes it fast.  The
-// warp clears its blocks' output regions first and applies the signs at the end, cooperatively;
-// magnitude bits go to the output plane by fire-and-forget atomic ORs (each block owns its region).
-// The older form, one warp per block with lane 0 decoding, stays as a tuning choice.
+// The kernel runs one code-block per lane, 1, 2 or 4 (8, 16 by tuning) in a warp, and takes all
+// work that is not a block's own serial chain out of the lanes' loops (t1dec_stripe.cuh).  What
+// bounds it: the chain of dependent instructions per symbol (about 95 warp instructions and 430
+// cycles a symbol with one block per warp), and with 4 blocks per warp instruction issue, since
+// the lanes are at different kinds of symbols.  Round trips host to host on B200, against a decoder
+// whose lanes kept 64-bit row masks and gathered each column's neighbourhood themselves: 512 x 512
+// gray 15.3 -> 6.5 ms, 2048 x 2048 colour 18.8 -> 12.9 ms, 4096 x 4096 colour 28.2 -> 22.5 ms.
+// The warp clears its blocks' output regions first and applies the signs at the end; magnitude bits
+// go to the output plane by fire-and-forget atomic ORs (each block owns its region).
 #include <atomic>
 
 #include <cub/cub.cuh>
@@ -18,8 +18,6 @@
 #include "j2k_internal.cuh"
 
 namespace {
-
-constexpr int kWarps = 4;
 
 // T.800 Table C.2 (probability estimation), device and host copies
 __constant__ uint16_t d_qe[47] = {
@@ -269,237 +267,7 @@ struct RawD {
     }
 };
 
-// Serial decode of one code-block into magnitudes (blk, pre-zeroed) and sign/state masks in S
-// (a DecSmem, or a LaneState of a block decoded beside others in the same warp).  Host-callable
-// so that the exact device logic can be checked on the CPU.  STYLED: the block was coded with
-// code-block style `style` (contexts reset per pass, a new codeword segment after every
-// terminated pass, located by the pass ends `pe`; raw-coded passes read as bits).  RED: magnitude
-// bits are set by atomic ORs whose result is not read (device only).
-template <bool STYLED = false, bool RED = false, class State>
-__host__ __device__ void decode_block(State& S, const DecTables& T, const uint8_t* data, int len, int numbps,
-                                      int npasses, int orient, int cw, int ch, int32_t* blk, size_t pitch,
-                                      int style = 0, const uint32_t* pe = nullptr) {
-        const uint8_t* zct = T.zc[orient];
-        const uint32_t* mq = T.mq;
-
-        auto reset_states = [&]() {
-            for (int k = 0; k < 19; ++k) S.st(k) = 0;
-            S.st(0) = 4 << 1;
-            S.st(17) = 3 << 1;
-            S.st(18) = 46 << 1;
-        };
-        reset_states();
-        Mqd m;
-        RawD rd;
-        bool raw = false;
-        if (!STYLED) m.init(data, len);
-        // the start of pass q of a styled block: context reset, and a new segment after a
-        // terminated pass
-        auto begin = [&](int q) {
-            if (!STYLED) return;
-            if (q > 0 && (style & J2K_CBLK_RESET)) reset_states();
-            raw = j2k_pass_raw(style, q);
-            if (q == 0 || j2k_pass_terminated(style, q - 1, npasses)) {
-                int e = q;
-                while (!j2k_pass_terminated(style, e, npasses)) ++e;
-                int b0 = q ? (int)min(pe[q - 1], (uint32_t)len) : 0;
-                int b1 = (int)min(pe[e], (uint32_t)len);
-                if (b1 < b0) b1 = b0;
-                if (raw) rd.init(data + b0, b1 - b0);
-                else m.init(data + b0, b1 - b0);
-            }
-        };
-        // one decision in context cx, and one sign in sign context sc (label | xor << 7)
-        auto dec = [&](int cx) -> int {
-            if (STYLED && raw) return rd.bit();
-            return m.decode(S.st(cx), mq);
-        };
-        auto dsign = [&](int sc) -> int {
-            if (STYLED && raw) return rd.bit();
-            return m.decode(S.st(sc & 31), mq) ^ (sc >> 7);
-        };
-        int pass = 0;
-        const int nb = numbps, np = npasses;
-        // a stripe column's neighbourhood, packed: bits 3r..3r+2 hold columns x-1..x+1 of block row
-        // y0-1+r (r = 0..5), from the significance (or sign) rows; stripe row k's 9-bit
-        // neighbourhood is then (W >> 3k) & 511 and its own bit 3k+4
-        auto colw = [&](int y0, int x) -> uint32_t {
-            uint32_t w = 0;
-#ifdef __CUDA_ARCH__
-            if (x > 0) {  // bits x-1..x+1 of each row: one funnel shift of its two halves
-                const int s5 = (x - 1) & 31;
-                const bool hiw = x - 1 >= 32;
-                for (int r = 0; r < 6; ++r) {
-                    const uint64_t m = S.sig(y0 + r);
-                    const uint32_t lo = (uint32_t)m, hi = (uint32_t)(m >> 32);
-                    const uint32_t t = hiw ? (hi >> s5) : __funnelshift_r(lo, hi, s5);
-                    w |= (t & 7u) << (3 * r);
-                }
-                return w;
-            }
-#endif
-            for (int r = 0; r < 6; ++r) w |= nb3(S.sig(y0 + r), x) << (3 * r);
-            return w;
-        };
-        // the sign bits sign_nbhd reads for stripe row k of column x (left and right in its row,
-        // above and below), from the sign rows as they are now
-        auto negnb = [&](int y0, int x, int k) -> uint32_t {
-            const uint64_t nu = S.neg(y0 + k), no = S.neg(y0 + k + 1), nd = S.neg(y0 + k + 2);
-            const uint32_t l = x > 0 ? (uint32_t)(no >> (x - 1)) & 1u : 0u;
-            const uint32_t r = x < 63 ? (uint32_t)(no >> (x + 1)) & 1u : 0u;
-            return (((uint32_t)(nu >> x) & 1u) << (3 * k + 1)) | (l << (3 * k + 3)) | (r << (3 * k + 5)) |
-                   (((uint32_t)(nd >> x) & 1u) << (3 * k + 7));
-        };
-        auto add_bit = [&](int x, int y, int p) {
-#ifdef __CUDA_ARCH__
-            if (RED) {
-                atomicOr(reinterpret_cast<unsigned int*>(blk + (size_t)y * pitch + x), 1u << p);
-                return;
-            }
-#endif
-            blk[(size_t)y * pitch + x] |= 1 << p;
-        };
-        auto n8of = [](uint32_t W, uint32_t NW, int k) { return sign_nbhd(W, NW, k); };
-        auto set_sig = [&](int x, int y, int neg, int p) {
-            S.sig(y + 1) |= 1ull << x;
-            if (neg) S.neg(y + 1) |= 1ull << x;
-            add_bit(x, y, p);
-        };
-        const uint64_t cols = cw >= 64 ? ~0ull : ((1ull << cw) - 1);
-        for (int p = nb - 1; p >= 0 && pass < np; --p) {
-            if (p != nb - 1) {
-                // significance propagation: only columns next to a significant sample can hold a
-                // decision; a column joins when its left neighbour gains a significant sample
-                begin(pass);
-                for (int y0 = 0; y0 < ch; y0 += 4) {
-                    const int ny = min(4, ch - y0);
-                    uint64_t cm = 0;
-                    for (int y = y0; y < y0 + ny; ++y) {
-                        const uint64_t own = S.sig(y + 1);
-                        uint64_t nbm = S.sig(y) | own | S.sig(y + 2);
-                        nbm |= (nbm << 1) | (nbm >> 1);
-                        cm |= ~own & nbm;
-                    }
-                    cm &= cols;
-                    uint64_t vacc[4] = {0, 0, 0, 0};  // this stripe's visits, stored once at its end
-                    while (cm) {
-                        const int x = ctz64(cm);
-                        cm &= cm - 1;
-                        uint32_t W = colw(y0, x), vb = 0;
-                        for (int k = 0; k < ny; ++k) {  // one decoding site: not unrolled
-                            if ((W >> (3 * k + 4)) & 1) continue;  // significant already
-                            const uint32_t n9 = (W >> (3 * k)) & 511;
-                            if (!(n9 & 0x1EF)) continue;           // no significant neighbour
-                            const int bit = dec(zct[n9]);
-                            vb |= 1u << k;
-                            if (bit) {
-                                const int sc = T.sc[n8of(W, negnb(y0, x, k), k)];
-                                const int sg = dsign(sc);
-                                set_sig(x, y0 + k, sg, p);
-                                W |= 1u << (3 * k + 4);
-                                cm |= (2ull << x) & cols;
-                            }
-                        }
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) vacc[k] |= (uint64_t)((vb >> k) & 1) << x;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < ny) S.vis(y0 + k + 1) |= vacc[k];
-                }
-                if (++pass >= np) break;
-                // magnitude refinement: significant samples not visited in this plane
-                begin(pass);
-                for (int y0 = 0; y0 < ch; y0 += 4) {
-                    const int ny = min(4, ch - y0);
-                    // per stripe row k, as masks over the columns (this pass changes none of
-                    // them): the samples to refine (significant, not visited in this plane), the
-                    // ones refined before (label 16), and the ones with a significant neighbour
-                    // (label 15, else 14)
-                    uint64_t mr[4] = {0, 0, 0, 0}, rf[4] = {0, 0, 0, 0}, nbs[4] = {0, 0, 0, 0};
-                    uint64_t rm = 0;
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        if (k >= ny) break;
-                        const uint64_t own = S.sig(y0 + k + 1), v3 = S.sig(y0 + k) | S.sig(y0 + k + 2);
-                        mr[k] = own & ~S.vis(y0 + k + 1) & cols;
-                        rf[k] = S.ref(y0 + k + 1);
-                        nbs[k] = v3 | (v3 << 1) | (v3 >> 1) | (own << 1) | (own >> 1);
-                        rm |= mr[k];
-                    }
-                    while (rm) {
-                        const int x = ctz64(rm);
-                        rm &= rm - 1;
-                        uint32_t mb = 0, rb = 0, nbb = 0;  // the column's rows, as 4-bit masks
-#pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            mb |= (uint32_t)((mr[k] >> x) & 1) << k;
-                            rb |= (uint32_t)((rf[k] >> x) & 1) << k;
-                            nbb |= (uint32_t)((nbs[k] >> x) & 1) << k;
-                        }
-                        while (mb) {  // one decoding site
-                            const int k = ctz64(mb);
-                            mb &= mb - 1;
-                            const int lab = ((rb >> k) & 1) ? 16 : (((nbb >> k) & 1) ? 15 : 14);
-                            if (dec(lab)) add_bit(x, y0 + k, p);
-                        }
-                    }
-                    // every sample of mr was refined in this pass
-#pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        if (k < ny) S.ref(y0 + k + 1) = rf[k] | mr[k];
-                }
-                if (++pass >= np) break;
-            }
-            // cleanup: every insignificant sample not visited in this plane
-            begin(pass);
-            for (int y0 = 0; y0 < ch; y0 += 4) {
-                const int ny = min(4, ch - y0);
-                // per stripe row k: the samples this pass codes (insignificant, not visited in
-                // this plane); a sample that becomes significant here is the one being coded, so
-                // the masks hold for the whole pass
-                uint64_t un[4] = {0, 0, 0, 0};
-                uint64_t um = 0;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    if (k >= ny) break;
-                    un[k] = ~S.sig(y0 + k + 1) & ~S.vis(y0 + k + 1) & cols;
-                    um |= un[k];
-                }
-                while (um) {
-                    const int x = ctz64(um);
-                    um &= um - 1;
-                    uint32_t W = colw(y0, x), U = 0;  // U: rows of the column to code
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) U |= (uint32_t)((un[k] >> x) & 1) << k;
-                    int start = 0;
-                    if (ny == 4 && W == 0 && U == 15) {
-                        // run-length mode: four insignificant, unvisited samples, no significant
-                        // neighbour (every bit of the column's neighbourhood is zero)
-                        if (!dec(17)) continue;
-                        int idx = dec(18) << 1;
-                        idx |= dec(18);
-                        const int sc = T.sc[0];
-                        const int sg = dsign(sc);
-                        set_sig(x, y0 + idx, sg, p);
-                        W |= 1u << (3 * idx + 4);
-                        start = idx + 1;
-                    }
-                    for (int k = start; k < ny; ++k) {
-                        if (!((U >> k) & 1)) continue;
-                        if (dec(zct[(W >> (3 * k)) & 511])) {
-                            const int sc = T.sc[n8of(W, negnb(y0, x, k), k)];
-                            const int sg = dsign(sc);
-                            set_sig(x, y0 + k, sg, p);
-                            W |= 1u << (3 * k + 4);
-                        }
-                    }
-                }
-            }
-            ++pass;
-            for (int r = 0; r < 66; ++r) S.vis(r) = 0;
-        }
-}
+#include "t1dec_stripe.cuh"
 
 // the checks a decoder kernel makes of a job before touching its region
 __device__ __forceinline__ bool dec_job_ok(const j2k_cb_job& J, const j2k_cb_desc& D, bool styled) {
@@ -517,50 +285,146 @@ __host__ __device__ __forceinline__ int32_t cut_half(int numbps, int npasses) {
     return 0;
 }
 
-template <bool STYLED>
-__global__ void __launch_bounds__(kWarps * 32)
-t1_decode_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __restrict__ bytes,
-                 const j2k_cb_job* __restrict__ jobs, int njobs, int32_t* __restrict__ coeff,
-                 uint32_t* __restrict__ err, int style, const uint32_t* __restrict__ pass_ends,
-                 const uint8_t* __restrict__ job_style) {
-    __shared__ DecSmem smem[kWarps];
-    __shared__ DecTables tabs;
-    for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) fill_tables_entry(tabs, i);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int jid = blockIdx.x * kWarps + wid;
-    if (jid >= njobs) return;
-    DecSmem& S = smem[wid];
-    const j2k_cb_job J = jobs[jid];
-    const j2k_cb_desc D = descs[jid];
-    const int cw = J.cw, ch = J.ch, orient = J.orient;
-    // (a styled block's passes index its pass ends: at most 3 * 31 - 2 of them)
-    if (!dec_job_ok(J, D, STYLED)) {
-        if (lane == 0) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_BAD_JOB);
-        return;
-    }
-    const size_t pitch = J.pitch;
-    int32_t* blk = coeff + J.off;
-    for (int r = 0; r < ch; ++r)
-        for (int x = lane; x < cw; x += 32) blk[(size_t)r * pitch + x] = 0;
-    for (int r = lane; r < 66; r += 32) { S.sig_[r] = 0; S.neg_[r] = 0; S.ref_[r] = 0; S.vis_[r] = 0; }
-    if (lane < 19) S.st_[lane] = 0;
-    __syncwarp();
-    if (lane == 0 && D.numbps > 0 && D.npasses > 0)
-        decode_block<STYLED>(S, tabs, bytes + D.offset, D.length, D.numbps, D.npasses, orient, cw, ch, blk, pitch,
-                             job_style ? (int)job_style[jid] : style,
-                             STYLED ? pass_ends + (size_t)jid * J2K_PASS_STRIDE : nullptr);
-    __syncwarp();
-    const int32_t half = cut_half(D.numbps, D.npasses);
-    for (int r = 0; r < ch; ++r)
-        for (int x = lane; x < cw; x += 32) {
-            int32_t v = blk[(size_t)r * pitch + x];
-            if ((S.sig_[r + 1] >> x) & 1) v += half;
-            if ((S.neg_[r + 1] >> x) & 1) v = -v;
-            blk[(size_t)r * pitch + x] = v;
-        }
+// Warps per CTA of the stripe decoder: with 4 or 8 blocks per warp one CTA's state fills an SM's
+// shared memory (84 or 88 blocks; the 12288 blocks of a 4096 x 4096 colour image are then resident
+// at once on 148 SMs).
+template <int L>
+__host__ __device__ constexpr int stripe_warps() {
+    return L == 1 ? 16 : (L == 2 ? 20 : (L == 4 ? 21 : (L == 8 ? 11 : 5)));
+}
+constexpr size_t kStripeTablesBytes = (sizeof(StripeTables) + 15) & ~(size_t)15;
+template <int L>
+__host__ __device__ constexpr size_t stripe_smem_bytes(int warps) {
+    return kStripeTablesBytes + (size_t)warps * stripe_state_words<L>() * 4;
 }
 
+// L code-blocks per warp, one per lane (t1dec_stripe.cuh).  Groups of L consecutive blocks of
+// `order` (longest codewords first) go to the warps of all CTAs in turn, then from a queue.
+template <bool STYLED, int L>
+__global__ void __launch_bounds__(32 * stripe_warps<L>(), 1)
+t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __restrict__ bytes,
+                        const j2k_cb_job* __restrict__ jobs, int njobs, int32_t* __restrict__ coeff,
+                        uint32_t* __restrict__ err, int style, const uint32_t* __restrict__ pass_ends,
+                        const uint8_t* __restrict__ job_style, const uint32_t* __restrict__ order,
+                        uint32_t* __restrict__ queue) {
+    extern __shared__ __align__(16) uint8_t dsm[];
+    StripeTables& tabs = *reinterpret_cast<StripeTables*>(dsm);
+    for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) fill_stripe_tables_entry(tabs, i);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const StripeState<L> S{reinterpret_cast<uint32_t*>(dsm + kStripeTablesBytes) + wid * stripe_state_words<L>()};
+    constexpr int R = (8 * L + 31) / 32;  // rounds of 32 (block, word) items per stripe
+    const int ngroups = (njobs + L - 1) / L;
+    for (int g = wid * (int)gridDim.x + (int)blockIdx.x; g < ngroups;) {
+        const int j0 = g * L, nb = min(L, njobs - j0);
+        j2k_cb_job J{};
+        j2k_cb_desc D{};
+        bool ok = false;
+        const int jid = lane < nb ? (order ? (int)order[j0 + lane] : j0 + lane) : 0;
+        if (lane < nb) {
+            J = jobs[jid];
+            D = descs[jid];
+            ok = dec_job_ok(J, D, STYLED);
+            if (!ok) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_BAD_JOB);
+        }
+        const unsigned okmask = __ballot_sync(~0u, ok);
+        for (int i = lane; i < kStripeBitmapWords * L; i += 32) S.w[i] = 0;
+        for (int b = 0; b < nb; ++b) {
+            if (!((okmask >> b) & 1)) continue;
+            const int cw = __shfl_sync(~0u, (int)J.cw, b), ch = __shfl_sync(~0u, (int)J.ch, b);
+            const size_t pitch = __shfl_sync(~0u, J.pitch, b);
+            int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
+            for (int r = 0; r < ch; ++r)
+                for (int x = lane; x < cw; x += 32) blk[(size_t)r * pitch + x] = 0;
+        }
+        // this lane's block, and the sizes and pass counts of the blocks of its items
+        const int np = ok && D.numbps > 0 ? min((int)D.npasses, 3 * (int)D.numbps - 2) : 0;
+        StripeLane<L> me{S, &tabs, tabs.zc[J.orient & 3], lane, J.cw, J.ch, {}, {}, false};
+        int icw[R], ich[R], inp[R], inb[R];
+        uint32_t ipitch[R];
+        int32_t* iblk[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = lane + 32 * r, b = (i >> 3) & 31;
+            icw[r] = __shfl_sync(~0u, (int)J.cw, b);
+            ich[r] = __shfl_sync(~0u, (int)J.ch, b);
+            inp[r] = __shfl_sync(~0u, np, b);
+            inb[r] = __shfl_sync(~0u, (int)D.numbps, b);
+            ipitch[r] = __shfl_sync(~0u, J.pitch, b);
+            iblk[r] = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
+            if (i >= 8 * L) inp[r] = 0;
+        }
+        const int pmax = __reduce_max_sync(~0u, np > 0 ? (int)D.numbps : 0);
+        const int smax = (__reduce_max_sync(~0u, np > 0 ? (int)J.ch : 0) + 3) >> 2;
+        const int st = STYLED ? (job_style ? (int)job_style[jid] : style) : 0;
+        __syncwarp();
+        // t = 3 * bit-plane + 2, 1, 0 for its three passes: the blocks of a warp code the same
+        // plane at the same time (their lowest planes, which hold most symbols, are alike; counted
+        // from the first pass they would be apart by the difference of their plane counts)
+        for (int t = 3 * pmax - 1; t >= 0; --t) {
+            const int p = t / 3, kind = kPassCU - t % 3;
+            auto pass_of = [&](int numbps) { return 3 * (numbps - 1 - p) - t % 3; };  // its number in the block
+            const int q = pass_of(D.numbps);
+            const bool on = q >= 0 && q < np;
+            if (on)
+                me.template begin<STYLED>(q, D.npasses, bytes + D.offset, D.length, st,
+                                          STYLED ? pass_ends + (size_t)jid * J2K_PASS_STRIDE : nullptr);
+            bool ion[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) ion[r] = pass_of(inb[r]) >= 0 && pass_of(inb[r]) < inp[r];
+            for (int s = 0; s < smax; ++s) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int i = lane + 32 * r;
+                    if (ion[r] && 4 * s < ich[r]) {
+                        if (kind == kPassMR) stripe_prepare_mr<L>(S, s, i & 7, i >> 3, icw[r]);
+                        else stripe_prepare_zc<L>(S, kind, s, i & 7, i >> 3, icw[r], stripe_rows(ich[r], s));
+                    }
+                }
+                __syncwarp();
+                if (on && 4 * s < me.ch) {
+                    const uint32_t rv = stripe_rows(me.ch, s);
+                    if (kind == kPassSP) me.template decode_zc<STYLED, kPassSP>(rv);
+                    else if (kind == kPassMR) me.template decode_mr<STYLED>();
+                    else me.template decode_zc<STYLED, kPassCU>(rv);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int i = lane + 32 * r;
+                    if (ion[r] && 4 * s < ich[r]) {
+                        const uint32_t ones = kind == kPassMR
+                                                  ? stripe_finish_mr<L>(S, s, i & 7, i >> 3, icw[r])
+                                                  : stripe_finish_zc<L>(S, kind, s, i & 7, i >> 3, icw[r]);
+                        stripe_add_bits(ones, iblk[r], ipitch[r], s, i & 7, p);
+                    }
+                }
+                __syncwarp();
+            }
+        }
+        // signs, and the middle of the undecoded interval of a cut block
+        const int32_t my_half = ok ? cut_half(D.numbps, D.npasses) : 0;
+        for (int b = 0; b < nb; ++b) {
+            if (!((okmask >> b) & 1)) continue;
+            const int cw = __shfl_sync(~0u, (int)J.cw, b), ch = __shfl_sync(~0u, (int)J.ch, b);
+            const size_t pitch = __shfl_sync(~0u, J.pitch, b);
+            int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
+            const int32_t half = __shfl_sync(~0u, my_half, b);
+            for (int r = 0; r < ch; ++r)
+                for (int x = lane; x < cw; x += 32) {
+                    const int sh = 4 * (x & 7) + (r & 3);
+                    int32_t v = __ldcg(blk + (size_t)r * pitch + x);
+                    if ((S.sig(r >> 2, x >> 3, b) >> sh) & 1) v += half;
+                    if ((S.neg(r >> 2, x >> 3, b) >> sh) & 1) v = -v;
+                    blk[(size_t)r * pitch + x] = v;
+                }
+        }
+        __syncwarp();
+        int nx = 0;
+        if (lane == 0) nx = (int)(gridDim.x * (blockDim.x >> 5) + atomicAdd(queue, 1u));
+        g = __shfl_sync(~0u, nx, 0);
+    }
+}
 
 constexpr size_t kTablesBytes = (sizeof(DecTables) + 15) & ~(size_t)15;
 // warps per CTA of the lane-per-block decoders for L blocks per warp: 32 blocks per CTA for
@@ -575,80 +439,8 @@ __host__ __device__ constexpr size_t lanes_smem_bytes() {
     return kTablesBytes + (size_t)cta_warps<L>() * lane_state_bytes<L>();
 }
 
-// One code-block per lane: a CTA takes 32 consecutive jobs (of `order` when given: the jobs
-// sorted by codeword length, longest first, so that the blocks sharing a warp take about as long
-// and the longest start first) in 32 / L warps of L (lanes 0..L-1 of a warp decode, one block each); every lane of the warp helps clear its blocks' regions first
-// and apply the signs at the end.  Dynamic shared memory: the tables, then each warp's
-// LaneState<L> area.
-template <bool STYLED, int L>
-__global__ void __launch_bounds__(32 * cta_warps<L>())
-t1_decode_lanes_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __restrict__ bytes,
-                       const j2k_cb_job* __restrict__ jobs, int njobs, int32_t* __restrict__ coeff,
-                       uint32_t* __restrict__ err, int style, const uint32_t* __restrict__ pass_ends,
-                       const uint8_t* __restrict__ job_style, const uint32_t* __restrict__ order) {
-    extern __shared__ __align__(16) uint8_t dsm[];
-    DecTables& tabs = *reinterpret_cast<DecTables*>(dsm);
-    for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) fill_tables_entry(tabs, i);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int j0 = (blockIdx.x * cta_warps<L>() + wid) * L;
-    if (j0 >= njobs) return;
-    const int nb = min(L, njobs - j0);
-    uint8_t* wsm = dsm + kTablesBytes + (size_t)wid * lane_state_bytes<L>();
-    uint64_t* base = reinterpret_cast<uint64_t*>(wsm);
-    uint8_t* stb = wsm + (size_t)4 * 66 * L * 8;
-    j2k_cb_job J{};
-    j2k_cb_desc D{};
-    bool ok = false;
-    // this lane's job: position j0 + lane of the order (longest codewords first), or of the list
-    const int jid = lane < nb ? (order ? (int)order[j0 + lane] : j0 + lane) : 0;
-    if (lane < nb) {
-        J = jobs[jid];
-        D = descs[jid];
-        ok = dec_job_ok(J, D, STYLED);
-        if (!ok) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_BAD_JOB);
-    }
-    const unsigned okmask = __ballot_sync(~0u, ok);
-    for (int i = lane; i < 4 * 66 * L; i += 32) base[i] = 0;
-    for (int b = 0; b < nb; ++b) {
-        if (!((okmask >> b) & 1)) continue;
-        const int cw = __shfl_sync(~0u, (int)J.cw, b), ch = __shfl_sync(~0u, (int)J.ch, b);
-        const size_t pitch = __shfl_sync(~0u, J.pitch, b);
-        int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
-        for (int r = 0; r < ch; ++r)
-            for (int x = lane; x < cw; x += 32) blk[(size_t)r * pitch + x] = 0;
-    }
-    __syncwarp();
-    if (ok && D.numbps > 0 && D.npasses > 0) {
-        LaneState<L> S{base, stb, lane};
-        decode_block<STYLED, true>(S, tabs, bytes + D.offset, D.length, D.numbps, D.npasses, J.orient, J.cw, J.ch,
-                                   coeff + J.off, J.pitch, job_style ? (int)job_style[jid] : style,
-                                   STYLED ? pass_ends + (size_t)jid * J2K_PASS_STRIDE : nullptr);
-    }
-    __syncwarp();
-    const int32_t my_half = ok ? cut_half(D.numbps, D.npasses) : 0;
-    for (int b = 0; b < nb; ++b) {
-        if (!((okmask >> b) & 1)) continue;
-        const int cw = __shfl_sync(~0u, (int)J.cw, b), ch = __shfl_sync(~0u, (int)J.ch, b);
-        const size_t pitch = __shfl_sync(~0u, J.pitch, b);
-        int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
-        const int32_t half = __shfl_sync(~0u, my_half, b);
-        for (int r = 0; r < ch; ++r) {
-            const uint64_t sg = base[(0 * 66 + r + 1) * L + b], ng = base[(1 * 66 + r + 1) * L + b];
-            for (int x = lane; x < cw; x += 32) {
-                int32_t v = __ldcg(blk + (size_t)r * pitch + x);
-                if ((sg >> x) & 1) v += half;
-                if ((ng >> x) & 1) v = -v;
-                blk[(size_t)r * pitch + x] = v;
-            }
-        }
-    }
-}
-
-
-// symbol kinds, pass kinds and pending symbols of decode_block_steps
+// symbol kinds and pending symbols of decode_block_steps
 enum : int { kSymZC = 0, kSymSign = 1, kSymMR = 2, kSymRL = 3, kSymUni = 4 };
-enum : int { kPassCU = 0, kPassSP = 1, kPassMR = 2 };
 enum : int { kPendNone = 0, kPendSign = 1, kPendUni1 = 2, kPendUni2 = 3 };
 
 // The same decode as decode_block (unstyled blocks), written as a loop of one symbol per step:
@@ -913,14 +705,58 @@ t1_decode_steps_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __r
 
 }  // namespace
 
-// Host execution of the device decoder logic for one block (used by the test suite): the pass /
-// stripe / column loops that the default decoder kernel runs in each lane, or (steps != 0) the
+// Host execution of the device decoder logic for one block (used by the test suite): the stripe
+// decoder that the default kernel runs, its warp-wide parts one item after another, or (steps) the
 // one-symbol-per-step loop of J2K_TUNE_T1D_STEPS.
+template <bool STYLED>
+static void decode_stripes_host(const uint8_t* data, int len, int numbps, int npasses, int orient, int cw, int ch,
+                                int32_t* out, size_t pitch, int style, const uint32_t* pe) {
+    static const StripeTables T = [] {  // built once, thread-safely
+        StripeTables t{};
+        for (int i = 0; i < 4 * 512; ++i) fill_stripe_tables_entry(t, i);
+        return t;
+    }();
+    uint32_t words[stripe_state_words<1>()] = {};
+    const StripeState<1> S{words};
+    StripeLane<1> me{S, &T, T.zc[orient], 0, cw, ch, {}, {}, false};
+    const int np = std::min(npasses, 3 * numbps - 2), ns = (ch + 3) / 4;
+    for (int q = 0; q < np; ++q) {
+        const int kind = q == 0 ? kPassCU : (q + 2) % 3, p = numbps - 1 - (q + 2) / 3;
+        me.template begin<STYLED>(q, npasses, data, len, style, pe);
+        for (int s = 0; s < ns; ++s) {
+            const uint32_t rv = stripe_rows(ch, s);
+            for (int i = 0; i < 8; ++i) {
+                if (kind == kPassMR) stripe_prepare_mr<1>(S, s, i, 0, cw);
+                else stripe_prepare_zc<1>(S, kind, s, i, 0, cw, rv);
+            }
+            if (kind == kPassSP) me.template decode_zc<STYLED, kPassSP>(rv);
+            else if (kind == kPassMR) me.template decode_mr<STYLED>();
+            else me.template decode_zc<STYLED, kPassCU>(rv);
+            for (int i = 0; i < 8; ++i) {
+                const uint32_t ones = kind == kPassMR ? stripe_finish_mr<1>(S, s, i, 0, cw)
+                                                      : stripe_finish_zc<1>(S, kind, s, i, 0, cw);
+                stripe_add_bits(ones, out, pitch, s, i, p);
+            }
+        }
+    }
+    for (int y = 0; y < ch; ++y)
+        for (int x = 0; x < cw; ++x)
+            if ((S.neg(y >> 2, x >> 3, 0) >> (4 * (x & 7) + (y & 3))) & 1)
+                out[(size_t)y * pitch + x] = -out[(size_t)y * pitch + x];
+}
+
 static int decode_block_host(const uint8_t* data, int len, int numbps, int npasses, int orient, int cw, int ch,
                              int32_t* out, size_t pitch, bool steps) {
     if (cw < 1 || ch < 1 || cw > 64 || ch > 64 || orient < 0 || orient > 3 || numbps < 0 || numbps > 31 ||
         npasses < 0 || npasses > 3 * numbps || len < 0 || (len > 0 && !data) || !out || pitch < (size_t)cw)
         return -1;  // the checks the kernel makes of a descriptor, and the host buffers
+    for (int y = 0; y < ch; ++y)
+        for (int x = 0; x < cw; ++x) out[(size_t)y * pitch + x] = 0;
+    if (numbps == 0 || npasses == 0) return 0;
+    if (!steps) {
+        decode_stripes_host<false>(data, len, numbps, npasses, orient, cw, ch, out, pitch, 0, nullptr);
+        return 0;
+    }
     DecSmem S;
     for (int r = 0; r < 66; ++r) S.sig_[r] = S.neg_[r] = S.ref_[r] = S.vis_[r] = 0;
     for (int k = 0; k < 19; ++k) S.st_[k] = 0;
@@ -929,12 +765,7 @@ static int decode_block_host(const uint8_t* data, int len, int numbps, int npass
         for (int i = 0; i < 4 * 512; ++i) fill_tables_entry(t, i);
         return t;
     }();
-    for (int y = 0; y < ch; ++y)
-        for (int x = 0; x < cw; ++x) out[(size_t)y * pitch + x] = 0;
-    if (numbps > 0 && npasses > 0) {
-        if (steps) decode_block_steps(S, T, data, len, numbps, npasses, orient, cw, ch, out, pitch);
-        else decode_block(S, T, data, len, numbps, npasses, orient, cw, ch, out, pitch);
-    }
+    decode_block_steps(S, T, data, len, numbps, npasses, orient, cw, ch, out, pitch);
     for (int y = 0; y < ch; ++y)
         for (int x = 0; x < cw; ++x)
             if ((S.neg_[y + 1] >> x) & 1) out[(size_t)y * pitch + x] = -out[(size_t)y * pitch + x];
@@ -960,40 +791,34 @@ extern "C" int j2k_t1_decode_block_styled_host(const uint8_t* data, int len, con
         npasses < 0 || npasses > 3 * numbps || npasses > J2K_PASS_STRIDE - 1 || len < 0 || (len > 0 && !data) ||
         !out || pitch < (size_t)cw || !pass_ends || style < 0 || style > 7)
         return -1;
-    DecSmem S;
-    for (int r = 0; r < 66; ++r) S.sig_[r] = S.neg_[r] = S.ref_[r] = S.vis_[r] = 0;
-    for (int k = 0; k < 19; ++k) S.st_[k] = 0;
-    static const DecTables T = [] {
-        DecTables t{};
-        for (int i = 0; i < 4 * 512; ++i) fill_tables_entry(t, i);
-        return t;
-    }();
     for (int y = 0; y < ch; ++y)
         for (int x = 0; x < cw; ++x) out[(size_t)y * pitch + x] = 0;
     if (numbps > 0 && npasses > 0)
-        decode_block<true>(S, T, data, len, numbps, npasses, orient, cw, ch, out, pitch, style, pass_ends);
-    for (int y = 0; y < ch; ++y)
-        for (int x = 0; x < cw; ++x)
-            if ((S.neg_[y + 1] >> x) & 1) out[(size_t)y * pitch + x] = -out[(size_t)y * pitch + x];
+        decode_stripes_host<true>(data, len, numbps, npasses, orient, cw, ch, out, pitch, style, pass_ends);
     return 0;
 }
 
 template <bool STYLED, int L>
-static j2k_status launch_lanes(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs,
-                               const uint8_t* bytes, const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff,
-                               int style, const uint32_t* pass_ends, const uint8_t* job_style,
-                               const uint32_t* order) {
-    constexpr size_t smem = lanes_smem_bytes<L>();
-    const unsigned grid = (unsigned)((njobs + L * cta_warps<L>() - 1) / (L * cta_warps<L>()));
+static j2k_status launch_stripe(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs, const uint8_t* bytes,
+                                const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff, int style,
+                                const uint32_t* pass_ends, const uint8_t* job_style, const uint32_t* order) {
     static std::atomic<uint64_t> attr_set{0};  // devices whose attribute is set, per instantiation
     const uint64_t bit = 1ull << (ctx->device & 63);
     if (!(attr_set.load() & bit)) {
-        J2K_CUDA(ctx, cudaFuncSetAttribute(t1_decode_lanes_kernel<STYLED, L>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        J2K_CUDA(ctx, cudaFuncSetAttribute(t1_decode_stripe_kernel<STYLED, L>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)stripe_smem_bytes<L>(stripe_warps<L>())));
         attr_set.fetch_or(bit);
     }
-    t1_decode_lanes_kernel<STYLED, L><<<grid, 32 * cta_warps<L>(), smem, st>>>(
-        descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err, style, pass_ends, job_style, order);
+    uint32_t* queue = (uint32_t*)j2k_scratch(ctx, SCR_DECQ, 4);
+    if (!queue) return J2K_ERR_OUT_OF_MEMORY;
+    J2K_CUDA(ctx, cudaMemsetAsync(queue, 0, 4, st));
+    // the groups spread over the SMs first, then over the warps of a CTA
+    const size_t groups = (njobs + L - 1) / L, sms = (size_t)ctx->sm_count;
+    const unsigned grid = (unsigned)std::min(groups, sms);
+    const int warps = (int)std::min<size_t>((groups + grid - 1) / grid, (size_t)stripe_warps<L>());
+    t1_decode_stripe_kernel<STYLED, L><<<grid, 32 * warps, stripe_smem_bytes<L>(warps), st>>>(
+        descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err, style, pass_ends, job_style, order, queue);
     J2K_CUDA(ctx, cudaGetLastError());
     return J2K_OK;
 }
@@ -1047,6 +872,19 @@ static j2k_status launch_steps(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc*
     return J2K_OK;
 }
 
+// Blocks per warp: the fewest with which all blocks are resident at once (16, 40 and 84 blocks an
+// SM with 1, 2 and 4 per warp), since a block alone in its warp runs fastest and a second wave
+// costs as much as the first, and 4 for more.  Round trips host to host on B200, 1 / 2 / 4 / 8
+// blocks per warp: 70 blocks of a 512 x 512 gray image 7.0 / 9.9 / 13.4 / 17.7 ms, 777 blocks
+// (1024 x 1024 colour) 8.3 / 10.8 / 13.5 / 19.1, 3072 blocks (2048 x 2048 colour) 14.8 / 12.7 /
+// 14.6 / 19.1, 12288 blocks (4096 x 4096 colour) 48 / 34 / 22.7 / 25.6.
+static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t njobs) {
+    const size_t sms = (size_t)ctx->sm_count;
+    for (int l : {1, 2})
+        if (njobs <= sms * l * (l == 1 ? stripe_warps<1>() : stripe_warps<2>())) return l;
+    return 4;
+}
+
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
                               const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff,
                               cudaStream_t st, int style, const uint32_t* pass_ends, const uint8_t* job_style) {
@@ -1054,46 +892,32 @@ j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint
     if ((style || job_style) && !pass_ends)
         return j2k_fail(ctx, J2K_ERR_INVALID_ARG, "a styled decode needs the pass ends");
     const bool styled = style || job_style;
-    const int L = ctx->t1d_lanes;
-    if (L == 0) {  // one warp per block, lane 0 decoding
-        const unsigned g = (unsigned)((njobs + kWarps - 1) / kWarps);
-        if (styled)
-            t1_decode_kernel<true><<<g, kWarps * 32, 0, st>>>(descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err,
-                                                              style, pass_ends, job_style);
-        else
-            t1_decode_kernel<false><<<g, kWarps * 32, 0, st>>>(descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err,
-                                                               0, nullptr, nullptr);
-        J2K_CUDA(ctx, cudaGetLastError());
-        return J2K_OK;
-    }
+    const int forced = ctx->t1d_lanes;
     if (!styled && ctx->t1d_steps) {
-        switch (L) {
+        switch (forced) {
         case 8: return launch_steps<8>(ctx, st, descs, bytes, d_jobs, njobs, coeff);
         case 16: return launch_steps<16>(ctx, st, descs, bytes, d_jobs, njobs, coeff);
         case 32: return launch_steps<32>(ctx, st, descs, bytes, d_jobs, njobs, coeff);
         default: break;
         }
     }
+    const int L = forced < 0 ? stripe_blocks_per_warp(ctx, njobs)
+                             : (forced <= 1 ? 1 : (forced == 2 ? 2 : (forced <= 4 ? 4 : (forced <= 8 ? 8 : 16))));
     const uint32_t* ord = nullptr;
     if (ctx->t1d_order && njobs > (size_t)L) {
         ord = decode_order(ctx, st, descs, njobs);
         if (!ord) return J2K_ERR_OUT_OF_MEMORY;
     }
     switch ((styled ? 100 : 0) + L) {
-    case 2: return launch_lanes<false, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 3: return launch_lanes<false, 3>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 4: return launch_lanes<false, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 6: return launch_lanes<false, 6>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 8: return launch_lanes<false, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 16: return launch_lanes<false, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 32: return launch_lanes<false, 32>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 102: return launch_lanes<true, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 103: return launch_lanes<true, 3>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 106: return launch_lanes<true, 6>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 104: return launch_lanes<true, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 108: return launch_lanes<true, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 116: return launch_lanes<true, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 132: return launch_lanes<true, 32>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    default: return j2k_fail(ctx, J2K_ERR_INVALID_ARG, "tier-1 decoder: blocks per warp must be 0, 2, 3, 4, 6, 8, 16 or 32");
+    case 1: return launch_stripe<false, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
+    case 2: return launch_stripe<false, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
+    case 4: return launch_stripe<false, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
+    case 8: return launch_stripe<false, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
+    case 16: return launch_stripe<false, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
+    case 101: return launch_stripe<true, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
+    case 102: return launch_stripe<true, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
+    case 104: return launch_stripe<true, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
+    case 108: return launch_stripe<true, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
+    default: return launch_stripe<true, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
     }
 }

@@ -1,0 +1,482 @@
+// Tier-1 block decoder, stripe by stripe (T.800 Annex D; included by t1dec.cu inside its anonymous
+// namespace, after DecTables).
+//
+// A warp decodes L code-blocks side by side, lane b the symbols of block b.  The symbols of a block
+// form one serial chain, so everything that does not belong to that chain is taken out of it and
+// done by the whole warp together, once per pass and stripe of four rows:
+//   prepare  turns the block's bitmaps into one 32-bit word per stripe column that holds all the
+//            column's symbols need (the 3 x 6 significance neighbourhood and the signs around it, or
+//            the refinement labels), and the set of columns that have a symbol;
+//   decode   lane b walks its columns in one flat loop, a significance / refinement decision per
+//            turn: fetch the next column when the last one is done, decode, update the word in
+//            registers (a sample that turns significant reaches the next column as a carry);
+//   finish   turns the column words back into the bitmaps.
+// The lanes of a warp go through the bit-planes, passes and stripes together, so that they meet on
+// the same instructions.
+//
+// Bitmaps: one word per 8 columns of a stripe, a nibble per column (bit j = stripe row j).
+// Column word of the propagation and cleanup passes:
+//   bits 0-17   significance, row r = 0..5 (the row above the stripe, its four rows, the row below)
+//               at 3r: column x-1, x, x+1
+//   bits 18-21  signs of column x-1, stripe rows 0..3
+//   bits 22-27  signs of column x, rows above..below
+//   bits 28-31  signs of column x+1, stripe rows 0..3
+// (a sign bit counts only where the sample is significant).  Column word of the refinement pass:
+// per stripe row k at 3k: to refine, refined before, has a significant neighbour.
+//
+// The parts are host-callable (one lane at a time), which is how they are tested without a GPU.
+
+#define T1D_HD __host__ __device__ __forceinline__
+
+T1D_HD int ctz32(uint32_t v) {
+#ifdef __CUDA_ARCH__
+    return __ffs((int)v) - 1;
+#else
+    return __builtin_ctz(v);
+#endif
+}
+
+T1D_HD int popc32(uint32_t v) {
+#ifdef __CUDA_ARCH__
+    return __popc(v);
+#else
+    return __builtin_popcount(v);
+#endif
+}
+
+// 4 bits to bits 0, 3, 6, 9 and back
+T1D_HD uint32_t spread4(uint32_t n) {
+    n = (n | (n << 4)) & 0xC3u;
+    return (n | (n << 2)) & 0x249u;
+}
+T1D_HD uint32_t gather4(uint32_t x) {
+    x &= 0x249u;
+    x = (x | (x >> 2)) & 0xC3u;
+    return (x | (x >> 4)) & 0xFu;
+}
+
+// Words of a warp's L blocks, interleaved by block so that the lanes' accesses fall in distinct
+// banks: four bitmaps of 16 stripes x 8 words, 64 column words, 2 words of column sets, 19 contexts.
+template <int L>
+struct StripeState {
+    uint32_t* w;
+    T1D_HD uint32_t& sig(int s, int q, int b) const { return w[(s * 8 + q) * L + b]; }
+    T1D_HD uint32_t& neg(int s, int q, int b) const { return w[(128 + s * 8 + q) * L + b]; }
+    T1D_HD uint32_t& vis(int s, int q, int b) const { return w[(256 + s * 8 + q) * L + b]; }
+    T1D_HD uint32_t& ref(int s, int q, int b) const { return w[(384 + s * 8 + q) * L + b]; }
+    T1D_HD uint32_t& col(int x, int b) const { return w[(512 + x) * L + b]; }
+    T1D_HD uint32_t& ctx(int k, int b) const { return w[(576 + k) * L + b]; }
+    // column set of block b, a byte per 8 columns (the bytes of one block are contiguous)
+    T1D_HD uint8_t* cols(int b) const { return reinterpret_cast<uint8_t*>(w + 595 * L) + 8 * b; }
+    T1D_HD uint32_t& colset(int h, int b) const { return (w + 595 * L)[2 * b + h]; }
+};
+template <int L>
+__host__ __device__ constexpr int stripe_state_words() {
+    return 597 * L;
+}
+constexpr int kStripeBitmapWords = 512;  // per block, cleared at the start
+
+enum : int { kPassSP = 0, kPassMR = 1, kPassCU = 2 };
+
+// rows of a column word (propagation / cleanup) with any significant sample in the 3 x 3 window,
+// the centre included, at 3k
+T1D_HD uint32_t near_rows(uint32_t W) {
+    const uint32_t t = W | (W >> 1) | (W >> 2);
+    return t | (t >> 3) | (t >> 6);
+}
+
+// prepare: word q (8 columns) of stripe s of block b, whose rows below the block are outside rv (the
+// stripe's valid rows at 3k) and whose width is cw
+template <int L>
+T1D_HD void stripe_prepare_zc(const StripeState<L>& S, int kind, int s, int q, int b, int cw, uint32_t rv) {
+    if (8 * q >= cw) {
+        S.cols(b)[q] = 0;
+        return;
+    }
+    uint32_t sg[3][3], ng[3][3];  // [stripe s-1, s, s+1][word q-1, q, q+1]
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const bool in = s + i >= 1 && s + i <= 16 && q + j >= 1 && q + j <= 8;
+            sg[i][j] = in ? S.sig(s + i - 1, q + j - 1, b) : 0u;
+            ng[i][j] = in ? S.neg(s + i - 1, q + j - 1, b) : 0u;
+        }
+    uint32_t own_ng = ng[1][1];
+    if (kind == kPassCU) own_ng |= S.vis(s, q, b) & ~sg[1][1];  // visited samples, see stripe_decode
+    // column i - 1 of the word for i = 0 (the word to the left) .. 9 (to the right)
+    auto sig_col = [&](int i) -> uint32_t {
+        const int j = i == 0 ? 0 : (i == 9 ? 2 : 1), sh = 4 * ((i + 7) & 7);
+        return (spread4((sg[1][j] >> sh) & 15u) << 3) | ((sg[0][j] >> (sh + 3)) & 1u) |
+               (((sg[2][j] >> sh) & 1u) << 15);
+    };
+    auto neg_col = [&](int i) -> uint32_t {
+        const int j = i == 0 ? 0 : (i == 9 ? 2 : 1), sh = 4 * ((i + 7) & 7);
+        return (ng[1][j] >> sh) & 15u;
+    };
+    uint32_t v0 = sig_col(0), v1 = sig_col(1), n0 = neg_col(0), n1 = neg_col(1), set = 0;
+#pragma unroll
+    for (int i = 1; i <= 8; ++i) {
+        const uint32_t v2 = sig_col(i + 1), n2 = neg_col(i + 1);
+        const int sh = 4 * (i - 1);
+        const uint32_t vert = ((ng[0][1] >> (sh + 3)) & 1u) | (((own_ng >> sh) & 15u) << 1) |
+                              (((ng[2][1] >> sh) & 1u) << 5);
+        const uint32_t W = v0 | (v1 << 1) | (v2 << 2) | (n0 << 18) | (vert << 22) | (n2 << 28);
+        S.col(8 * q + i - 1, b) = W;
+        uint32_t c = ~(W >> 4) & rv;
+        if (kind == kPassSP) c &= near_rows(W);
+        else c &= ~spread4((W >> 23) & 15u);
+        set |= (uint32_t)(c != 0) << (i - 1);
+        v0 = v1;
+        v1 = v2;
+        n0 = n1;
+        n1 = n2;
+    }
+    if (cw - 8 * q < 8) set &= (1u << (cw - 8 * q)) - 1u;
+    S.cols(b)[q] = (uint8_t)set;
+}
+
+// samples of word q that the refinement pass codes (significant before this plane), and the number
+// of those in the words before it: within a word the bits are in coding order already
+template <int L>
+T1D_HD uint32_t stripe_mr_symbols(const StripeState<L>& S, int s, int q, int b, int* before) {
+    int n = 0;
+    for (int i = 0; i < q; ++i) n += popc32(S.sig(s, i, b) & ~S.vis(s, i, b));
+    *before = n;
+    return S.sig(s, q, b) & ~S.vis(s, q, b);
+}
+
+// prepare of a refinement stripe: no decision changes another one's context here, so the stripe's
+// labels are listed in coding order (a byte each, in the column words) and their number put in
+// column set word 0
+template <int L>
+T1D_HD void stripe_prepare_mr(const StripeState<L>& S, int s, int q, int b, int cw) {
+    if (8 * q >= cw) return;
+    uint32_t vert = 0, h3[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        const bool in = q + j >= 1 && q + j <= 8;
+        const uint32_t m = in ? S.sig(s, q + j - 1, b) : 0u;
+        const uint32_t a = in && s > 0 ? S.sig(s - 1, q + j - 1, b) : 0u;
+        const uint32_t e = in && s < 15 ? S.sig(s + 1, q + j - 1, b) : 0u;
+        const uint32_t ud = ((m << 1) & 0xEEEEEEEEu) | ((a >> 3) & 0x11111111u) | ((m >> 1) & 0x77777777u) |
+                            ((e << 3) & 0x88888888u);
+        h3[j] = m | ud;
+        if (j == 1) vert = ud;
+    }
+    const uint32_t nb = vert | (h3[1] << 4) | (h3[0] >> 28) | (h3[1] >> 4) | (h3[2] << 28);
+    const uint32_t r = S.ref(s, q, b);
+    int at = 0;
+    uint32_t m = stripe_mr_symbols(S, s, q, b, &at);
+    S.ref(s, q, b) = r | m;
+    if (8 * (q + 1) >= cw) S.colset(0, b) = (uint32_t)(at + popc32(m));
+    while (m) {
+        const int i = ctz32(m);
+        m &= m - 1;
+        reinterpret_cast<uint8_t*>(&S.col(at >> 2, b))[at & 3] =
+            (uint8_t)(((r >> i) & 1u) ? 16u : 14u + ((nb >> i) & 1u));
+        ++at;
+    }
+}
+
+// finish: the decisions of a refinement stripe (32 to a word, in coding order) back to their samples
+template <int L>
+T1D_HD uint32_t stripe_finish_mr(const StripeState<L>& S, int s, int q, int b, int cw) {
+    if (8 * q >= cw) return 0;
+    int at = 0;
+    uint32_t ones = 0;
+    for (uint32_t m = stripe_mr_symbols(S, s, q, b, &at); m; m &= m - 1, ++at)
+        ones |= ((S.col(at >> 5, b) >> (at & 31)) & 1u) << ctz32(m);
+    return ones;
+}
+
+// finish: the column words of a propagation or cleanup stripe back into the bitmaps; returns the
+// samples that turned significant
+template <int L>
+T1D_HD uint32_t stripe_finish_zc(const StripeState<L>& S, int kind, int s, int q, int b, int cw) {
+    if (8 * q >= cw) return 0;
+    const uint32_t seen = S.cols(b)[q];  // the columns whose word holds visits (stripe_decode)
+    uint32_t sg = 0, ng = 0, vs = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const uint32_t W = S.col(8 * q + i, b);
+        sg |= gather4(W >> 4) << (4 * i);
+        ng |= ((W >> 23) & 15u) << (4 * i);
+        if (kind == kPassSP && ((seen >> i) & 1u)) vs |= gather4(W) << (4 * i);
+    }
+    const uint32_t ones = sg & ~S.sig(s, q, b);
+    S.sig(s, q, b) = sg;
+    S.neg(s, q, b) = ng & sg;
+    if (kind == kPassSP) S.vis(s, q, b) = vs;
+    return ones;
+}
+
+// bit p of the magnitudes of word q's samples `ones`.  A block's samples belong to one lane at a
+// time; the atomic is a store that needs no load to return (its result is not read).
+T1D_HD void stripe_add_bits(uint32_t ones, int32_t* blk, size_t pitch, int s, int q, int p) {
+    while (ones) {
+        const int i = ctz32(ones);
+        ones &= ones - 1;
+        int32_t* at = blk + (size_t)(4 * s + (i & 3)) * pitch + 8 * q + (i >> 2);
+#ifdef __CUDA_ARCH__
+        atomicOr(reinterpret_cast<unsigned int*>(at), 1u << p);
+#else
+        *at |= 1 << p;
+#endif
+    }
+}
+
+// The MQ decoder (T.800 C.3) with the interval and code registers in the upper halves of 32-bit
+// words, so that the leading-zero count of A is the renormalisation shift.  The byte after the
+// current one is loaded a byte-in ahead.  A context's state is one word: Qe << 16 | MPS << 14 |
+// table index after an MPS << 7 | table index after an LPS (index = state * 2 + MPS).
+struct MqReg {
+    const uint8_t* data;
+    int len, bp, CT;
+    uint32_t A, C, B, n1;
+    T1D_HD uint32_t byte(int i) const { return i < len ? data[i] : 0xFFu; }
+    T1D_HD void bytein() {
+        const bool ff = B == 0xFFu, end = ff && n1 > 0x8Fu;
+        C += end ? 0xFF00u : n1 << (ff ? 9 : 8);
+        CT = ff && !end ? 7 : 8;
+        if (!end) {
+            B = n1;
+            ++bp;
+            n1 = byte(bp + 1);
+        }
+    }
+    T1D_HD void init(const uint8_t* d, int n) {
+        data = d;
+        len = n;
+        bp = 0;
+        B = byte(0);
+        n1 = byte(1);
+        C = B << 16;
+        bytein();
+        C <<= 7;
+        CT -= 7;
+        A = 0x80000000u;
+    }
+    // one decision in a context of state word e; returns the decision, the number of
+    // renormalisation shifts in *shift (0: the state stays) and the state after it in *next
+    T1D_HD uint32_t decide(uint32_t e, const uint32_t* tab, uint32_t* next, int* shift) {
+        const uint32_t qe = e & 0xFFFF0000u, a1 = A - qe;
+        const bool lo = C < qe, lps = lo != (a1 < qe);
+        C -= lo ? 0u : qe;
+        A = lo ? qe : a1;
+        int sh = clz32(A);
+        *shift = sh;
+        *next = e;
+        if (sh) *next = tab[lps ? e & 127u : (e >> 7) & 127u];
+        while (sh > CT) {  // the shifts up to the next byte, the byte, the rest
+            A <<= CT;
+            C <<= CT;
+            sh -= CT;
+            bytein();
+        }
+        A <<= sh;
+        C <<= sh;
+        CT -= sh;
+        return ((e >> 14) & 1u) ^ (uint32_t)lps;
+    }
+};
+
+// entry of the 94-entry state table (index = state * 2 + MPS)
+__host__ __device__ inline uint32_t stripe_mq_entry(int i) {
+    const int st = i >> 1, mps = i & 1;
+    const int sw = st == 0 || st == 6 || st == 14;
+    return ((uint32_t)QE(st) << 16) | ((uint32_t)mps << 14) | ((uint32_t)(NMPS(st) * 2 + mps) << 7) |
+           (uint32_t)(NLPS(st) * 2 + (mps ^ sw));
+}
+
+// Lookup tables of the stripe decoder.  sc is indexed by the column word's own bit layout: bits 1,
+// 3, 5, 7 the significance above, left, right, below; bits 4, 0, 2, 6 their signs.
+struct StripeTables {
+    uint8_t zc[4][512];
+    uint8_t sc[256];
+    uint32_t mq[94];
+};
+__host__ __device__ inline void fill_stripe_tables_entry(StripeTables& T, int i) {
+    if (i < 4 * 512) {
+        const int o = i >> 9, n = i & 511;
+        const int h = ((n >> 3) & 1) + ((n >> 5) & 1), v = ((n >> 1) & 1) + ((n >> 7) & 1);
+        const int d = (n & 1) + ((n >> 2) & 1) + ((n >> 6) & 1) + ((n >> 8) & 1);
+        T.zc[o][n] = (uint8_t)zc_label_calc(o, h, v, d);
+    }
+    if (i < 256) {
+        auto c = [&](int sg, int ng) { return ((i >> sg) & 1) ? (((i >> ng) & 1) ? -1 : 1) : 0; };
+        int hc = max(-1, min(1, c(3, 0) + c(5, 2))), vc = max(-1, min(1, c(1, 4) + c(7, 6)));
+        int xr = 0;
+        if (hc < 0 || (hc == 0 && vc < 0)) { hc = -hc; vc = -vc; xr = 1; }
+        T.sc[i] = (uint8_t)((hc == 0 ? (vc ? 10 : 9) : 12 + vc) | (xr << 7));
+    }
+    if (i < 94) T.mq[i] = stripe_mq_entry(i);
+}
+
+// One lane's block and its coder.
+template <int L>
+struct StripeLane {
+    StripeState<L> S;
+    const StripeTables* T;
+    const uint8_t* zc;
+    int b, cw, ch;
+    MqReg m;
+    RawD rd;
+    bool raw;
+
+    T1D_HD void reset_contexts() const {
+        for (int k = 0; k < 19; ++k) S.ctx(k, b) = T->mq[k == 0 ? 4 * 2 : (k == 17 ? 3 * 2 : (k == 18 ? 46 * 2 : 0))];
+    }
+    template <bool STYLED>
+    T1D_HD uint32_t dec(uint32_t cx) {
+        if (STYLED && raw) return (uint32_t)rd.bit();
+        uint32_t& e = S.ctx((int)cx, b);
+        uint32_t next;
+        int sh;
+        const uint32_t d = m.decide(e, T->mq, &next, &sh);
+        if (sh) e = next;
+        return d;
+    }
+    // the start of pass q of npasses: contexts and segments of a styled block
+    template <bool STYLED>
+    T1D_HD void begin(int q, int npasses, const uint8_t* data, int len, int style, const uint32_t* pe) {
+        if (q == 0) reset_contexts();
+        if (!STYLED) {
+            if (q == 0) m.init(data, len);
+            return;
+        }
+        if (q > 0 && (style & J2K_CBLK_RESET)) reset_contexts();
+        raw = j2k_pass_raw(style, q);
+        if (q == 0 || j2k_pass_terminated(style, q - 1, npasses)) {  // a new segment
+            int e = q;
+            while (!j2k_pass_terminated(style, e, npasses)) ++e;
+            int b0 = q ? (int)min(pe[q - 1], (uint32_t)len) : 0;
+            int b1 = (int)min(pe[e], (uint32_t)len);
+            if (b1 < b0) b1 = b0;
+            if (raw) rd.init(data + b0, b1 - b0);
+            else m.init(data + b0, b1 - b0);
+        }
+    }
+
+    // Propagation (KIND kPassSP) or cleanup (kPassCU) symbols of a stripe: a symbol per turn, with
+    // one decoding site for the zero-coding, run-length, index and sign symbols alike, so that
+    // lanes at different kinds of symbols decode together.
+    template <bool STYLED, int KIND>
+    T1D_HD void decode_zc(uint32_t rv) {
+        enum : int { kZero = 0, kSign = 1, kRun = 2, kIndex1 = 3, kIndex2 = 4 };
+        uint32_t next_set = S.colset(1, b);
+        const uint32_t wide_hi = cw >= 64 ? ~0u : (cw > 32 ? (1u << (cw - 32)) - 1u : 0u);
+        uint32_t W = 0, carry = 0;
+        for (int h = 0; h < 2; ++h) {
+            uint32_t set = h ? next_set : S.colset(0, b), all = set;
+            const uint32_t wide = h ? wide_hi : (cw >= 32 ? ~0u : (1u << cw) - 1u);
+            uint32_t c = 0, v = 0, pcx = 0;
+            int x = h ? -1 : -2, kind = kZero, k3 = 0;
+            uint32_t* at = nullptr;
+            while (set | c) {
+                if (!c) {
+                    const int nx = ctz32(set);
+                    set &= set - 1;
+                    at = &S.col(32 * h + nx, b);
+                    W = *at | (nx == x + 1 ? carry : 0u);
+                    x = nx;
+                    carry = 0;
+                    v = 0;
+                    c = ~(W >> 4) & rv;
+                    if (KIND == kPassSP) {
+                        c &= near_rows(W);
+                        if (!c) *at = W & ~0x249u;  // (a column reached by a carry alone)
+                    } else {
+                        c &= ~spread4((W >> 23) & 15u);
+                        // run-length mode: four samples to code, no significant one around
+                        kind = c == 0x249u && !(W & 0x3FFFFu) ? kRun : kZero;
+                    }
+                }
+                if (c) {
+                    if (kind <= kRun && kind != kSign) k3 = ctz32(c);
+                    uint32_t cx = zc[(W >> k3) & 511u];
+                    if (kind != kZero) cx = kind == kRun ? 17u : pcx & 31u;
+                    uint32_t bit = dec<STYLED>(cx);
+                    bool ask = false;  // a sample turned significant: its sign is the next symbol
+                    if (kind == kZero) {
+                        if (KIND == kPassSP) v |= 1u << k3;
+                        ask = bit != 0;
+                        c &= c - 1;
+                    } else if (kind == kSign) {
+                        if (!(STYLED && raw)) bit ^= pcx >> 7;
+                        const int k = (k3 * 11) >> 5;
+                        W |= (16u << k3) | (bit << (23 + k));
+                        carry |= (8u << k3) | (bit << (18 + k));
+                        kind = kZero;
+                        if (KIND == kPassSP) {  // the next column has a candidate now
+                            const uint32_t nx = x < 31 ? (2u << x) & wide : 0u;
+                            set |= nx;
+                            all |= nx;
+                            if (x == 31 && h == 0) next_set |= 1u & wide_hi;
+                            c = ~(W >> 4) & near_rows(W) & rv;
+                        }
+                        c &= 0x249u & (~1u << k3);  // rows below this one
+                    } else if (kind == kRun) {
+                        c = bit ? c : 0u;
+                        kind = bit ? kIndex1 : kZero;
+                        pcx = 18u;
+                    } else if (kind == kIndex1) {
+                        k3 = 6 * (int)bit;
+                        kind = kIndex2;
+                    } else {
+                        k3 += 3 * (int)bit;
+                        ask = true;
+                    }
+                    if (ask) {
+                        const uint32_t y = W >> k3, z = W >> (18 + ((k3 * 11) >> 5));
+                        pcx = T->sc[(y & 0xAAu) | (z & 0x51u) | ((z >> 8) & 4u)];
+                        kind = kSign;
+                        c |= 0x80000000u;  // (the column is not done: bit 31 is no row)
+                    }
+                    if (!c) *at = KIND == kPassSP ? (W & ~0x249u) | v : W;
+                }
+            }
+            if (KIND == kPassSP) S.colset(h, b) = all;
+            if (x != 31) carry = 0;  // only column 31 is next to column 32
+        }
+    }
+
+    // refinement symbols of a stripe, listed by stripe_prepare_mr; the context state of the next
+    // symbol is loaded a symbol ahead
+    template <bool STYLED>
+    T1D_HD void decode_mr() {
+        const int n = (int)S.colset(0, b);
+        uint32_t out = 0;
+        if (STYLED && raw) {
+            for (int i = 0; i < n; ++i) {
+                out |= (uint32_t)rd.bit() << (i & 31);
+                if ((i & 31) == 31 || i == n - 1) S.col(i >> 5, b) = out, out = 0;
+            }
+            return;
+        }
+        if (n == 0) return;
+        uint32_t labels = S.col(0, b), cx = labels & 31u, e = S.ctx((int)cx, b);
+        for (int i = 0; i < n; ++i) {
+            labels >>= 8;
+            if ((i & 3) == 3) labels = S.col(((i + 1) >> 2) & 63, b);
+            const uint32_t ncx = min(labels & 31u, 18u);  // (past the last label: any context)
+            uint32_t ne = S.ctx((int)ncx, b), next;
+            int sh;
+            out |= m.decide(e, T->mq, &next, &sh) << (i & 31);
+            if (sh) {
+                S.ctx((int)cx, b) = next;
+                if (ncx == cx) ne = next;
+            }
+            cx = ncx;
+            e = ne;
+            if ((i & 31) == 31) S.col(i >> 5, b) = out, out = 0;
+        }
+        if (n & 31) S.col(n >> 5, b) = out;
+    }
+};
+
+// valid rows of stripe s of a block of ch rows, at 3k
+T1D_HD uint32_t stripe_rows(int ch, int s) {
+    const int n = ch - 4 * s;
+    return n >= 4 ? 0x249u : 0x249u & ((1u << (3 * n)) - 1u);
+}
