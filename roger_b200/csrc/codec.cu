@@ -269,17 +269,14 @@ static j2k_status encode_planes(j2k_encoder* e) {
     const size_t csz = 4;
     J2K_TRY(e->coef.ensure(ctx, n * csz * e->ncomp));
     size_t w1 = (e->w + 1) / 2, h1 = (e->h + 1) / 2, w2 = (w1 + 1) / 2, h2 = (h1 + 1) / 2;
-    void* ll0 = j2k_scratch(ctx, SCR_LL0, w1 * h1 * 4);
-    void* ll1 = j2k_scratch(ctx, SCR_LL1, w2 * h2 * 4);
+    // the components side by side: one launch per level
+    const int nc = e->ncomp;
+    void* ll0 = j2k_scratch(ctx, SCR_LL0, w1 * h1 * 4 * nc);
+    void* ll1 = j2k_scratch(ctx, SCR_LL1, w2 * h2 * 4 * nc);
     if (!ll0 || !ll1) return J2K_ERR_OUT_OF_MEMORY;
-    for (int c = 0; c < e->ncomp; ++c) {
-        const char* src = (const char*)e->planes.p + (size_t)c * n * 4;
-        char* dst = (char*)e->coef.p + (size_t)c * n * csz;
-        J2K_TRY(j2k_dwt_fwd_impl(ctx, e->lossy ? J2K_W97 : J2K_W53, e->lossy ? J2K_ORDER_T800 : e->order,
-                                 src, e->w, dst, e->w, e->w, e->h, e->levels,
-                                 quant ? e->steps.data() : nullptr, ll0, ll1, j2k_dwt_tile{64, 64},
-                                 ctx->stream));
-    }
+    J2K_TRY(j2k_dwt_fwd_impl(ctx, e->lossy ? J2K_W97 : J2K_W53, e->lossy ? J2K_ORDER_T800 : e->order, e->planes.p,
+                             e->w, e->coef.p, e->w, e->w, e->h, e->levels, quant ? e->steps.data() : nullptr, ll0, ll1,
+                             j2k_dwt_tile{64, 64}, ctx->stream, nc, n, n));
     e->have_result = true;
     if (e->dwt_only) return J2K_OK;
     return run_tier1(e);
@@ -852,8 +849,8 @@ j2k_status j2k_decoder_run_batch(j2k_decoder* d, const j2k_decode_item* items, i
         byte0[k + 1] = byte0[k] + it.nbytes;
         out_off[k + 1] = out_off[k] + (size_t)it.w * it.h * it.ncomp;
         const size_t w1 = (it.w + 1) / 2, h1 = (it.h + 1) / 2;
-        max_ll0 = std::max(max_ll0, w1 * h1 * 4);
-        max_ll1 = std::max(max_ll1, ((w1 + 1) / 2) * ((h1 + 1) / 2) * 4);
+        max_ll0 = std::max(max_ll0, w1 * h1 * 4 * it.ncomp);
+        max_ll1 = std::max(max_ll1, ((w1 + 1) / 2) * ((h1 + 1) / 2) * 4 * it.ncomp);
         desc_total += it.count;
     }
     // one upload: descriptors and codewords through the page-locked staging buffer
@@ -928,11 +925,10 @@ j2k_status j2k_decoder_run_batch(j2k_decoder* d, const j2k_decode_item* items, i
             if (it.steps) steps.assign(it.steps, it.steps + 3 * lv[k] + 1);
             else steps = default_steps(w, h, lv[k]);
         }
-        for (int c = 0; c < it.ncomp; ++c)
-            J2K_TRY(j2k_dwt_inv_impl(ctx, lossy ? J2K_W97 : J2K_W53, J2K_ORDER_T800,
-                                     (const char*)d->coef.p + (coef_off[k] + (size_t)c * px) * 4, w,
-                                     (char*)d->planes.p + (coef_off[k] + (size_t)c * px) * 4, w, w, h, lv[k],
-                                     lossy ? steps.data() : nullptr, ll0, ll1, j2k_dwt_tile{64, 64}, ctx->stream));
+        J2K_TRY(j2k_dwt_inv_impl(ctx, lossy ? J2K_W97 : J2K_W53, J2K_ORDER_T800,
+                                 (const char*)d->coef.p + coef_off[k] * 4, w, (char*)d->planes.p + coef_off[k] * 4, w, w,
+                                 h, lv[k], lossy ? steps.data() : nullptr, ll0, ll1, j2k_dwt_tile{64, 64}, ctx->stream,
+                                 it.ncomp, px, px));
         const int mct = it.ncomp >= 3 ? (lossy ? J2K_MCT_ICT : J2K_MCT_RCT) : J2K_MCT_NONE;
         J2K_TRY(j2k_launch_planar_inv(ctx, (const char*)d->planes.p + coef_off[k] * 4, lossy ? J2K_F32 : J2K_I32, w,
                                       px, it.ncomp, mct, (uint8_t*)d->out.p + out_off[k], w * it.ncomp, w, h,
@@ -1045,15 +1041,12 @@ j2k_status j2k_decoder_run_codeblocks(j2k_decoder* d, const j2k_cb_desc* descs, 
         else steps = default_steps(w, h, levels);
     }
     size_t w1 = (w + 1) / 2, h1 = (h + 1) / 2, w2 = (w1 + 1) / 2, h2 = (h1 + 1) / 2;
-    void* ll0 = j2k_scratch(ctx, SCR_LL0, w1 * h1 * 4);
-    void* ll1 = j2k_scratch(ctx, SCR_LL1, w2 * h2 * 4);
+    void* ll0 = j2k_scratch(ctx, SCR_LL0, w1 * h1 * 4 * ncomp);
+    void* ll1 = j2k_scratch(ctx, SCR_LL1, w2 * h2 * 4 * ncomp);
     if (!ll0 || !ll1) return J2K_ERR_OUT_OF_MEMORY;
-    for (int c = 0; c < ncomp; ++c) {
-        J2K_TRY(j2k_dwt_inv_impl(ctx, d->lossy ? J2K_W97 : J2K_W53, d->lossy ? J2K_ORDER_T800 : order,
-                                 (const char*)d->coef.p + (size_t)c * n * 4, w,
-                                 (char*)d->planes.p + (size_t)c * n * 4, w, w, h, levels,
-                                 d->lossy ? steps.data() : nullptr, ll0, ll1, j2k_dwt_tile{64, 64}, ctx->stream));
-    }
+    J2K_TRY(j2k_dwt_inv_impl(ctx, d->lossy ? J2K_W97 : J2K_W53, d->lossy ? J2K_ORDER_T800 : order, d->coef.p, w,
+                             d->planes.p, w, w, h, levels, d->lossy ? steps.data() : nullptr, ll0, ll1,
+                             j2k_dwt_tile{64, 64}, ctx->stream, ncomp, n, n));
     int mct = ncomp >= 3 ? (d->lossy ? J2K_MCT_ICT : J2K_MCT_RCT) : J2K_MCT_NONE;
     uint8_t* dst = out;
     if (!out_on_device) {
