@@ -6,22 +6,12 @@
 // (oclbpc.cl:19-111) are completed here from ITU-T T.800 Annex D (contexts, run-length mode,
 // sign coding) and Annex C (MQ coder).
 //
-// Phase A — one warp per code-block.  Every row of the block is a 64-bit mask (bit x =
-// column x) for significance, visited-in-SPP, refined and sign; magnitude bit-planes are sliced
-// into masks with __ballot_sync.  Per stripe (4 rows) and pass:
-//   * significance propagation membership is the causal fixpoint of
-//       N(c,j) = M(c,j) & (E(c,j) | N(c-1,j-1) | N(c-1,j) | N(c-1,j+1) | N(c,j-1)),
-//     solved with a carry-propagate run fill along each row (M & (~(M+S) | S)) iterated over
-//     the 4 rows; all lanes compute it redundantly (uniform, no divergence);
-//   * once the newly significant set is known every context is a function of masks, so lane l
-//     forms the ZC/SC/MR/RL labels for stripe columns 2l and 2l+1 in parallel, and a warp
-//     prefix sum places the symbols in scan order.
-// The output is the exact (context, decision) sequence of the serial coder, one byte per
-// symbol (label in bits 0-4, decision in bit 7; sign symbols also carry their context's XOR
-// bit in bit 5, so that a raw-coded pass can recover the sign itself).
+// Phase A — one warp per code-block writes the exact (context, decision) sequence of the serial
+// coder (t1sym.cuh), one byte per symbol: label in bits 0-4, decision in bit 7; sign symbols also
+// carry their context's XOR bit in bit 5, so that a raw-coded pass can recover the sign itself.
 //
-// Phase B — one lane per code-block runs the MQ encoder over its symbol stream (T.800 C.2,
-// FLUSH of C.2.9, trailing 0xFF dropped); codeword bytes are written as aligned 32-bit words.
+// Phase B — one lane per code-block runs the MQ encoder over its symbol stream (T.800 C.2, FLUSH of
+// C.2.9, trailing 0xFF dropped; mq_enc.cuh); codeword bytes are written as aligned 32-bit words.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -33,55 +23,6 @@ namespace {
 constexpr int kWarpsPerCta = 8;
 constexpr int kRows = 64;
 constexpr int kPlaneWords = 32 * kRows;  // per-block bit-plane scratch: 64 rows x 32 planes
-
-struct WarpSmem {
-    uint64_t sig[kRows + 2], vis[kRows + 2], ref[kRows + 2], neg[kRows + 2];  // index r+1
-    uint64_t bits[kRows];                                                      // current plane
-};
-
-// T.800 Table D.1 zero-coding label from (h, v, d) counts
-__device__ __forceinline__ int zc_label_calc(int orient, int h, int v, int d) {
-    if (orient == J2K_BAND_HH) {
-        int hv = h + v;
-        if (d >= 3) return 8;
-        if (d == 2) return hv >= 1 ? 7 : 6;
-        if (d == 1) return hv >= 2 ? 5 : (hv == 1 ? 4 : 3);
-        return hv >= 2 ? 2 : (hv == 1 ? 1 : 0);
-    }
-    if (orient == J2K_BAND_HL) { int t = h; h = v; v = t; }
-    if (h == 2) return 8;
-    if (h == 1) return v >= 1 ? 7 : (d >= 1 ? 6 : 5);
-    if (v == 2) return 4;
-    if (v == 1) return 3;
-    return d >= 2 ? 2 : d;
-}
-
-// (label | xor<<7) of T.800 Tables D.2/D.3 from the horizontal / vertical contributions
-__device__ __forceinline__ int sc_code(int hc, int vc) {
-    hc = max(-1, min(1, hc));
-    vc = max(-1, min(1, vc));
-    int x = 0;
-    if (hc < 0 || (hc == 0 && vc < 0)) { hc = -hc; vc = -vc; x = 1; }
-    int lab = hc == 0 ? (vc ? 10 : 9) : 12 + vc;
-    return lab | (x << 7);
-}
-
-template <typename T>
-__device__ __forceinline__ T dil(T m) { return m | (T)(m << 1) | (T)(m >> 1); }
-
-// 4-bit window of a row mask around this lane's column pair: bit 0 = column c0-1 ...
-// bit 3 = column c0+2 (columns outside 0..63 read as 0)
-template <typename T>
-__device__ __forceinline__ uint32_t win4(T m, int c0) {
-    return (uint32_t)(c0 ? (m >> (c0 - 1)) : (T)(m << 1)) & 0xF;
-}
-
-// the lane's own columns c0 and c0+1 of a row mask (bit 0 = column c0; columns past the mask
-// read as 0): bits 1-2 of win4 without its left-edge case
-template <typename T>
-__device__ __forceinline__ uint32_t own2(T m, int c0) {
-    return (uint32_t)(m >> c0) & 3u;
-}
 
 // warp exclusive prefix sum; returns the total in *tot
 __device__ __forceinline__ int warp_excl(int v, int lane, int* tot) {
@@ -95,382 +36,7 @@ __device__ __forceinline__ int warp_excl(int v, int lane, int* tot) {
     return inc - v;
 }
 
-// Context/decision emission for one coded sample: ZC (or SC) from 3-bit neighbour windows.
-// zlut: 256-entry zero-coding table of this orientation indexed by the 8 neighbour bits
-// (W E N S NW NE SW SE); slut: sign table indexed by (sig W E N S) | (neg W E N S) << 4.
-struct Lut {
-    const uint8_t* z;
-    const uint8_t* s;
-};
-
-// One code-block's phase A (bit-plane slicing, the three passes per plane, symbol emission).  MT is
-// the row-mask type and CPL the columns per lane: 64-bit masks and two columns per lane for blocks
-// wider than 32, 32-bit masks and one column per lane otherwise (all 32 lanes busy, half the mask
-// work per stripe).
-template <typename MT, int CPL>
-__device__ __forceinline__ void phase_a_block(WarpSmem& S, const j2k_cb_job& J, int jid, int lane,
-                                              const int32_t* __restrict__ coeff, const uint8_t* zlut,
-                                              const uint8_t* slut, uint8_t* __restrict__ syms,
-                                              uint32_t* __restrict__ nsyms, uint32_t* __restrict__ pass_end,
-                                              uint64_t* __restrict__ planes, j2k_cb_desc* __restrict__ descs,
-                                              uint32_t* __restrict__ err, int pad) {
-    const int cw = J.cw, ch = J.ch;
-    const size_t pitch = J.pitch;
-    const int32_t* blk = coeff + J.off;
-    const uint8_t* zl = zlut + J.orient * 256;
-    const MT colmask = (MT)(cw >= 64 ? ~0ull : ((1ull << cw) - 1));
-
-    // ---- bit-plane slicing: lane p ends up holding plane p of each row and stores it
-    uint32_t mor = 0;
-    for (int r = 0; r < ch; ++r) {
-        int32_t v0 = (lane < cw) ? blk[(size_t)r * pitch + lane] : 0;
-        int32_t v1 = (lane + 32 < cw) ? blk[(size_t)r * pitch + lane + 32] : 0;
-        uint32_t m0 = v0 < 0 ? (uint32_t)(-(int64_t)v0) : (uint32_t)v0;
-        uint32_t m1 = v1 < 0 ? (uint32_t)(-(int64_t)v1) : (uint32_t)v1;
-        mor |= m0 | m1;
-        uint64_t ng = (uint64_t)__ballot_sync(0xffffffffu, v0 < 0) |
-                      ((uint64_t)__ballot_sync(0xffffffffu, v1 < 0) << 32);
-        uint32_t any = __reduce_or_sync(0xffffffffu, m0 | m1);
-        uint64_t mine = 0;
-        for (int p = 0; p < 32 && (any >> p); ++p) {
-            uint64_t pm = (uint64_t)__ballot_sync(0xffffffffu, (m0 >> p) & 1) |
-                          ((uint64_t)__ballot_sync(0xffffffffu, (m1 >> p) & 1) << 32);
-            if (lane == p) mine = pm;
-        }
-        planes[r * 32 + lane] = mine;  // row-major [row][plane]: one coalesced 256-byte store
-        if (lane == 0) S.neg[r + 1] = ng;
-    }
-    mor = __reduce_or_sync(0xffffffffu, mor);
-    const int numbps = mor ? 32 - __clz(mor) : 0;
-    for (int r = lane; r < kRows + 2; r += 32) {
-        S.sig[r] = 0;
-        S.vis[r] = 0;
-        S.ref[r] = 0;
-        if (r == 0 || r > ch) S.neg[r] = 0;
-    }
-    j2k_cb_desc d;
-    d.offset = (uint32_t)J.out_off;
-    d.length = 0;
-    d.numbps = (uint8_t)numbps;
-    d.npasses = (uint8_t)(numbps ? 3 * numbps - 2 : 0);
-    d.orient = J.orient;
-    d.band = J.band;
-    d.x0 = J.px0;
-    d.y0 = J.py0;
-    d.cw = J.cw;
-    d.ch = J.ch;
-    d.comp = J.comp;
-    d.reserved = 0;
-    if (numbps > 31) {
-        if (lane == 0) {
-            atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_PLANES);
-            nsyms[jid] = 0;
-            descs[jid] = d;
-        }
-        __syncwarp();
-        return;
-    }
-    __syncwarp();
-    uint8_t* out = syms + J.sym_off;
-    uint32_t* pend = pass_end + (size_t)jid * 92;
-    const int cap = (int)J.sym_cap;
-    int pos = 0, npass = 0;
-    bool ovf = false;
-    const int nstripes = (ch + 3) >> 2;
-    const int c0 = CPL * lane;
-    const bool active = c0 < cw;
-    // columns of this lane present: c0 (and c0+1 with two columns per lane)
-    const uint32_t ownmask = active ? (CPL == 2 && c0 + 1 < cw ? 3u : 1u) : 0u;
-
-    for (int p = numbps - 1; p >= 0 && !ovf; --p) {
-        // current plane into shared (rows beyond ch are zero)
-        S.bits[lane] = lane < ch ? planes[lane * 32 + p] : 0;
-        S.bits[lane + 32] = lane + 32 < ch ? planes[(lane + 32) * 32 + p] : 0;
-        __syncwarp();
-        if (p != numbps - 1) {
-            // ------------------------- significance propagation pass
-            for (int s = 0; s < nstripes && !ovf; ++s) {
-                const int r0 = 4 * s;
-                MT O[6], N[6], C[4], M[4], E[4], K[4], B[4];
-#pragma unroll
-                for (int j = 0; j < 6; ++j) O[j] = S.sig[r0 + j];
-                bool anyk = false;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const MT V = (r0 + j < ch) ? colmask : (MT)0;
-                    C[j] = ~O[j + 1] & V;
-                    E[j] = C[j] & dil((MT)(O[j] | O[j + 1] | O[j + 2]));  // dilation distributes over OR
-                    anyk |= E[j] != 0;
-                }
-                if (!anyk) continue;  // no candidate has a significant neighbour: nothing coded
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    B[j] = S.bits[(r0 + j) & 63];
-                    M[j] = C[j] & B[j];
-                }
-                N[0] = N[5] = 0;
-                N[1] = N[2] = N[3] = N[4] = 0;
-                if ((M[0] | M[1] | M[2] | M[3]) != 0) {  // else no sample becomes significant
-                    // Sweeps top to bottom (each row from the row above as just computed); a row's
-                    // fill is stable unless the row below, computed after it, seeds one of its
-                    // samples outside the runs already filled (row 3's lower neighbour is the next
-                    // stripe, not yet coded: always zero).  The fixpoint is the least one either way.
-                    do {
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            MT seeds = M[j] & (E[j] | ((N[j] | N[j + 2]) << 1) | N[j]);
-                            N[j + 1] = M[j] & (MT)(~(MT)(M[j] + seeds) | seeds);
-                        }
-                    } while (((M[0] & (MT)(N[2] << 1) & ~N[1]) | (M[1] & (MT)(N[3] << 1) & ~N[2]) |
-                              (M[2] & (MT)(N[4] << 1) & ~N[3])) != 0);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) K[j] = C[j] & (E[j] | ((N[j] | N[j + 1] | N[j + 2]) << 1) | N[j]);
-                // per-lane windows
-                uint32_t a[6], o[6], ng[6], kk = 0, bb = 0;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    o[j] = win4(O[j], c0);
-                    a[j] = win4(O[j] | N[j], c0);
-                    ng[j] = win4(S.neg[r0 + j], c0);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    kk |= (own2(K[j], c0) & ownmask) << (2 * j);
-                    bb |= own2(B[j], c0) << (2 * j);
-                }
-                // the newly significant samples are the coded ones whose bit is 1 (N = K & B)
-                const uint32_t nn4 = kk & bb;
-                int cnt = __popc(kk) + __popc(nn4);
-                int tot;
-                int off = pos + warp_excl(cnt, lane, &tot);
-                if (pos + tot > cap) {
-                    ovf = true;
-                    break;
-                }
-                if (cnt) {
-#pragma unroll
-                    for (int k = 0; k < CPL; ++k)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int bitpos = 2 * j + k;
-                            if (!((kk >> bitpos) & 1)) continue;
-                            const uint32_t up = ((a[j] >> k) & 3) | ((o[j] >> k) & 4);
-                            const uint32_t md = ((a[j + 1] >> k) & 1) | ((o[j + 1] >> k) & 4);
-                            const uint32_t dn = ((a[j + 2] >> k) & 1) | ((o[j + 2] >> k) & 6);
-                            // index: W E N S NW NE SW SE
-                            const uint32_t zi = (md & 1) | ((md >> 1) & 2) | ((up & 2) << 1) | ((dn & 2) << 2) |
-                                                ((up & 1) << 4) | ((up & 4) << 3) | ((dn & 1) << 6) | ((dn & 4) << 5);
-                            const int bit = (bb >> bitpos) & 1;
-                            out[off++] = (uint8_t)(zl[zi] | (bit << 7));
-                            if (bit) {
-                                const uint32_t sg4 = (zi & 15);
-                                const uint32_t nw = ng[j + 1] >> k, nu = ng[j] >> k, nd = ng[j + 2] >> k;
-                                const uint32_t ng4 = (nw & 1) | ((nw >> 1) & 2) | ((nu & 2) << 1) | ((nd & 2) << 2);
-                                const int sc = slut[sg4 | (ng4 << 4)];
-                                const int sgn = (ng[j + 1] >> (k + 1)) & 1;
-                                out[off++] = (uint8_t)((sc & 31) | ((sc >> 7) << 5) | ((sgn ^ (sc >> 7)) << 7));
-                            }
-                        }
-                }
-                pos += tot;
-                if (lane == 0) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        S.sig[r0 + j + 1] = O[j + 1] | N[j + 1];
-                        S.vis[r0 + j + 1] = K[j];
-                    }
-                }
-                __syncwarp();
-            }
-            if (lane == 0) pend[npass] = (uint32_t)pos;
-            ++npass;
-            if (pad) {  // the next pass starts on a 16-byte boundary (a coding unit of its own)
-                pos = (pos + 15) & ~15;
-                ovf |= pos > cap;
-            }
-            // ------------------------- magnitude refinement pass
-            for (int s = 0; s < nstripes && !ovf; ++s) {
-                const int r0 = 4 * s;
-                MT SG[6], R[4];
-                bool anyr = false;
-#pragma unroll
-                for (int j = 0; j < 6; ++j) SG[j] = S.sig[r0 + j];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    R[j] = SG[j + 1] & ~S.vis[r0 + j + 1];
-                    anyr |= R[j] != 0;
-                }
-                if (!anyr) continue;
-                uint32_t rr = 0, rf = 0, nb = 0, bb = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const MT nbm = dil((MT)(SG[j] | SG[j + 2])) | (MT)(SG[j + 1] << 1) | (MT)(SG[j + 1] >> 1);
-                    rr |= (own2(R[j], c0) & ownmask) << (2 * j);
-                    rf |= own2(S.ref[r0 + j + 1], c0) << (2 * j);
-                    nb |= own2(nbm, c0) << (2 * j);
-                    bb |= own2(S.bits[(r0 + j) & 63], c0) << (2 * j);
-                }
-                const int cnt = __popc(rr);
-                int tot;
-                int off = pos + warp_excl(cnt, lane, &tot);
-                if (pos + tot > cap) {
-                    ovf = true;
-                    break;
-                }
-                if (cnt) {
-#pragma unroll
-                    for (int k = 0; k < CPL; ++k)
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int bitpos = 2 * j + k;
-                            if (!((rr >> bitpos) & 1)) continue;
-                            const int lab = ((rf >> bitpos) & 1) ? 16 : (((nb >> bitpos) & 1) ? 15 : 14);
-                            out[off++] = (uint8_t)(lab | (((bb >> bitpos) & 1) << 7));
-                        }
-                }
-                pos += tot;
-                if (lane == 0) {
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) S.ref[r0 + j + 1] |= R[j];
-                }
-                __syncwarp();
-            }
-            if (lane == 0) pend[npass] = (uint32_t)pos;
-            ++npass;
-            if (pad) {  // the next pass starts on a 16-byte boundary (a coding unit of its own)
-                pos = (pos + 15) & ~15;
-                ovf |= pos > cap;
-            }
-        }
-        // ------------------------- cleanup pass
-        for (int s = 0; s < nstripes && !ovf; ++s) {
-            const int r0 = 4 * s;
-            const bool full = r0 + 3 < ch;
-            MT O[6], C[4], N[4];
-            bool anyc = false;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) O[j] = S.sig[r0 + j];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const MT V = (r0 + j < ch) ? colmask : (MT)0;
-                C[j] = V & ~O[j + 1] & ~S.vis[r0 + j + 1];
-                N[j] = C[j] & S.bits[(r0 + j) & 63];
-                anyc |= C[j] != 0;
-            }
-            if (!anyc) continue;
-            uint32_t a[6], o[6], ng[6], cc = 0, nn4 = 0;
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                o[j] = win4(O[j], c0);
-                a[j] = win4((j >= 1 && j <= 4) ? (O[j] | N[j - 1]) : O[j], c0);
-                ng[j] = win4(S.neg[r0 + j], c0);
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                cc |= (own2(C[j], c0) & ownmask) << (2 * j);
-                nn4 |= (own2(N[j], c0) & ownmask) << (2 * j);
-            }
-            // per column: run-length mode?  (full stripe, 4 candidates, no significant neighbour)
-            uint32_t rlmask = 0;  // bit k: column c0+k codes in run-length mode
-            int cnt = 0;
-#pragma unroll
-            for (int k = 0; k < CPL; ++k) {
-                const uint32_t colc = (cc >> k) & 0x55;  // bits 0,2,4,6: rows 0..3
-                const uint32_t coln = (nn4 >> k) & 0x55;
-                bool rl = false;
-                if (full && colc == 0x55) {
-                    uint32_t q = 0;
-#pragma unroll
-                    for (int j = 1; j <= 4; ++j) q |= ((a[j] >> k) & 1) | ((o[j] >> k) & 4);
-                    q |= ((o[0] >> k) & 7) | ((o[5] >> k) & 7);
-                    rl = q == 0;
-                }
-                if (rl) {
-                    rlmask |= 1u << k;
-                    if (coln) {
-                        const int first = (__ffs(coln) - 1) >> 1;  // row of the first 1
-                        int rest = 0;
-                        for (int j = first + 1; j < 4; ++j) rest += 1 + ((coln >> (2 * j)) & 1);
-                        cnt += 1 + 2 + 1 + rest;
-                    } else {
-                        cnt += 1;
-                    }
-                } else {
-                    cnt += __popc(colc) + __popc(coln);
-                }
-            }
-            int tot;
-            int off = pos + warp_excl(cnt, lane, &tot);
-            if (pos + tot > cap) {
-                ovf = true;
-                break;
-            }
-            if (cnt) {
-#pragma unroll
-                for (int k = 0; k < CPL; ++k) {
-                    const uint32_t colc = (cc >> k) & 0x55;
-                    const uint32_t coln = (nn4 >> k) & 0x55;
-                    if (!colc) continue;
-                    int jstart = 0;
-                    if ((rlmask >> k) & 1) {
-                        out[off++] = (uint8_t)(17 | ((coln != 0) << 7));
-                        if (!coln) continue;
-                        const int first = (__ffs(coln) - 1) >> 1;
-                        out[off++] = (uint8_t)(18 | (((first >> 1) & 1) << 7));
-                        out[off++] = (uint8_t)(18 | ((first & 1) << 7));
-                        // sign of the first significant sample: its four neighbours are insignificant
-                        const int sgn = (ng[first + 1] >> (k + 1)) & 1;
-                        const int sc = slut[0];
-                        out[off++] = (uint8_t)((sc & 31) | ((sc >> 7) << 5) | ((sgn ^ (sc >> 7)) << 7));
-                        jstart = first + 1;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        if (j < jstart || !((colc >> (2 * j)) & 1)) continue;
-                        const uint32_t up = ((a[j] >> k) & 3) | ((o[j] >> k) & 4);
-                        const uint32_t md = ((a[j + 1] >> k) & 1) | ((o[j + 1] >> k) & 4);
-                        const uint32_t dn = ((a[j + 2] >> k) & 1) | ((o[j + 2] >> k) & 6);
-                        const uint32_t zi = (md & 1) | ((md >> 1) & 2) | ((up & 2) << 1) | ((dn & 2) << 2) |
-                                            ((up & 1) << 4) | ((up & 4) << 3) | ((dn & 1) << 6) | ((dn & 4) << 5);
-                        const int bit = (coln >> (2 * j)) & 1;
-                        out[off++] = (uint8_t)(zl[zi] | (bit << 7));
-                        if (bit) {
-                            const uint32_t nw = ng[j + 1] >> k, nu = ng[j] >> k, nd = ng[j + 2] >> k;
-                            const uint32_t ng4 = (nw & 1) | ((nw >> 1) & 2) | ((nu & 2) << 1) | ((nd & 2) << 2);
-                            const int sc = slut[(zi & 15) | (ng4 << 4)];
-                            const int sgn = (ng[j + 1] >> (k + 1)) & 1;
-                            out[off++] = (uint8_t)((sc & 31) | ((sc >> 7) << 5) | ((sgn ^ (sc >> 7)) << 7));
-                        }
-                    }
-                }
-            }
-            pos += tot;
-            if (lane == 0) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) S.sig[r0 + j + 1] = O[j + 1] | N[j];
-            }
-            __syncwarp();
-        }
-        if (lane == 0) pend[npass] = (uint32_t)pos;
-        ++npass;
-        if (pad) {
-            pos = (pos + 15) & ~15;
-            ovf |= pos > cap;
-        }
-        for (int r = lane; r < kRows + 2; r += 32) S.vis[r] = 0;
-        __syncwarp();
-    }
-    if (ovf) {
-        if (lane == 0) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_SYM_CAPACITY);
-        pos = 0;
-    }
-    if (lane == 0) {
-        nsyms[jid] = (uint32_t)pos;
-        descs[jid] = d;
-    }
-    __syncwarp();
-}
+#include "t1sym.cuh"
 
 // MINB: resident CTAs per SM the register budget is cut for (2: no spills; 3: a few spilled
 // registers, more warps to hide the ALU chains)
@@ -481,23 +47,9 @@ t1_symbols_kernel(const int32_t* __restrict__ coeff, const j2k_cb_job* __restric
                   uint8_t* __restrict__ syms, uint32_t* __restrict__ nsyms,
                   uint32_t* __restrict__ pass_end, uint64_t* __restrict__ plane_scratch,
                   j2k_cb_desc* __restrict__ descs, uint32_t* __restrict__ err, int pad) {
-    __shared__ WarpSmem smem[kWarpsPerCta];
-    __shared__ uint8_t zlut[4][256];
-    __shared__ uint8_t slut[256];
-    for (int i = threadIdx.x; i < 4 * 256; i += blockDim.x) {
-        int o = i >> 8, b = i & 255;
-        int W = b & 1, E = (b >> 1) & 1, N = (b >> 2) & 1, S = (b >> 3) & 1;
-        int d = ((b >> 4) & 1) + ((b >> 5) & 1) + ((b >> 6) & 1) + ((b >> 7) & 1);
-        zlut[o][b] = (uint8_t)zc_label_calc(o, W + E, N + S, d);
-    }
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) {
-        int sg = i & 15, ng = i >> 4;
-        auto ct = [&](int k) { return ((sg >> k) & 1) ? (((ng >> k) & 1) ? -1 : 1) : 0; };
-        slut[i] = (uint8_t)sc_code(ct(0) + ct(1), ct(2) + ct(3));
-    }
-    __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    WarpSmem& S = smem[wid];
+    extern __shared__ __align__(16) uint8_t sym_smem[];
+    SymSmem& S = reinterpret_cast<SymSmem*>(sym_smem)[wid];
     // persistent: each warp pulls code-blocks from the device-side queue until it is empty;
     // its bit-plane scratch slot is reused from block to block
     uint64_t* planes = plane_scratch + (size_t)(blockIdx.x * kWarpsPerCta + wid) * kPlaneWords;
@@ -515,12 +67,12 @@ t1_symbols_kernel(const int32_t* __restrict__ coeff, const j2k_cb_job* __restric
         }
         continue;
     }
-    if (J.cw <= 32)
-        phase_a_block<uint32_t, 1>(S, J, jid, lane, coeff, &zlut[0][0], slut, syms, nsyms, pass_end, planes, descs,
-                                   err, pad);
+    if (J.cw > 32)
+        symbols_of_block<4, 2, uint64_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
+    else if (J.ch > 32)
+        symbols_of_block<2, 2, uint32_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
     else
-        phase_a_block<uint64_t, 2>(S, J, jid, lane, coeff, &zlut[0][0], slut, syms, nsyms, pass_end, planes, descs,
-                                   err, pad);
+        symbols_of_block<1, 4, uint32_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
     }  // queue loop
 }
 
@@ -1322,11 +874,10 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
     uint8_t* syms = (uint8_t*)j2k_scratch(ctx, SCR_SYMS, sym_bytes + 64);
     // persistent phase A: one bit-plane slot per resident warp
     int per_sm = 0;
-    const bool occ3 = ctx->t1a_ctas == 3;
-    if (occ3)
-        J2K_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, t1_symbols_kernel<3>, kWarpsPerCta * 32, 0));
-    else
-        J2K_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, t1_symbols_kernel<2>, kWarpsPerCta * 32, 0));
+    const auto symbols = ctx->t1a_ctas == 3 ? t1_symbols_kernel<3> : t1_symbols_kernel<2>;
+    constexpr size_t sym_smem = kWarpsPerCta * sizeof(SymSmem);
+    J2K_CUDA(ctx, cudaFuncSetAttribute(symbols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sym_smem));
+    J2K_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, symbols, kWarpsPerCta * 32, sym_smem));
     per_sm = std::max(per_sm, 1);
     const size_t ctas = std::min<size_t>((njobs + kWarpsPerCta - 1) / kWarpsPerCta, (size_t)per_sm * ctx->sm_count);
     uint64_t* planes = (uint64_t*)j2k_scratch(ctx, SCR_PLANES, ctas * kWarpsPerCta * kPlaneWords * 8 + 64);
@@ -1343,14 +894,8 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
     J2K_CUDA(ctx, cudaMemsetAsync(queue, 0, 4, st));
     // with per-pass coding units (RESET | TERMALL) every pass's symbols start 16-byte aligned
     const int pad = (style & (J2K_CBLK_RESET | J2K_CBLK_TERMALL)) == (J2K_CBLK_RESET | J2K_CBLK_TERMALL) ? 1 : 0;
-    if (occ3)
-        t1_symbols_kernel<3><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(coeff, d_jobs, (int)njobs, d_order, queue,
-                                                                          syms, nsyms, pend, planes, descs, ctx->d_err,
-                                                                          pad);
-    else
-        t1_symbols_kernel<2><<<(unsigned)ctas, kWarpsPerCta * 32, 0, st>>>(coeff, d_jobs, (int)njobs, d_order, queue,
-                                                                          syms, nsyms, pend, planes, descs, ctx->d_err,
-                                                                          pad);
+    symbols<<<(unsigned)ctas, kWarpsPerCta * 32, sym_smem, st>>>(coeff, d_jobs, (int)njobs, d_order, queue, syms, nsyms,
+                                                                 pend, planes, descs, ctx->d_err, pad);
     J2K_CUDA(ctx, cudaGetLastError());
     if (style)
         return encode_styled_units(ctx, d_jobs, njobs, descs, bytes, sym_bytes, syms, pend, style, pass_ends, st);
