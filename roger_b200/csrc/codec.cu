@@ -665,8 +665,8 @@ j2k_status j2k_encoder_autotune(j2k_encoder* e, int reps, int* report) {
     reps = std::max(reps, 1);
     // candidates: {tier-0 warps per SM, tier-1 warps per SM, tier-1 blocks per warp, blocks per
     // warp after the tiers}; 0 warps: no tier
-    const int cand[8][4] = {{1, 2, 4, 16}, {1, 2, 4, 8}, {1, 2, 4, 32}, {1, 0, 0, 8},
-                            {1, 0, 0, 16}, {0, 0, 0, 8}, {2, 2, 4, 16}, {1, 2, 8, 16}};
+    const int cand[8][4] = {{1, 0, 0, 8}, {1, 0, 0, 16}, {1, 0, 0, 32}, {1, 1, 4, 16},
+                            {1, 1, 4, 32}, {1, 2, 4, 16}, {0, 0, 0, 16}, {0, 0, 0, 32}};
     cudaEvent_t e0, e1;
     J2K_CUDA(ctx, cudaEventCreate(&e0));
     J2K_CUDA(ctx, cudaEventCreate(&e1));

@@ -193,13 +193,10 @@ j2k_status j2k_ctx_create(int device, j2k_ctx** out) {
         return J2K_ERR_CUDA;
     }
     c->stream = c->own_stream;
-    // MQ schedule (longest blocks first): one warp per SM with one block each, two warps per SM
-    // with four blocks each, then 16 blocks per warp
+    // MQ schedule (longest blocks first): one warp pair per SM with one block each, then as many
+    // blocks per pair as the number of blocks asks for (mq_lanes 0)
     c->mq_tier_warps[0] = c->sm_count;
     c->mq_tier_lanes[0] = 1;
-    c->mq_tier_warps[1] = 2 * c->sm_count;
-    c->mq_tier_lanes[1] = 4;
-    c->mq_lanes = 16;
     *out = c;
     return J2K_OK;
     J2K_API_END

@@ -190,10 +190,6 @@ struct MqCoder {
     }
 };
 
-// The symbol loop of one lane: n symbols at syms (16-byte aligned; bits 0-4 context, bit 7
-// decision).  Symbols come in 16-byte chunks, two in flight; the state of the next symbol's context
-// is loaded a symbol ahead and replaced when this symbol changes the same context.  ends.at() is
-// called after symbol i - 1 wherever ends.next() == i.
 struct MqNoEnds {
     MQ_HD uint32_t next() const { return 0xFFFFFFFFu; }
     MQ_HD void at(const MqCoder&) {}
@@ -246,31 +242,49 @@ struct MqMem {
     }
 };
 
-template <int SHIFT, class Ends>
-MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, const MqMem<SHIFT> mem, Ends& ends) {
-    const uint4* sp = reinterpret_cast<const uint4*>(syms);
-    const int nchunks = (n + 15) >> 4;
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    uint4 c0 = nchunks > 0 ? MQ_LOAD16(sp) : z, c1 = nchunks > 1 ? MQ_LOAD16(sp + 1) : z;
-    uint32_t cx = mem.context(c0.x, 0);
-    MqState cur = mem.state(cx);
-    // four symbols, of which `left` exist; without branches, so that the chains of neighbouring
-    // symbols overlap
-    const auto group = [&](uint32_t w, uint32_t wnext, int left, uint32_t done) {
-        uint32_t a[4];
-        int s[4];
+// The interval part's walk over a symbol stream: n symbols at syms (16-byte aligned; bits 0-4
+// context, bit 7 decision) in 16-byte chunks, two in flight; the state of the next symbol's context
+// is loaded a symbol ahead and replaced when this symbol changes the same context.
+template <int SHIFT>
+struct MqSymbols {
+    const MqMem<SHIFT> mem;
+    const uint4* sp;
+    int n, nchunks;
+    uint4 c0, c1;
+    uint32_t cx;
+    MqState cur;
+    MQ_HD MqSymbols(const uint8_t* syms, int count, MqMem<SHIFT> m)
+        : mem(m), sp(reinterpret_cast<const uint4*>(syms)), n(count), nchunks((count + 15) >> 4) {
+        const uint4 z = make_uint4(0, 0, 0, 0);
+        c0 = nchunks > 0 ? MQ_LOAD16(sp) : z;
+        c1 = nchunks > 1 ? MQ_LOAD16(sp + 1) : z;
+        cx = mem.context(c0.x, 0);
+        cur = mem.state(cx);
+    }
+    // chunk k (in order), then the one after it in c0
+    MQ_HD uint4 next(int k) {
+        const uint4 w = c0;
+        c0 = c1;
+        c1 = k + 2 < nchunks ? MQ_LOAD16(sp + k + 2) : make_uint4(0, 0, 0, 0);
+        return w;
+    }
+    // four symbols w, of which `left` exist, the next one in wnext: put(j, value added to C, shifts
+    // << 23); without branches, so that the chains of neighbouring symbols overlap
+    template <class Put>
+    MQ_HD void group(MqCoder& e, uint32_t w, uint32_t wnext, int left, Put put) {
 #ifdef __CUDA_ARCH__
 #pragma unroll
 #endif
         for (int j = 0; j < 4; ++j) {
-            a[j] = 0;
-            s[j] = 0;
-            if (j > 0 && j >= left) continue;
+            if (j > 0 && j >= left) {
+                put(j, 0u, 0u);
+                continue;
+            }
             const uint32_t ncx = j < 3 ? mem.context(w, j + 1) : mem.context(wnext, 0);
             const MqState nx = mem.state(ncx);
-            uint32_t to;
-            const uint32_t moved = e.interval(cur, w << (24 - 8 * j), &a[j], &to);
-            s[j] = (int)(moved >> 23);
+            uint32_t to, add;
+            const uint32_t moved = e.interval(cur, w << (24 - 8 * j), &add, &to);
+            put(j, add, moved);
             const MqState up = mem.entry(to);
             mem.store_if(moved, cx, up);
             // the next symbol's state: the one loaded ahead, unless this symbol has changed it
@@ -278,45 +292,69 @@ MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, const MqMem<SHIFT> 
             cur = MqState{changed ? up.x : nx.x, changed ? up.y : nx.y};
             cx = ncx;
         }
-        if (ends.next() > done + 4u) {
-            e.code4(a, s);
-        } else {  // a plane ends in this group: symbol by symbol
-#ifdef __CUDA_ARCH__
-#pragma unroll
-#endif
-            for (int j = 0; j < 4; ++j) {
-                e.C += a[j];
-                e.shift(s[j]);
-                while (ends.next() == done + j + 1u) ends.at(e);
-            }
-        }
-    };
-    int k = 0;
-    for (; 16 * k + 16 <= n; ++k) {
-        uint32_t wa = c0.x, wb = c0.y, wc = c0.z, wd = c0.w;
-        c0 = c1;
-        c1 = k + 2 < nchunks ? MQ_LOAD16(sp + k + 2) : z;
+    }
+    // all symbols in order: each(w, wnext, left, number of the first) for every four
+    template <class Group>
+    MQ_HD void walk(Group each) {
+        int k = 0;
+        for (; 16 * k + 16 <= n; ++k) {
+            const uint4 c = next(k);
+            uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w;
 #ifdef __CUDA_ARCH__
 #pragma unroll 1
 #endif
-        for (int q = 0; q < 4; ++q) {
-            group(wa, wb, 4, (uint32_t)(16 * k + 4 * q));
+            for (int q = 0; q < 4; ++q) {
+                each(wa, wb, 4, 16 * k + 4 * q);
+                wa = wb;
+                wb = wc;
+                wc = wd;
+                wd = c0.x;
+            }
+        }
+        uint32_t wa = c0.x, wb = c0.y, wc = c0.z, wd = c0.w;
+#ifdef __CUDA_ARCH__
+#pragma unroll 1
+#endif
+        for (int i = 16 * k; i < n; i += 4) {
+            each(wa, wb, n - i, i);
             wa = wb;
             wb = wc;
             wc = wd;
-            wd = c0.x;
         }
     }
-    uint32_t wa = c0.x, wb = c0.y, wc = c0.z, wd = c0.w;
+};
+
+// The code part of four symbols that follow symbol `done`; ends.at() is called after symbol i - 1
+// wherever ends.next() == i.
+template <class Ends>
+MQ_HD void mq_code_group(MqCoder& e, const uint32_t (&a)[4], const int (&s)[4], uint32_t done, Ends& ends) {
+    if (ends.next() > done + 4u) {
+        e.code4(a, s);
+    } else {  // a plane ends in this group: symbol by symbol
 #ifdef __CUDA_ARCH__
-#pragma unroll 1
+#pragma unroll
 #endif
-    for (int i = 16 * k; i < n; i += 4) {
-        group(wa, wb, n - i, (uint32_t)i);
-        wa = wb;
-        wb = wc;
-        wc = wd;
+        for (int j = 0; j < 4; ++j) {
+            e.C += a[j];
+            e.shift(s[j]);
+            while (ends.next() == done + j + 1u) ends.at(e);
+        }
     }
+}
+
+// Both parts by one lane
+template <int SHIFT, class Ends>
+MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, MqMem<SHIFT> mem, Ends& ends) {
+    MqSymbols<SHIFT> src(syms, n, mem);
+    src.walk([&](uint32_t w, uint32_t wnext, int left, int done) {
+        uint32_t a[4];
+        int s[4];
+        src.group(e, w, wnext, left, [&](int j, uint32_t add, uint32_t moved) {
+            a[j] = add;
+            s[j] = (int)(moved >> 23);
+        });
+        mq_code_group(e, a, s, (uint32_t)done, ends);
+    });
 }
 
 MQ_HD MqState mq_table_entry(uint32_t qe, uint32_t nmps, uint32_t nlps, uint32_t sw, uint32_t mps) {

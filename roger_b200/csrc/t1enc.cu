@@ -114,8 +114,8 @@ __device__ __forceinline__ void reset_mq_states(MqState* st, int stride, const M
     st[18 * stride] = tab[46 * 2];
 }
 
-// The byte-by-byte MQ encoder registers of the general styled coder and the state + code warp pair,
-// and the byte writer of raw passes.
+// The byte-by-byte MQ encoder registers of the general styled coder, and the byte writer of raw
+// passes.
 struct MqEnc {
     uint32_t A, C, B;   // B: pending output byte (may still receive a carry)
     int CT, bp;         // bp: index of B (-1 before the first byte)
@@ -197,222 +197,113 @@ struct MqPlaneEnds {
     }
 };
 
-// One lane per block (mq_enc.cuh).  Bound by the dependent instructions of a symbol at few warps per
-// scheduler (12288 blocks of a 4096 x 4096 colour image are 1129 warps for 592 schedulers): 43
-// instructions and 104 cycles a symbol for a block alone in its warp, 57 and 165 with 32 in a warp.
-// The integer coder it replaced (a leading-zero count and a branch to the byte output in every
-// symbol's chain) took 51 instructions and over 200 cycles alone, 85 with 16.  70 blocks of a 512 x
-// 512 gray image: 2.8 -> 1.67 ms; 4096 x 4096 colour: 4.4 -> 3.0 ms.
+// One block per lane of a warp pair (mq_enc.cuh): warp 0 runs the interval part and puts four
+// symbols' additions and shifts into a ring in shared memory, warp 1 takes them through the code
+// part a chunk of 16 symbols behind.  The two parts are serial chains of their own, so a symbol
+// costs the longer one instead of both.  Bound by the interval chain: 34 instructions and 85 cycles
+// a symbol for a block alone in its pair, about 145 with 32 blocks.  One warp with both parts takes
+// 104 and 165 cycles: whole encodes of a 512 x 512 gray image 1.9 ms against 1.58 with pairs, of a
+// 4096 x 4096 colour image 4.1 against 3.7.  An integer coder with a leading-zero count and a branch
+// to the byte output in every symbol's chain took over 200 cycles (2.8 and 6.0 ms).
 // RATE: also record the plane ends (MqPlaneEnds) into plane_bytes[job * 32 + k].
 template <bool RATE>
-__global__ void __launch_bounds__(kMqThreads)
+__global__ void __launch_bounds__(2 * kMqThreads)
 t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jobs, const uint32_t* __restrict__ nsyms,
              const uint32_t* __restrict__ order, int njobs, uint8_t* __restrict__ bytes,
              j2k_cb_desc* __restrict__ descs, uint32_t* __restrict__ err, const uint32_t* __restrict__ pend,
              uint32_t* __restrict__ plane_bytes, MqSchedule sched, int lanes) {
     __shared__ MqState tab[94];
     __shared__ MqState cst[32 * kMqThreads];
+    __shared__ uint4 ring[2][4][kMqThreads];  // [chunk parity][group][lane]
+    __shared__ float last_a[kMqThreads];
     fill_mq_table(tab);
-    __syncwarp();
-    const int lane = threadIdx.x;
-    // warp w takes blocks in longest-first order: the schedule's tiers first (warps with fewer
-    // blocks each), then `lanes` blocks per warp
+    const int lane = threadIdx.x & 31;
+    // pair w takes blocks in longest-first order: the schedule's tiers first (pairs with fewer
+    // blocks each), then `lanes` blocks per pair
     const int w = blockIdx.x;
-    int gid = -1, wbase = 0, gbase = 0;
+    int gid = -1, mine = lanes, wbase = 0, gbase = 0;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (gid < 0 && w < wbase + sched.warps[k]) {
-            if (lane >= sched.lanes[k]) return;
-            gid = gbase + (w - wbase) * sched.lanes[k] + lane;
+            mine = sched.lanes[k];
+            gid = gbase + (w - wbase) * mine + lane;
         }
         wbase += sched.warps[k];
         gbase += sched.warps[k] * sched.lanes[k];
     }
-    if (gid < 0) {
-        if (lane >= lanes) return;
-        gid = gbase + (w - wbase) * lanes + lane;
-    }
-    if (gid >= njobs) return;
-    const int jid = order ? (int)order[gid] : gid;
-    MqState* st = cst + lane;
-    reset_mq_states(st, kMqThreads, tab);
-    const j2k_cb_job J = jobs[jid];
-    const int n = (int)min(nsyms[jid], J.sym_cap);
+    if (gid < 0) gid = gbase + (w - wbase) * lanes + lane;
+    const bool live = lane < mine && gid < njobs;
+    const int jid = live ? (order ? (int)order[gid] : gid) : 0;
+    j2k_cb_job J{};
+    if (live) J = jobs[jid];
+    const int n = live ? (int)min(nsyms[jid], J.sym_cap) : 0;
+    const int chunks = (__reduce_max_sync(0xffffffffu, n) + 15) >> 4;  // the same in both warps
+    __syncthreads();
     MqCoder e;
     e.init(reinterpret_cast<uint32_t*>(bytes + J.out_off), (int)J.out_cap);
-    if (RATE) {
-        MqPlaneEnds ends{pend + (size_t)jid * 92, plane_bytes + (size_t)jid * 32, descs[jid].npasses, 0, 0};
+    if (threadIdx.x < 32) {
+        MqState* st = cst + lane;
+        reset_mq_states(st, kMqThreads, tab);
+        MqSymbols<5> src(syms + J.sym_off, n, MqMem<5>(st, tab));
+        for (int k = 0; k < chunks; ++k) {
+            const uint4 c = src.next(k);
+            uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w, ev[4];
+            const auto put = [&](int j, uint32_t add, uint32_t moved) { ev[j] = add | (moved >> 7); };
+            if (16 * k + 16 <= n) {
+#pragma unroll 1
+                for (int q = 0; q < 4; ++q) {
+                    src.group(e, wa, wb, 4, put);
+                    ring[k & 1][q][lane] = make_uint4(ev[0], ev[1], ev[2], ev[3]);
+                    wa = wb;
+                    wb = wc;
+                    wc = wd;
+                    wd = src.c0.x;
+                }
+            } else {
+#pragma unroll 1
+                for (int q = 0; 16 * k + 4 * q < n; ++q) {
+                    src.group(e, wa, wb, n - 16 * k - 4 * q, put);
+                    ring[k & 1][q][lane] = make_uint4(ev[0], ev[1], ev[2], ev[3]);
+                    wa = wb;
+                    wb = wc;
+                    wc = wd;
+                }
+            }
+            if (16 * k + 16 >= n) last_a[lane] = e.A;  // (again in every chunk after the last symbol)
+            __syncthreads();
+        }
+        return;
+    }
+    MqPlaneEnds ends{};
+    ends.end = 0xFFFFFFFFu;
+    if (RATE && live) {
+        ends = MqPlaneEnds{pend + (size_t)jid * 92, plane_bytes + (size_t)jid * 32, descs[jid].npasses, 0, 0};
         ends.start();
         while (ends.next() == 0u) ends.at(e);  // passes with no symbols at all
-        mq_encode(e, syms + J.sym_off, n, MqMem<5>(st, tab), ends);
-    } else {
-        MqNoEnds ends;
-        mq_encode(e, syms + J.sym_off, n, MqMem<5>(st, tab), ends);
     }
-    int len = n > 0 ? e.flush() : 0;
+    MqNoEnds none;
+    for (int k = 0; k < chunks; ++k) {
+        __syncthreads();  // chunk k is in the ring; the interval warp goes on with chunk k + 1
+#pragma unroll 1
+        for (int q = 0; q < 4 && 16 * k + 4 * q < n; ++q) {
+            const uint4 r = ring[k & 1][q][lane];
+            const uint32_t a[4] = {r.x & 0xFFFFu, r.y & 0xFFFFu, r.z & 0xFFFFu, r.w & 0xFFFFu};
+            const int s[4] = {(int)(r.x >> 16), (int)(r.y >> 16), (int)(r.z >> 16), (int)(r.w >> 16)};
+            if (RATE) mq_code_group(e, a, s, (uint32_t)(16 * k + 4 * q), ends);
+            else mq_code_group(e, a, s, (uint32_t)(16 * k + 4 * q), none);
+        }
+    }
+    if (!live) return;
+    int len = 0;
+    if (n > 0) {
+        e.A = last_a[lane];
+        len = e.flush();
+    }
     if (e.ovf || len > (int)J.out_cap) {
         atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_OUT_CAPACITY);
         len = 0;
     }
     descs[jid].length = len;
-}
-
-// ---- decoupled MQ coder: probability-state warp + code-register warp ---------------------------
-//
-// The MQ recurrences split cleanly: the interval register A and the 19 context states never
-// read the code register C, and C (with its byte output) only needs, per symbol, the value
-// Qe, whether Qe is added to C, and the renormalisation shift.  Warp 0 of each CTA runs the
-// A/state recurrence for 32 blocks (one per lane, branch-free) and writes one packed entry
-// per symbol (Qe | add<<16 | shift<<17) into a double-buffered shared ring; warp 1 runs the C
-// recurrence and the T.800 C.2 byte output one 32-symbol chunk behind.  Each warp carries
-// half of the serial chain and the two halves overlap.
-constexpr int kPairChunk = 32;
-
-__global__ void __launch_bounds__(64)
-t1_mq_pair_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jobs, const uint32_t* __restrict__ nsyms,
-                  const uint32_t* __restrict__ order, int njobs, uint8_t* __restrict__ bytes,
-                   j2k_cb_desc* __restrict__ descs, uint32_t* __restrict__ err) {
-    __shared__ uint32_t tab[47];
-    __shared__ uint32_t cst[20 * 32];
-    __shared__ uint32_t ring[2][kPairChunk][32];
-    __shared__ uint32_t finalA[32];
-    for (int i = threadIdx.x; i < 47; i += blockDim.x)
-        tab[i] = (uint32_t)c_qe[i] | ((uint32_t)c_nmps[i] << 16) | ((uint32_t)c_nlps[i] << 22) |
-                 ((uint32_t)(i == 0 || i == 6 || i == 14) << 28);
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int gid = blockIdx.x * 32 + lane;
-    const bool live = gid < njobs;
-    const int jid = live ? (order ? (int)order[gid] : gid) : 0;
-    const j2k_cb_job J = jobs[jid];
-    const size_t sym_cap = J.sym_cap, cap_per_block = J.out_cap;
-    const int n = live ? (int)min((size_t)nsyms[jid], sym_cap) : 0;
-    int nmax = n;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-    const int nchunks = (nmax + kPairChunk - 1) / kPairChunk;
-    if (warp == 0) {
-        // ------------------------------------------------ probability-state warp
-        uint32_t* st = cst + lane;  // context k at st[32*k]
-        for (int k = 0; k < 19; ++k) st[32 * k] = tab[0];
-        st[0] = tab[4];
-        st[32 * 17] = tab[3];
-        st[32 * 18] = tab[46];
-        uint32_t A = 0x8000;
-        const uint4* sp4 = reinterpret_cast<const uint4*>(syms + J.sym_off);
-        const int nq = (n + 15) >> 4;  // 16-symbol chunks of this lane
-        const uint4 z4 = make_uint4(0, 0, 0, 0);
-        uint4 q0 = nq > 0 ? __ldcs(sp4) : z4, q1 = nq > 1 ? __ldcs(sp4 + 1) : z4;
-        uint4 q2 = nq > 2 ? __ldcs(sp4 + 2) : z4, q3 = nq > 3 ? __ldcs(sp4 + 3) : z4;
-        int cx = min((int)(q0.x & 31), 18);
-        uint32_t ent = st[32 * cx];
-        for (int k = 0; k <= nchunks; ++k) {
-            if (k < nchunks) {
-                const uint32_t w[9] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x};
-                const int base = k * kPairChunk;
-                uint32_t* rb = &ring[k & 1][0][lane];
-#pragma unroll
-                for (int j = 0; j < kPairChunk; ++j) {
-                    const bool valid = base + j < n;
-                    const uint32_t sym = (w[j >> 2] >> (8 * (j & 3))) & 0xFF;
-                    const uint32_t nsym = (w[(j + 1) >> 2] >> (8 * ((j + 1) & 3))) & 0xFF;
-                    const int ncx = min((int)(nsym & 31), 18);
-                    uint32_t nent = st[32 * ncx];
-                    const uint32_t qe = valid ? (ent & 0xFFFF) : 0u;
-                    const int mps = ent >> 31;
-                    const bool is_mps = !valid || ((int)(sym >> 7) == mps);
-                    const uint32_t a1 = A - qe;
-                    const bool fast = is_mps && (a1 & 0x8000);
-                    const bool addc = fast || (is_mps != (a1 < qe));
-                    const uint32_t a2 = addc ? a1 : qe;
-                    const int sh = __clz(a2) - 16;
-                    A = a2 << sh;
-                    const int nidx = is_mps ? (ent >> 16) & 63 : (ent >> 22) & 63;
-                    const uint32_t nmps = (uint32_t)(mps ^ (!is_mps & (int)((ent >> 28) & 1)));
-                    const uint32_t upd = tab[nidx] | (nmps << 31);
-                    if (!fast) {
-                        st[32 * cx] = upd;
-                        if (ncx == cx) nent = upd;
-                    }
-                    rb[32 * j] = qe | ((uint32_t)addc << 16) | ((uint32_t)sh << 17);
-                    cx = ncx;
-                    ent = nent;
-                }
-                // advance the symbol window by two 16-symbol chunks, keeping two in flight
-                const int nextq = 2 * (k + 1);
-                q0 = q2;
-                q1 = q3;
-                q2 = nextq + 2 < nq ? __ldcs(sp4 + nextq + 2) : z4;
-                q3 = nextq + 3 < nq ? __ldcs(sp4 + nextq + 3) : z4;
-            } else {
-                finalA[lane] = A;
-            }
-            __syncthreads();
-        }
-    } else {
-        // ------------------------------------------------ code-register warp
-        MqEnc e;
-        e.A = 0;
-        e.C = 0;
-        e.B = 0;
-        e.CT = 12;
-        e.bp = -1;
-        e.out = reinterpret_cast<uint32_t*>(bytes + J.out_off);
-        e.cap = (int)cap_per_block;
-        e.wacc = 0;
-        e.wn = 0;
-        e.wbase = 0;
-        e.ovf = false;
-        for (int k = 0; k <= nchunks; ++k) {
-            if (k > 0) {
-                const uint32_t* rb = &ring[(k - 1) & 1][0][lane];
-#pragma unroll 8
-                for (int j = 0; j < kPairChunk; ++j) {
-                    const uint32_t en = rb[32 * j];
-                    e.C += (en & 0xFFFF) & (0u - ((en >> 16) & 1));
-                    int sh = (int)(en >> 17);
-                    if (sh < e.CT) {
-                        e.C <<= sh;
-                        e.CT -= sh;
-                    } else {
-                        while (sh > 0) {
-                            const int kk = min(sh, e.CT);
-                            e.C <<= kk;
-                            e.CT -= kk;
-                            sh -= kk;
-                            if (e.CT == 0) e.byteout();
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        if (!live) return;
-        int len = 0;
-        if (n > 0) {
-            e.A = finalA[lane];
-            uint32_t tempc = e.C + e.A;
-            e.C |= 0xFFFF;
-            if (e.C >= tempc) e.C -= 0x8000;
-            e.C <<= e.CT;
-            e.byteout();
-            e.C <<= e.CT;
-            e.byteout();
-            len = e.bp + 1;
-            if (e.B == 0xFF) len--;
-            e.push(e.B);
-            uint8_t* bb = bytes + J.out_off;
-            for (int k = 0; k < e.wn; ++k) {
-                if (e.wbase + k < e.cap) bb[e.wbase + k] = (uint8_t)(e.wacc >> (8 * k));
-                else e.ovf = true;
-            }
-        }
-        if (e.ovf || len > (int)cap_per_block) {
-            atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_OUT_CAPACITY);
-            len = 0;
-        }
-        descs[jid].length = len;
-    }
 }
 
 // ---- code-block styles: coding units --------------------------------------------------------
@@ -862,6 +753,16 @@ static j2k_status encode_styled_units(j2k_ctx* ctx, const j2k_cb_job* d_jobs, si
     return J2K_OK;
 }
 
+// Rate control also needs the distortion of each truncation point (the coefficients are still in
+// place); the MQ coder has recorded the byte positions at every bit-plane end.
+static j2k_status launch_dist(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_job* d_jobs, const j2k_cb_desc* descs,
+                              size_t njobs, double* dist, cudaStream_t st) {
+    t1_dist_kernel<<<(unsigned)((njobs + kDistWarps - 1) / kDistWarps), kDistWarps * 32, 0, st>>>(coeff, d_jobs, descs,
+                                                                                                 (int)njobs, dist);
+    J2K_CUDA(ctx, cudaGetLastError());
+    return J2K_OK;
+}
+
 j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_job* d_jobs, size_t njobs,
                               j2k_cb_desc* descs, uint8_t* bytes, size_t sym_bytes,
                               const uint32_t* d_order, cudaStream_t st, uint32_t* plane_bytes, double* dist,
@@ -907,13 +808,7 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
     if (!tbuf) return J2K_ERR_OUT_OF_MEMORY;
     J2K_CUDA(ctx, cub::DeviceRadixSort::SortPairsDescending(tbuf, tmp, nsyms, keys_out, idx_in, idx_out,
                                                             (int)njobs, 0, 32, st));
-    if (ctx->mq_variant == 1 && !(plane_bytes && dist)) {  // the rate path runs the one-lane coder
-        unsigned gp = (unsigned)((njobs + 31) / 32);
-        t1_mq_pair_kernel<<<gp, 64, 0, st>>>(syms, d_jobs, nsyms, idx_out, (int)njobs, bytes, descs, ctx->d_err);
-        J2K_CUDA(ctx, cudaGetLastError());
-        return J2K_OK;
-    }
-    const int lanes = ctx->mq_lanes;  // active lanes (blocks) per warp: 32, 16 or 8
+    const bool rate = plane_bytes && dist;
     // tiers of the schedule, cut to the blocks there are
     MqSchedule sc{};
     size_t left = njobs, warps = 0;
@@ -925,20 +820,16 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
         left -= std::min(left, wk * l);
         warps += wk;
     }
+    // blocks per pair after the tiers: two more pairs per SM hold the rest, up to full warps.  Whole
+    // encodes on B200 after a tier of one block per SM, by blocks per pair: 777 blocks 1 2.68, 2 2.12,
+    // 4 2.08 ms; 3072 blocks 4 3.26, 8 2.85, 12 2.77; 12288 blocks 8 6.8, 16 5.6, 24 and 32 4.8 (before
+    // the context modelling took a third of that)
+    const size_t per = 2 * (size_t)ctx->sm_count;
+    const int lanes = ctx->mq_lanes ? ctx->mq_lanes : (int)std::min<size_t>(std::max<size_t>((left + per - 1) / per, 1), 32);
     warps += (left + lanes - 1) / lanes;
-    const bool rate = plane_bytes && dist;
-    // rate control also records the byte positions at every bit-plane end, and the distortion
-    // of each truncation point (the coefficients are still in place)
-    if (rate) {
-        t1_mq_kernel<true><<<(unsigned)warps, kMqThreads, 0, st>>>(syms, d_jobs, nsyms, idx_out, (int)njobs, bytes, descs,
-                                                                   ctx->d_err, pend, plane_bytes, sc, lanes);
-        J2K_CUDA(ctx, cudaGetLastError());
-        t1_dist_kernel<<<(unsigned)((njobs + kDistWarps - 1) / kDistWarps), kDistWarps * 32, 0, st>>>(
-            coeff, d_jobs, descs, (int)njobs, dist);
-    } else {
-        t1_mq_kernel<false><<<(unsigned)warps, kMqThreads, 0, st>>>(syms, d_jobs, nsyms, idx_out, (int)njobs, bytes, descs,
-                                                                    ctx->d_err, nullptr, nullptr, sc, lanes);
-    }
+    const auto mq = rate ? t1_mq_kernel<true> : t1_mq_kernel<false>;
+    mq<<<(unsigned)warps, 2 * kMqThreads, 0, st>>>(syms, d_jobs, nsyms, idx_out, (int)njobs, bytes, descs, ctx->d_err, pend,
+                                               plane_bytes, sc, lanes);
     J2K_CUDA(ctx, cudaGetLastError());
-    return J2K_OK;
+    return rate ? launch_dist(ctx, coeff, d_jobs, descs, njobs, dist, st) : J2K_OK;
 }
