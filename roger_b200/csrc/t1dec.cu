@@ -4,14 +4,16 @@
 // DWT).  Decoding is serial per code-block: every context depends on the bits decoded before it.
 // The kernel runs one code-block per lane, 1, 2 or 4 (8, 16 by tuning) in a warp, and takes all
 // work that is not a block's own serial chain out of the lanes' loops (t1dec_stripe.cuh).  What
-// bounds it: the chain of dependent instructions per symbol (about 95 warp instructions and 430
-// cycles a symbol with one block per warp), and with 4 blocks per warp instruction issue, since
-// the lanes are at different kinds of symbols.  Round trips host to host on B200, against a decoder
-// whose lanes kept 64-bit row masks and gathered each column's neighbourhood themselves: 512 x 512
-// gray 15.3 -> 6.5 ms, 2048 x 2048 colour 18.8 -> 12.9 ms, 4096 x 4096 colour 28.2 -> 22.5 ms.
+// bounds it: the chain of dependent instructions per symbol (about 91 warp instructions and 360
+// cycles a symbol with one block per warp), and with 4 blocks per warp the ALU pipe, since the lanes
+// are at different kinds of symbols (1.74 times the instructions of one).  Round trips host to host
+// on B200, against a decoder whose lanes kept 64-bit row masks and gathered each column's
+// neighbourhood themselves: 512 x 512 gray 15.3 -> 5.7 ms, 2048 x 2048 colour 18.8 -> 10.5 ms,
+// 4096 x 4096 colour 28.2 -> 21.8 ms.
 // The warp clears its blocks' output regions first and applies the signs at the end; magnitude bits
 // go to the output plane by fire-and-forget atomic ORs (each block owns its region).
 #include <atomic>
+#include <cstring>
 
 #include <cub/cub.cuh>
 
@@ -339,7 +341,7 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
         }
         // this lane's block, and the sizes and pass counts of the blocks of its items
         const int np = ok && D.numbps > 0 ? min((int)D.npasses, 3 * (int)D.numbps - 2) : 0;
-        StripeLane<L> me{S, &tabs, tabs.zc[J.orient & 3], lane, J.cw, J.ch, {}, {}, false};
+        StripeLane<L> me{S, LaneMem<L>(S, tabs, J.orient & 3, lane < L ? lane : 0), lane, J.cw, J.ch, {}, {}, false};
         int icw[R], ich[R], inp[R], inb[R];
         uint32_t ipitch[R];
         int32_t* iblk[R];
@@ -718,7 +720,7 @@ static void decode_stripes_host(const uint8_t* data, int len, int numbps, int np
     }();
     uint32_t words[stripe_state_words<1>()] = {};
     const StripeState<1> S{words};
-    StripeLane<1> me{S, &T, T.zc[orient], 0, cw, ch, {}, {}, false};
+    StripeLane<1> me{S, LaneMem<1>(S, T, orient, 0), 0, cw, ch, {}, {}, false};
     const int np = std::min(npasses, 3 * numbps - 2), ns = (ch + 3) / 4;
     for (int q = 0; q < np; ++q) {
         const int kind = q == 0 ? kPassCU : (q + 2) % 3, p = numbps - 1 - (q + 2) / 3;
@@ -875,9 +877,9 @@ static j2k_status launch_steps(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc*
 // Blocks per warp: the fewest with which all blocks are resident at once (16, 40 and 84 blocks an
 // SM with 1, 2 and 4 per warp), since a block alone in its warp runs fastest and a second wave
 // costs as much as the first, and 4 for more.  Round trips host to host on B200, 1 / 2 / 4 / 8
-// blocks per warp: 70 blocks of a 512 x 512 gray image 7.0 / 9.9 / 13.4 / 17.7 ms, 777 blocks
-// (1024 x 1024 colour) 8.3 / 10.8 / 13.5 / 19.1, 3072 blocks (2048 x 2048 colour) 14.8 / 12.7 /
-// 14.6 / 19.1, 12288 blocks (4096 x 4096 colour) 48 / 34 / 22.7 / 25.6.
+// blocks per warp: 70 blocks of a 512 x 512 gray image 5.7 / 7.6 / 10.2 / 14.2 ms, 777 blocks
+// (1024 x 1024 colour) 6.8 / 8.4 / 10.4 / 15.5, 3072 blocks (2048 x 2048 colour) 12.5 / 10.5 /
+// 11.8 / 15.5, 12288 blocks (4096 x 4096 colour) 43 / 32 / 21.8 / 22.0.
 static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t njobs) {
     const size_t sms = (size_t)ctx->sm_count;
     for (int l : {1, 2})

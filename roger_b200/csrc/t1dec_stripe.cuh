@@ -28,11 +28,11 @@
 
 #define T1D_HD __host__ __device__ __forceinline__
 
-T1D_HD int ctz32(uint32_t v) {
+T1D_HD int ctz32(uint32_t v) {  // -1 for 0
 #ifdef __CUDA_ARCH__
     return __ffs((int)v) - 1;
 #else
-    return __builtin_ctz(v);
+    return v ? __builtin_ctz(v) : -1;
 #endif
 }
 
@@ -55,8 +55,15 @@ T1D_HD uint32_t gather4(uint32_t x) {
     return (x | (x >> 4)) & 0xFu;
 }
 
+// MQ state of a context: x = Qe as a float, the MPS in the sign bit; y = Qe << 16 | table entry after
+// an LPS << 8 | entry after an MPS (entries of the 94-entry table, state * 2 + MPS)
+struct alignas(8) MqdState {
+    uint32_t x, y;
+};
+
 // Words of a warp's L blocks, interleaved by block so that the lanes' accesses fall in distinct
-// banks: four bitmaps of 16 stripes x 8 words, 64 column words, 2 words of column sets, 19 contexts.
+// banks: four bitmaps of 16 stripes x 8 words, 64 column words, 19 context states of 2 words, 2
+// words of column sets.
 template <int L>
 struct StripeState {
     uint32_t* w;
@@ -65,14 +72,14 @@ struct StripeState {
     T1D_HD uint32_t& vis(int s, int q, int b) const { return w[(256 + s * 8 + q) * L + b]; }
     T1D_HD uint32_t& ref(int s, int q, int b) const { return w[(384 + s * 8 + q) * L + b]; }
     T1D_HD uint32_t& col(int x, int b) const { return w[(512 + x) * L + b]; }
-    T1D_HD uint32_t& ctx(int k, int b) const { return w[(576 + k) * L + b]; }
+    T1D_HD MqdState& ctx(int k, int b) const { return reinterpret_cast<MqdState*>(w + 576 * L)[k * L + b]; }
     // column set of block b, a byte per 8 columns (the bytes of one block are contiguous)
-    T1D_HD uint8_t* cols(int b) const { return reinterpret_cast<uint8_t*>(w + 595 * L) + 8 * b; }
-    T1D_HD uint32_t& colset(int h, int b) const { return (w + 595 * L)[2 * b + h]; }
+    T1D_HD uint8_t* cols(int b) const { return reinterpret_cast<uint8_t*>(w + 614 * L) + 8 * b; }
+    T1D_HD uint32_t& colset(int h, int b) const { return (w + 614 * L)[2 * b + h]; }
 };
 template <int L>
 __host__ __device__ constexpr int stripe_state_words() {
-    return 597 * L;
+    return 616 * L;
 }
 constexpr int kStripeBitmapWords = 512;  // per block, cleared at the start
 
@@ -226,14 +233,33 @@ T1D_HD void stripe_add_bits(uint32_t ones, int32_t* blk, size_t pitch, int s, in
     }
 }
 
-// The MQ decoder (T.800 C.3) with the interval and code registers in the upper halves of 32-bit
-// words, so that the leading-zero count of A is the renormalisation shift.  The byte after the
-// current one is loaded a byte-in ahead.  A context's state is one word: Qe << 16 | MPS << 14 |
-// table index after an MPS << 7 | table index after an LPS (index = state * 2 + MPS).
+T1D_HD uint32_t float_bits(float f) {
+#ifdef __CUDA_ARCH__
+    return __float_as_uint(f);
+#else
+    uint32_t u;
+    memcpy(&u, &f, 4);
+    return u;
+#endif
+}
+T1D_HD float bits_float(uint32_t u) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float f;
+    memcpy(&f, &u, 4);
+    return f;
+#endif
+}
+
+// The MQ decoder (T.800 C.3).  A is kept as a float of the 16-bit register's value (integers below
+// 2^16: exact), whose exponent is restored to renormalise, so that no leading-zero count is in the
+// chain; C has its 16 compared bits on top.  The byte after the current one is loaded a byte-in ahead.
 struct MqReg {
     const uint8_t* data;
     int len, bp, CT;
-    uint32_t A, C, B, n1;
+    float A;
+    uint32_t C, B, n1;
     T1D_HD uint32_t byte(int i) const { return i < len ? data[i] : 0xFFu; }
     T1D_HD void bytein() {
         const bool ff = B == 0xFFu, end = ff && n1 > 0x8Fu;
@@ -255,38 +281,39 @@ struct MqReg {
         bytein();
         C <<= 7;
         CT -= 7;
-        A = 0x80000000u;
+        A = 32768.0f;
     }
-    // one decision in a context of state word e; returns the decision, the number of
-    // renormalisation shifts in *shift (0: the state stays) and the state after it in *next
-    T1D_HD uint32_t decide(uint32_t e, const uint32_t* tab, uint32_t* next, int* shift) {
-        const uint32_t qe = e & 0xFFFF0000u, a1 = A - qe;
-        const bool lo = C < qe, lps = lo != (a1 < qe);
-        C -= lo ? 0u : qe;
-        A = lo ? qe : a1;
-        int sh = clz32(A);
-        *shift = sh;
-        *next = e;
-        if (sh) *next = tab[lps ? e & 127u : (e >> 7) & 127u];
+    // one decision in a context of state e: the decision; *moved != 0 when the state changes, to
+    // table entry *to
+    T1D_HD uint32_t decide(MqdState e, uint32_t* moved, uint32_t* to) {
+        constexpr uint32_t EXP = 0x47000000u;  // exponent field of 0x8000 <= A < 0x10000
+        const uint32_t Q = e.y & 0xFFFF0000u;
+        const float q = bits_float(e.x & 0x7FFFFFFFu), a1 = A - q;
+        const bool lo = C < Q, lps = lo != (a1 < q);
+        C -= lo ? 0u : Q;
+        const uint32_t m = float_bits(lo ? q : a1);
+        A = bits_float((m & 0x7FFFFFu) | EXP);
+        *moved = EXP - (m & 0x7F800000u);
+        *to = (e.y >> (lps ? 8 : 0)) & 0x7Fu;
+        int sh = (int)(*moved >> 23);
         while (sh > CT) {  // the shifts up to the next byte, the byte, the rest
-            A <<= CT;
             C <<= CT;
             sh -= CT;
             bytein();
         }
-        A <<= sh;
         C <<= sh;
         CT -= sh;
-        return ((e >> 14) & 1u) ^ (uint32_t)lps;
+        return (e.x >> 31) ^ (uint32_t)lps;
     }
 };
 
 // entry of the 94-entry state table (index = state * 2 + MPS)
-__host__ __device__ inline uint32_t stripe_mq_entry(int i) {
+__host__ __device__ inline MqdState stripe_mq_entry(int i) {
     const int st = i >> 1, mps = i & 1;
     const int sw = st == 0 || st == 6 || st == 14;
-    return ((uint32_t)QE(st) << 16) | ((uint32_t)mps << 14) | ((uint32_t)(NMPS(st) * 2 + mps) << 7) |
-           (uint32_t)(NLPS(st) * 2 + (mps ^ sw));
+    return MqdState{float_bits((float)QE(st)) | ((uint32_t)mps << 31),
+                    ((uint32_t)QE(st) << 16) | ((uint32_t)(NLPS(st) * 2 + (mps ^ sw)) << 8) |
+                        (uint32_t)(NMPS(st) * 2 + mps)};
 }
 
 // Lookup tables of the stripe decoder.  sc is indexed by the column word's own bit layout: bits 1,
@@ -294,7 +321,7 @@ __host__ __device__ inline uint32_t stripe_mq_entry(int i) {
 struct StripeTables {
     uint8_t zc[4][512];
     uint8_t sc[256];
-    uint32_t mq[94];
+    MqdState mq[94];
 };
 __host__ __device__ inline void fill_stripe_tables_entry(StripeTables& T, int i) {
     if (i < 4 * 512) {
@@ -313,29 +340,94 @@ __host__ __device__ inline void fill_stripe_tables_entry(StripeTables& T, int i)
     if (i < 94) T.mq[i] = stripe_mq_entry(i);
 }
 
+// What a lane's symbol loops touch: its block's column words and context states and the tables.  On
+// the device 32-bit shared-memory addresses that the compiler cannot see through (it computes the
+// address of a shared array anew for every access otherwise, special-register read included).
+template <int L>
+struct LaneMem {
+#ifdef __CUDA_ARCH__
+    uint32_t cols, ctxs, zcs, scs, mqs;
+    __device__ __forceinline__ LaneMem(const StripeState<L>& S, const StripeTables& T, int orient, int b)
+        : cols(addr(&S.col(0, b))), ctxs(addr(&S.ctx(0, b))), zcs(addr(T.zc[orient])), scs(addr(T.sc)), mqs(addr(T.mq)) {
+        asm volatile("" : "+r"(cols), "+r"(ctxs), "+r"(zcs), "+r"(scs), "+r"(mqs));
+    }
+    __device__ __forceinline__ static uint32_t addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+    __device__ __forceinline__ uint32_t col(int x) const {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(cols + x * (4 * L)) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ void col_set(int x, uint32_t v) const {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(cols + x * (4 * L)), "r"(v) : "memory");
+    }
+    __device__ __forceinline__ MqdState ctx(uint32_t k) const { return load(ctxs + k * (8 * L)); }
+    __device__ __forceinline__ MqdState entry(uint32_t i) const { return load(mqs + 8 * i); }
+    __device__ __forceinline__ void ctx_set_if(uint32_t cond, uint32_t k, MqdState v) const {
+        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.shared.v2.u32 [%0], {%1, %2};\n}" ::"r"(
+                         ctxs + k * (8 * L)),
+                     "r"(v.x), "r"(v.y), "r"(cond)
+                     : "memory");
+    }
+    __device__ __forceinline__ uint32_t zc(uint32_t i) const { return byte(zcs + i); }
+    __device__ __forceinline__ uint32_t sc(uint32_t i) const { return byte(scs + i); }
+    __device__ __forceinline__ static MqdState load(uint32_t at) {
+        MqdState v;
+        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(at) : "memory");
+        return v;
+    }
+    __device__ __forceinline__ static uint32_t byte(uint32_t at) {
+        uint32_t v;
+        asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+        return v;
+    }
+#else
+    const StripeState<L>& S;
+    const StripeTables& T;
+    int o, b;
+    LaneMem(const StripeState<L>& s, const StripeTables& t, int orient, int blk) : S(s), T(t), o(orient), b(blk) {}
+    uint32_t col(int x) const { return S.col(x, b); }
+    void col_set(int x, uint32_t v) const { S.col(x, b) = v; }
+    MqdState ctx(uint32_t k) const { return S.ctx((int)k, b); }
+    MqdState entry(uint32_t i) const { return T.mq[i]; }
+    void ctx_set_if(uint32_t cond, uint32_t k, MqdState v) const {
+        if (cond) S.ctx((int)k, b) = v;
+    }
+    uint32_t zc(uint32_t i) const { return T.zc[o][i]; }
+    uint32_t sc(uint32_t i) const { return T.sc[i]; }
+#endif
+};
+
 // One lane's block and its coder.
 template <int L>
 struct StripeLane {
     StripeState<L> S;
-    const StripeTables* T;
-    const uint8_t* zc;
+    LaneMem<L> mem;
     int b, cw, ch;
     MqReg m;
     RawD rd;
     bool raw;
 
     T1D_HD void reset_contexts() const {
-        for (int k = 0; k < 19; ++k) S.ctx(k, b) = T->mq[k == 0 ? 4 * 2 : (k == 17 ? 3 * 2 : (k == 18 ? 46 * 2 : 0))];
+        for (int k = 0; k < 19; ++k)
+            S.ctx(k, b) = mem.entry(k == 0 ? 4 * 2 : (k == 17 ? 3 * 2 : (k == 18 ? 46 * 2 : 0)));
+    }
+    // one decision in context cx of state e; *up is the context's state after it where *moved
+    template <bool STYLED>
+    T1D_HD uint32_t dec(uint32_t cx, MqdState e, MqdState* up, uint32_t* moved) {
+        *up = e;
+        *moved = 0;
+        if (STYLED && raw) return (uint32_t)rd.bit();
+        uint32_t to;
+        const uint32_t d = m.decide(e, moved, &to);
+        *up = mem.entry(to);
+        mem.ctx_set_if(*moved, cx, *up);
+        return d;
     }
     template <bool STYLED>
     T1D_HD uint32_t dec(uint32_t cx) {
-        if (STYLED && raw) return (uint32_t)rd.bit();
-        uint32_t& e = S.ctx((int)cx, b);
-        uint32_t next;
-        int sh;
-        const uint32_t d = m.decide(e, T->mq, &next, &sh);
-        if (sh) e = next;
-        return d;
+        MqdState up;
+        uint32_t moved;
+        return dec<STYLED>(cx, mem.ctx(cx), &up, &moved);
     }
     // the start of pass q of npasses: contexts and segments of a styled block
     template <bool STYLED>
@@ -358,82 +450,126 @@ struct StripeLane {
         }
     }
 
-    // Propagation (KIND kPassSP) or cleanup (kPassCU) symbols of a stripe: a symbol per turn, with
-    // one decoding site for the zero-coding, run-length, index and sign symbols alike, so that
-    // lanes at different kinds of symbols decode together.
+    // samples of a column that a pass codes, at 3k
+    template <int KIND>
+    T1D_HD static uint32_t candidates(uint32_t W, uint32_t rv) {
+        const uint32_t c = ~(W >> 4) & rv;
+        return KIND == kPassSP ? c & near_rows(W) : c & ~spread4((W >> 23) & 15u);
+    }
+    // run-length mode: four samples to code, no significant one around them
+    template <int KIND>
+    T1D_HD static bool run_length(uint32_t W, uint32_t c) {
+        return KIND == kPassCU && c == 0x249u && !(W & 0x3FFFFu);
+    }
+
+    // Propagation (KIND kPassSP) or cleanup (kPassCU) symbols of a stripe, a zero-coding or run-length
+    // decision a turn.  While it is decoded the symbol that follows a 0 is made ready (next row or
+    // next column, its label and its context's state), which is most of a turn's latency; a 1 takes
+    // the slow way: sign, column word, and the next symbol anew.
     template <bool STYLED, int KIND>
     T1D_HD void decode_zc(uint32_t rv) {
-        enum : int { kZero = 0, kSign = 1, kRun = 2, kIndex1 = 3, kIndex2 = 4 };
         uint32_t next_set = S.colset(1, b);
         const uint32_t wide_hi = cw >= 64 ? ~0u : (cw > 32 ? (1u << (cw - 32)) - 1u : 0u);
-        uint32_t W = 0, carry = 0;
+        uint32_t carry = 0;  // what the column before leaves to the next one
         for (int h = 0; h < 2; ++h) {
+            const int x0 = 32 * h;
             uint32_t set = h ? next_set : S.colset(0, b), all = set;
             const uint32_t wide = h ? wide_hi : (cw >= 32 ? ~0u : (1u << cw) - 1u);
-            uint32_t c = 0, v = 0, pcx = 0;
-            int x = h ? -1 : -2, kind = kZero, k3 = 0;
-            uint32_t* at = nullptr;
-            while (set | c) {
-                if (!c) {
+            int x = h ? -1 : -2;
+            uint32_t W = 0, c = 0, v = 0;
+            // the next column that has a symbol (propagation: one reached by a carry may have none)
+            const auto fetch = [&]() {
+                do {
                     const int nx = ctz32(set);
                     set &= set - 1;
-                    at = &S.col(32 * h + nx, b);
-                    W = *at | (nx == x + 1 ? carry : 0u);
+                    W = mem.col(x0 + nx) | (nx == x + 1 ? carry : 0u);
                     x = nx;
                     carry = 0;
-                    v = 0;
-                    c = ~(W >> 4) & rv;
-                    if (KIND == kPassSP) {
-                        c &= near_rows(W);
-                        if (!c) *at = W & ~0x249u;  // (a column reached by a carry alone)
-                    } else {
-                        c &= ~spread4((W >> 23) & 15u);
-                        // run-length mode: four samples to code, no significant one around
-                        kind = c == 0x249u && !(W & 0x3FFFFu) ? kRun : kZero;
-                    }
-                }
-                if (c) {
-                    if (kind <= kRun && kind != kSign) k3 = ctz32(c);
-                    uint32_t cx = zc[(W >> k3) & 511u];
-                    if (kind != kZero) cx = kind == kRun ? 17u : pcx & 31u;
-                    uint32_t bit = dec<STYLED>(cx);
-                    bool ask = false;  // a sample turned significant: its sign is the next symbol
-                    if (kind == kZero) {
-                        if (KIND == kPassSP) v |= 1u << k3;
-                        ask = bit != 0;
-                        c &= c - 1;
-                    } else if (kind == kSign) {
-                        if (!(STYLED && raw)) bit ^= pcx >> 7;
-                        const int k = (k3 * 11) >> 5;
-                        W |= (16u << k3) | (bit << (23 + k));
-                        carry |= (8u << k3) | (bit << (18 + k));
-                        kind = kZero;
-                        if (KIND == kPassSP) {  // the next column has a candidate now
-                            const uint32_t nx = x < 31 ? (2u << x) & wide : 0u;
-                            set |= nx;
-                            all |= nx;
-                            if (x == 31 && h == 0) next_set |= 1u & wide_hi;
-                            c = ~(W >> 4) & near_rows(W) & rv;
+                    c = candidates<KIND>(W, rv);
+                    if (KIND == kPassSP && !c) mem.col_set(x0 + x, W & ~0x249u);
+                } while (KIND == kPassSP && !c && set);
+                v = 0;
+            };
+            const auto put = [&]() { mem.col_set(x0 + x, KIND == kPassSP ? (W & ~0x249u) | v : W); };
+            if (set) fetch();
+            if (c) {
+                bool run = run_length<KIND>(W, c);
+                int k3 = ctz32(c);
+                uint32_t cx = run ? 17u : mem.zc((W >> k3) & 511u);
+                MqdState e = mem.ctx(cx);
+                for (;;) {
+                    // the symbol after a 0: the column's next row, or the next column
+                    const uint32_t c2 = run ? 0u : c & (c - 1);
+                    const int nx = ctz32(set) & 31;
+                    const uint32_t Wn = mem.col(x0 + nx) | (nx == x + 1 ? carry : 0u);
+                    const uint32_t W2 = c2 ? W : Wn, d2 = c2 ? c2 : candidates<KIND>(Wn, rv);
+                    const int k32 = ctz32(d2) & 15;
+                    const bool run2 = !c2 && run_length<KIND>(Wn, d2);
+                    const uint32_t cx2 = run2 ? 17u : mem.zc((W2 >> k32) & 511u);
+                    MqdState e2 = mem.ctx(cx2);
+                    MqdState up;
+                    uint32_t moved;
+                    uint32_t bit = dec<STYLED>(cx, e, &up, &moved);
+                    if (KIND == kPassSP) v |= 1u << k3;
+                    if (!bit) {
+                        if (!c2) {
+                            put();
+                            if (!set) break;
+                            if (KIND == kPassSP && !d2) {  // reached by a carry, without a sample to code
+                                fetch();
+                                if (!c) break;
+                                k3 = ctz32(c);
+                                cx = mem.zc((W >> k3) & 511u);
+                                e = mem.ctx(cx);
+                                continue;
+                            }
+                            x = nx;
+                            set &= set - 1;
+                            v = 0;
+                            carry = 0;
                         }
-                        c &= 0x249u & (~1u << k3);  // rows below this one
-                    } else if (kind == kRun) {
-                        c = bit ? c : 0u;
-                        kind = bit ? kIndex1 : kZero;
-                        pcx = 18u;
-                    } else if (kind == kIndex1) {
-                        k3 = 6 * (int)bit;
-                        kind = kIndex2;
-                    } else {
-                        k3 += 3 * (int)bit;
-                        ask = true;
+                        const bool changed = cx2 == cx && moved != 0;
+                        e.x = changed ? up.x : e2.x;
+                        e.y = changed ? up.y : e2.y;
+                        W = W2;
+                        c = d2;
+                        k3 = k32;
+                        cx = cx2;
+                        run = run2;
+                        continue;
                     }
-                    if (ask) {
-                        const uint32_t y = W >> k3, z = W >> (18 + ((k3 * 11) >> 5));
-                        pcx = T->sc[(y & 0xAAu) | (z & 0x51u) | ((z >> 8) & 4u)];
-                        kind = kSign;
-                        c |= 0x80000000u;  // (the column is not done: bit 31 is no row)
+                    if (KIND == kPassCU && run) {  // the row of the first 1
+                        uint32_t k = 0;
+#pragma unroll 1
+                        for (int i = 0; i < 2; ++i) k = 2 * k + dec<STYLED>(18u);
+                        k3 = 3 * (int)k;
                     }
-                    if (!c) *at = KIND == kPassSP ? (W & ~0x249u) | v : W;
+                    const int k = (k3 * 11) >> 5;
+                    const uint32_t y = W >> k3, z = W >> (18 + k);
+                    const uint32_t sc = mem.sc((y & 0xAAu) | (z & 0x51u) | ((z >> 8) & 4u));
+                    uint32_t sg = dec<STYLED>(sc & 31u);
+                    if (!(STYLED && raw)) sg ^= sc >> 7;
+                    W |= (16u << k3) | (sg << (23 + k));
+                    carry |= (8u << k3) | (sg << (18 + k));
+                    if (KIND == kPassSP) {  // the next column has a candidate now
+                        const uint32_t add = x < 31 ? (2u << x) & wide : 0u;
+                        set |= add;
+                        all |= add;
+                        if (x == 31 && h == 0) next_set |= 1u & wide_hi;
+                        c = candidates<KIND>(W, rv);
+                    }
+                    c &= 0x249u & (~1u << k3);  // rows below this one
+                    run = false;
+                    if (!c) {
+                        put();
+                        if (!set) break;
+                        fetch();
+                        if (!c) break;
+                        run = run_length<KIND>(W, c);
+                    }
+                    k3 = ctz32(c);
+                    cx = run ? 17u : mem.zc((W >> k3) & 511u);
+                    e = mem.ctx(cx);
                 }
             }
             if (KIND == kPassSP) S.colset(h, b) = all;
@@ -450,28 +586,28 @@ struct StripeLane {
         if (STYLED && raw) {
             for (int i = 0; i < n; ++i) {
                 out |= (uint32_t)rd.bit() << (i & 31);
-                if ((i & 31) == 31 || i == n - 1) S.col(i >> 5, b) = out, out = 0;
+                if ((i & 31) == 31 || i == n - 1) mem.col_set(i >> 5, out), out = 0;
             }
             return;
         }
         if (n == 0) return;
-        uint32_t labels = S.col(0, b), cx = labels & 31u, e = S.ctx((int)cx, b);
+        uint32_t labels = mem.col(0), cx = labels & 31u;
+        MqdState e = mem.ctx(cx);
         for (int i = 0; i < n; ++i) {
             labels >>= 8;
-            if ((i & 3) == 3) labels = S.col(((i + 1) >> 2) & 63, b);
+            if ((i & 3) == 3) labels = mem.col(((i + 1) >> 2) & 63);
             const uint32_t ncx = min(labels & 31u, 18u);  // (past the last label: any context)
-            uint32_t ne = S.ctx((int)ncx, b), next;
-            int sh;
-            out |= m.decide(e, T->mq, &next, &sh) << (i & 31);
-            if (sh) {
-                S.ctx((int)cx, b) = next;
-                if (ncx == cx) ne = next;
-            }
+            const MqdState ne = mem.ctx(ncx);
+            MqdState up;
+            uint32_t moved;
+            out |= dec<false>(cx, e, &up, &moved) << (i & 31);
+            const bool changed = ncx == cx && moved != 0;
+            e.x = changed ? up.x : ne.x;
+            e.y = changed ? up.y : ne.y;
             cx = ncx;
-            e = ne;
-            if ((i & 31) == 31) S.col(i >> 5, b) = out, out = 0;
+            if ((i & 31) == 31) mem.col_set(i >> 5, out), out = 0;
         }
-        if (n & 31) S.col(n >> 5, b) = out;
+        if (n & 31) mem.col_set(n >> 5, out);
     }
 };
 
