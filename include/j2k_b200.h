@@ -78,7 +78,7 @@ enum {
                                  plane with the cluster barrier between levels.  0 (default): off */
     J2K_TUNE_T1D_LANES = 10,  /* tier-1 decoder: code-blocks decoded side by side in one warp, one per lane:
                                  0 (one), 2, 4, 8, 16; 3, 6 and 32 run as 4, 8 and 16.  Left alone, it is 1,
-                                 2 or 4 by the number of blocks */
+                                 2 or 4 by the number of samples */
     J2K_TUNE_T1D_STEPS = 11,  /* 1: with 8, 16 or 32 lanes, unstyled blocks are decoded in a loop of one
                                  symbol per step over 64-bit row masks; 0 (default): stripe by stripe */
     J2K_TUNE_PLANAR = 12,     /* interleaved-to-planar split of contiguous images: 0: 16 pixels per thread;

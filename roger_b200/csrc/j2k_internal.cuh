@@ -86,7 +86,7 @@ struct j2k_ctx {
     int dwt_tma = 0;             // fast forward DWT: strips staged by TMA tensor copies (persistent CTAs)
     int t1a_ctas = 2;            // tier-1 phase A: resident CTAs per SM its registers are cut for (2 or 3)
     int dwt_tail = 0;            // forward DWT: deep levels in one launch (1 cooperative, 2..5 clusters)
-    int t1d_lanes = -1;          // tier-1 decoder: code-blocks per warp (0: one), -1: by the number of blocks
+    int t1d_lanes = -1;          // tier-1 decoder: code-blocks per warp (0: one), -1: by the number of samples
     int t1d_steps = 0;           // tier-1 decoder: unstyled blocks by the one-symbol-per-step loop
     int planar_form = 1;         // planar split: 0 16 pixels per thread; 1 / 2: 4 pixels per thread and step
     int dwt97_rows = 1;          // differentiable 9/7: levels 64..1024 wide (powers of two) as full-row bands
@@ -261,9 +261,10 @@ struct j2k_pcrd_hulls {
 constexpr int J2K_TRUNC_EXTRA = 4;  // bytes kept beyond those produced at a plane end
 // style / pass_ends (device, J2K_PASS_STRIDE per job) locate the codeword segments of styled
 // blocks; style 0 decodes one segment of descs[i].length bytes.  job_style (device, one byte per
-// job, optional) gives each job its own style (pass ends then needed for every job).
+// job, optional) gives each job its own style (pass ends then needed for every job).  samples: the
+// samples of all jobs together (the kernel's launch shape follows from it).
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
-                              const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff,
+                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int32_t* coeff,
                               cudaStream_t st, int style = 0, const uint32_t* pass_ends = nullptr,
                               const uint8_t* job_style = nullptr);
 

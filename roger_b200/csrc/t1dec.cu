@@ -8,8 +8,8 @@
 // cycles a symbol with one block per warp), and with 4 blocks per warp the ALU pipe, since the lanes
 // are at different kinds of symbols (1.74 times the instructions of one).  Round trips host to host
 // on B200, against a decoder whose lanes kept 64-bit row masks and gathered each column's
-// neighbourhood themselves: 512 x 512 gray 15.3 -> 5.7 ms, 2048 x 2048 colour 18.8 -> 10.5 ms,
-// 4096 x 4096 colour 28.2 -> 21.8 ms.
+// neighbourhood themselves: 512 x 512 gray 15.3 -> 5.5 ms, 2048 x 2048 colour 18.8 -> 10.5 ms,
+// 4096 x 4096 colour 28.5 -> 20.5 ms.
 // The warp clears its blocks' output regions first and applies the signs at the end; magnitude bits
 // go to the output plane by fire-and-forget atomic ORs (each block owns its region).
 #include <atomic>
@@ -301,14 +301,16 @@ __host__ __device__ constexpr size_t stripe_smem_bytes(int warps) {
 }
 
 // L code-blocks per warp, one per lane (t1dec_stripe.cuh).  Groups of L consecutive blocks of
-// `order` (longest codewords first) go to the warps of all CTAs in turn, then from a queue.
+// `order` (longest codewords first) go to the warps of all CTAs in turn, then from a queue.  Blocks
+// of more than half the longest codeword (keys: the lengths in that order) get a warp of their own,
+// at most `alone` of them: a block runs fastest alone, and the others end before it anyway.
 template <bool STYLED, int L>
 __global__ void __launch_bounds__(32 * stripe_warps<L>(), 1)
 t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __restrict__ bytes,
                         const j2k_cb_job* __restrict__ jobs, int njobs, int32_t* __restrict__ coeff,
                         uint32_t* __restrict__ err, int style, const uint32_t* __restrict__ pass_ends,
                         const uint8_t* __restrict__ job_style, const uint32_t* __restrict__ order,
-                        uint32_t* __restrict__ queue) {
+                        const uint32_t* __restrict__ keys, int alone, uint32_t* __restrict__ queue) {
     extern __shared__ __align__(16) uint8_t dsm[];
     StripeTables& tabs = *reinterpret_cast<StripeTables*>(dsm);
     for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) fill_stripe_tables_entry(tabs, i);
@@ -316,9 +318,23 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const StripeState<L> S{reinterpret_cast<uint32_t*>(dsm + kStripeTablesBytes) + wid * stripe_state_words<L>()};
     constexpr int R = (8 * L + 31) / 32;  // rounds of 32 (block, word) items per stripe
-    const int ngroups = (njobs + L - 1) / L;
+    if (L > 1 && alone > 0) {  // the number of leading keys above half the first one
+        const uint32_t half = keys[0] / 2;
+        int lo = 0, hi = alone;  // it is in lo..hi
+        while (lo < hi) {
+            const int step = (hi - lo + 31) / 32, at = lo + lane * step;  // keys[lo], keys[lo + step], ...
+            const unsigned above = __ballot_sync(~0u, at < hi && keys[at] > half);
+            const int n = __popc(above);  // (a run of ones from bit 0: the keys fall)
+            if (n == 0) break;
+            const int last = lo + (n - 1) * step;  // above half; the next probe is not
+            hi = min(hi, last + step);
+            lo = last + 1;
+        }
+        alone = lo;
+    }
+    const int ngroups = alone + (njobs - alone + L - 1) / L;
     for (int g = wid * (int)gridDim.x + (int)blockIdx.x; g < ngroups;) {
-        const int j0 = g * L, nb = min(L, njobs - j0);
+        const int j0 = g < alone ? g : alone + (g - alone) * L, nb = g < alone ? 1 : min(L, njobs - j0);
         j2k_cb_job J{};
         j2k_cb_desc D{};
         bool ok = false;
@@ -803,7 +819,8 @@ extern "C" int j2k_t1_decode_block_styled_host(const uint8_t* data, int len, con
 template <bool STYLED, int L>
 static j2k_status launch_stripe(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs, const uint8_t* bytes,
                                 const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff, int style,
-                                const uint32_t* pass_ends, const uint8_t* job_style, const uint32_t* order) {
+                                const uint32_t* pass_ends, const uint8_t* job_style, const uint32_t* order,
+                                const uint32_t* keys) {
     static std::atomic<uint64_t> attr_set{0};  // devices whose attribute is set, per instantiation
     const uint64_t bit = 1ull << (ctx->device & 63);
     if (!(attr_set.load() & bit)) {
@@ -816,11 +833,14 @@ static j2k_status launch_stripe(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc
     if (!queue) return J2K_ERR_OUT_OF_MEMORY;
     J2K_CUDA(ctx, cudaMemsetAsync(queue, 0, 4, st));
     // the groups spread over the SMs first, then over the warps of a CTA
-    const size_t groups = (njobs + L - 1) / L, sms = (size_t)ctx->sm_count;
+    const size_t sms = (size_t)ctx->sm_count, resident = sms * stripe_warps<L>();
+    // blocks that can have a warp alone with all blocks still resident at once
+    const size_t alone = L > 1 && keys && resident * L > njobs ? std::min(njobs, (resident * L - njobs) / (L - 1)) : 0;
+    const size_t groups = alone + (njobs - alone + L - 1) / L;
     const unsigned grid = (unsigned)std::min(groups, sms);
     const int warps = (int)std::min<size_t>((groups + grid - 1) / grid, (size_t)stripe_warps<L>());
     t1_decode_stripe_kernel<STYLED, L><<<grid, 32 * warps, stripe_smem_bytes<L>(warps), st>>>(
-        descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err, style, pass_ends, job_style, order, queue);
+        descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err, style, pass_ends, job_style, order, keys, (int)alone, queue);
     J2K_CUDA(ctx, cudaGetLastError());
     return J2K_OK;
 }
@@ -837,7 +857,9 @@ __global__ void t1d_order_keys(const j2k_cb_desc* __restrict__ descs, int n, uin
 
 // The jobs sorted by codeword length, longest first (a stable radix sort: equal lengths keep
 // their list order), in scratch; nullptr with the error set when scratch runs out.
-static const uint32_t* decode_order(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs, size_t njobs) {
+// *keys: the lengths in that order.
+static const uint32_t* decode_order(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs, size_t njobs,
+                                    const uint32_t** keys) {
     const int n = (int)njobs;
     size_t tmp = 0;
     cub::DeviceRadixSort::SortPairsDescending(nullptr, tmp, (const uint32_t*)nullptr, (uint32_t*)nullptr,
@@ -853,6 +875,7 @@ static const uint32_t* decode_order(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_
                                                                       n, 0, 32, st),
                        "decode order sort") != J2K_OK)
         return nullptr;
+    *keys = keys_out;
     return ids_out;
 }
 
@@ -874,21 +897,21 @@ static j2k_status launch_steps(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc*
     return J2K_OK;
 }
 
-// Blocks per warp: the fewest with which all blocks are resident at once (16, 40 and 84 blocks an
-// SM with 1, 2 and 4 per warp), since a block alone in its warp runs fastest and a second wave
-// costs as much as the first, and 4 for more.  Round trips host to host on B200, 1 / 2 / 4 / 8
-// blocks per warp: 70 blocks of a 512 x 512 gray image 5.7 / 7.6 / 10.2 / 14.2 ms, 777 blocks
-// (1024 x 1024 colour) 6.8 / 8.4 / 10.4 / 15.5, 3072 blocks (2048 x 2048 colour) 12.5 / 10.5 /
-// 11.8 / 15.5, 12288 blocks (4096 x 4096 colour) 43 / 32 / 21.8 / 22.0.
-static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t njobs) {
-    const size_t sms = (size_t)ctx->sm_count;
-    for (int l : {1, 2})
-        if (njobs <= sms * l * (l == 1 ? stripe_warps<1>() : stripe_warps<2>())) return l;
-    return 4;
+// Blocks per warp by the work there is, as a number of full blocks of 4096 samples: one while those
+// would be resident at once that way (16 an SM), two up to 40 an SM, four for more (the long blocks
+// get warps of their own as far as all still fit).  A block runs fastest alone; sharing a warp saves
+// instructions, which counts once the ALU pipes are full.  Host to host on B200, 1 / 2 / 4 / 8 blocks
+// per warp: 70 blocks of a 512 x 512 gray image 5.5 ms, with two 7.6, four 10.2; 777 of 1024 x 1024
+// colour 6.7, 8.4, 10.4; 24 images of mixed sizes and block sizes (5071 blocks, the work of 1590)
+// 11.0 / 11.2 / 13.6 / 17.5; 3072 blocks of 2048 x 2048 colour 12.4 / 10.0 / 11.1 / 13.9; 12288 blocks
+// of 4096 x 4096 colour 42 / 32 / 20.0 / 21.6.
+static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t samples) {
+    const size_t full = samples / 4096, sms = (size_t)ctx->sm_count;
+    return full <= 16 * sms ? 1 : (full <= 40 * sms ? 2 : 4);
 }
 
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
-                              const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff,
+                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int32_t* coeff,
                               cudaStream_t st, int style, const uint32_t* pass_ends, const uint8_t* job_style) {
     if (njobs == 0) return J2K_OK;
     if ((style || job_style) && !pass_ends)
@@ -903,23 +926,23 @@ j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint
         default: break;
         }
     }
-    const int L = forced < 0 ? stripe_blocks_per_warp(ctx, njobs)
+    const int L = forced < 0 ? stripe_blocks_per_warp(ctx, samples)
                              : (forced <= 1 ? 1 : (forced == 2 ? 2 : (forced <= 4 ? 4 : (forced <= 8 ? 8 : 16))));
-    const uint32_t* ord = nullptr;
+    const uint32_t *ord = nullptr, *keys = nullptr;
     if (ctx->t1d_order && njobs > (size_t)L) {
-        ord = decode_order(ctx, st, descs, njobs);
+        ord = decode_order(ctx, st, descs, njobs, &keys);
         if (!ord) return J2K_ERR_OUT_OF_MEMORY;
     }
     switch ((styled ? 100 : 0) + L) {
-    case 1: return launch_stripe<false, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 2: return launch_stripe<false, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 4: return launch_stripe<false, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 8: return launch_stripe<false, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 16: return launch_stripe<false, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord);
-    case 101: return launch_stripe<true, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 102: return launch_stripe<true, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 104: return launch_stripe<true, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    case 108: return launch_stripe<true, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
-    default: return launch_stripe<true, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord);
+    case 1: return launch_stripe<false, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
+    case 2: return launch_stripe<false, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
+    case 4: return launch_stripe<false, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
+    case 8: return launch_stripe<false, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
+    case 16: return launch_stripe<false, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
+    case 101: return launch_stripe<true, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
+    case 102: return launch_stripe<true, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
+    case 104: return launch_stripe<true, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
+    case 108: return launch_stripe<true, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
+    default: return launch_stripe<true, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
     }
 }
