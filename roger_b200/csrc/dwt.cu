@@ -1397,6 +1397,7 @@ j2k_status inv_levels(j2k_ctx* ctx, const void* in, size_t in_pitch, void* out, 
     // even levels >= 2 use ll1 (level-2 size)
     const size_t z0 = (size_t)ws[1] * hs[1];
     const size_t z1 = levels >= 2 ? (size_t)ws[2] * hs[2] : 0;
+    bool after_fast = false;  // the level before this one ran the strip kernel
     for (int k = levels - 1; k >= 0; --k) {
         int cw = ws[k], chh = hs[k];
         dim3 grid((cw + TW - 1) / TW, (chh + TH - 1) / TH, n);
@@ -1419,23 +1420,28 @@ j2k_status inv_levels(j2k_ctx* ctx, const void* in, size_t in_pitch, void* out, 
                             ((wl & 1) == 0);
             const dim3 fg((cw + FTW - 1) / FTW, (chh + STH - 1) / STH, n);
             const SynExtra ex{};
-            // (not programmatic dependents: these kernels read their input through the read-only
-            // cache, which the previous level writes)
+            // every level after the deepest is a programmatic dependent of the one before, so its
+            // launch overlaps the previous level's last CTAs
+            const bool pdl = after_fast;
+            after_fast = true;
             const dim3 b(256);
             cudaError_t le;
             if (deq) {
                 if (k == levels - 1)
-                    le = launch_pdl(dwt_syn_fast<KERN, 0, int32_t, true, true, 0>, fg, b, stream, false,
+                    le = launch_pdl(dwt_syn_fast<KERN, 0, int32_t, true, true, 0>, fg, b, stream, pdl,
                                     (const int32_t*)in, in_pitch, lls, llp, cw, chh, o, op, st, zs, vec, ex);
                 else
-                    le = launch_pdl(dwt_syn_fast<KERN, 0, int32_t, true, false, 0>, fg, b, stream, false,
+                    le = launch_pdl(dwt_syn_fast<KERN, 0, int32_t, true, false, 0>, fg, b, stream, pdl,
                                     (const int32_t*)in, in_pitch, lls, llp, cw, chh, o, op, st, zs, vec, ex);
             } else {
-                le = launch_pdl(dwt_syn_fast<KERN, 0, T, false, false, 0>, fg, b, stream, false, (const T*)in,
+                le = launch_pdl(dwt_syn_fast<KERN, 0, T, false, false, 0>, fg, b, stream, pdl, (const T*)in,
                                 in_pitch, lls, llp, cw, chh, o, op, st, zs, vec, ex);
             }
             J2K_CUDA(ctx, le);
-        } else if (deq) {
+            continue;
+        }
+        after_fast = false;
+        if (deq) {
             if (k == levels - 1)
                 dwt_inv_level<KERN, ORDER, TW, TH, int32_t, true, true><<<grid, 256, 0, stream>>>(
                     (const int32_t*)in, in_pitch, lls, llp, cw, chh, o, op, st, zs);

@@ -306,7 +306,7 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
         const bool colok = t >= 4 && t < 252 && x < w;
 #pragma unroll
         for (int j = 0; j < STH; ++j)
-            sb[j] = (colok && y0 + j < h) ? __ldg(sub + (size_t)(y0 + j) * ex.sub_pitch + x) : 0.0f;
+            sb[j] = (colok && y0 + j < h) ? __ldcg(sub + (size_t)(y0 + j) * ex.sub_pitch + x) : 0.0f;
     }
     // 1. the strip's rows y0 - HV + r (mirrored, or zero outside the level for MODE 1), warp w
     //    taking rows w, w + 8, ...: lane l loads the band samples of natural columns
@@ -330,10 +330,12 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
                                    ? reinterpret_cast<const uint32_t*>(ll_src + (size_t)(gy >> 1) * llpitch)
                                    : srow;
         if (inner_x && vec_in) {
-            const uint2 l0 = __ldg(reinterpret_cast<const uint2*>(lsrc + lx));
-            const uint2 l1 = __ldg(reinterpret_cast<const uint2*>(lsrc + lx + 2));
-            const uint2 h0 = __ldg(reinterpret_cast<const uint2*>(srow + wl + lx));
-            const uint2 h1 = __ldg(reinterpret_cast<const uint2*>(srow + wl + lx + 2));
+            // (L2 only, as in the forward levels: a level launched as a dependent may start while the
+            // previous one runs, so an SM's L1 could still hold lines of its input buffer)
+            const uint2 l0 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx));
+            const uint2 l1 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx + 2));
+            const uint2 h0 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx));
+            const uint2 h1 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx + 2));
             rl[i][0] = l0.x; rl[i][1] = l0.y; rl[i][2] = l1.x; rl[i][3] = l1.y;
             rh[i][0] = h0.x; rh[i][1] = h0.y; rh[i][2] = h1.x; rh[i][3] = h1.y;
         } else {
@@ -344,8 +346,8 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
                     ge = mirror(ge, w);
                     go = mirror(go, w);
                 }
-                if (ge >= 0 && ge < w) rl[i][k] = __ldg(lsrc + (ge >> 1));
-                if (go >= 0 && go < w) rh[i][k] = __ldg(srow + wl + (go >> 1));
+                if (ge >= 0 && ge < w) rl[i][k] = __ldcg(lsrc + (ge >> 1));
+                if (go >= 0 && go < w) rh[i][k] = __ldcg(srow + wl + (go >> 1));
             }
         }
     }
