@@ -117,6 +117,39 @@ struct MqCoder {
         A = mq_float((m & 0x7FFFFFu) | kMqExp);
         return kMqExp - (m & 0x7F800000u);
     }
+    // Takes the bytes out of c, a C that has been shifted -ct times since the first of them was due;
+    // false, with everything as it was, when a byte read late may have been 0xFF when it was due.
+    MQ_HD bool bytes_late(uint64_t c, int ct) {
+        const uint32_t B0 = B, w0 = wacc;
+        const int cnt0 = cnt;
+        const bool ovf0 = ovf;
+        bool doubt = false;
+        do {
+            const int k = -ct;  // shifts since the byte was due (additions without a shift may follow)
+            const uint32_t ck = (uint32_t)(c >> k);
+            const bool carry = B != 0xFFu && (ck >> 27) != 0;
+            B += carry ? 1u : 0u;
+            const bool ff = B == 0xFFu;
+            const int low = ff ? 20 : 19;
+            const uint32_t v = (carry ? ck & 0x7FFFFFFu : ck) >> low;
+            doubt |= v == 0 || (ck >> 28) != 0;
+            push();
+            ++cnt;
+            B = v & 0xFFu;
+            c &= ((uint64_t)1 << (low + k)) - 1;
+            ct += ff ? 7 : 8;
+        } while (ct <= 0);
+        if (doubt) {
+            B = B0;
+            wacc = w0;
+            cnt = cnt0;
+            ovf = ovf0;
+            return false;
+        }
+        C = (uint32_t)c;
+        CT = ct;
+        return true;
+    }
     // code part of four symbols: values a added, shifts s
     MQ_HD void code4(const uint32_t (&a)[4], const int (&s)[4]) {
         const int S = s[0] + s[1] + s[2] + s[3];
@@ -126,40 +159,12 @@ struct MqCoder {
             CT -= S;
             return;
         }
-        bool exact = S > 32;
-        if (!exact) {
+        if (S <= 32) {
             uint64_t c = ((uint64_t)(C + a[0]) << s[0]) + a[1];
             c = (c << s[1]) + a[2];
             c = (c << s[2]) + a[3];
             c <<= s[3];
-            const uint32_t B0 = B, w0 = wacc;
-            const int cnt0 = cnt;
-            const bool ovf0 = ovf;
-            int ct = CT - S;
-            do {
-                const int k = -ct;  // shifts since the byte was due (additions without a shift may follow)
-                const uint32_t ck = (uint32_t)(c >> k);
-                const bool carry = B != 0xFFu && (ck >> 27) != 0;
-                B += carry ? 1u : 0u;
-                const bool ff = B == 0xFFu;
-                const int low = ff ? 20 : 19;
-                const uint32_t v = (carry ? ck & 0x7FFFFFFu : ck) >> low;
-                exact |= v == 0 || (ck >> 28) != 0;
-                push();
-                ++cnt;
-                B = v & 0xFFu;
-                c &= ((uint64_t)1 << (low + k)) - 1;
-                ct += ff ? 7 : 8;
-            } while (ct <= 0);
-            if (!exact) {
-                C = (uint32_t)c;
-                CT = ct;
-                return;
-            }
-            B = B0;
-            wacc = w0;
-            cnt = cnt0;
-            ovf = ovf0;
+            if (bytes_late(c, CT - S)) return;
         }
 #ifdef __CUDA_ARCH__
 #pragma unroll 1
@@ -168,6 +173,33 @@ struct MqCoder {
             C += j == 0 ? a[0] : (j == 1 ? a[1] : (j == 2 ? a[2] : a[3]));
             shift(j == 0 ? s[0] : (j == 1 ? s[1] : (j == 2 ? s[2] : s[3])));
         }
+    }
+    // code part of eight symbols, each an addition | shifts << 16; each half's additions are summed
+    // by themselves (32 bits hold them up to 15 shifts) before C comes in.  False where the symbols
+    // have to be coded one by one.
+    MQ_HD bool code8(const uint32_t (&e)[8]) {
+        uint32_t P[2] = {0, 0};
+        int S[2] = {0, 0};
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int j = 0; j < 4; ++j)
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t v = e[4 * h + j];
+                P[h] = (P[h] + (v & 0xFFFFu)) << (v >> 16);
+                S[h] += (int)(v >> 16);
+            }
+        const int both = S[0] + S[1];
+        if (both < CT) {
+            C = (((C << S[0]) + P[0]) << S[1]) + P[1];
+            CT -= both;
+            return true;
+        }
+        if (S[0] > 15 || S[1] > 15) return false;
+        return bytes_late(((uint64_t)C << both) + ((uint64_t)P[0] << S[1]) + P[1], CT - both);
     }
     // FLUSH (C.2.9); a last byte of 0xFF is dropped.  Returns the codeword's length.
     MQ_HD int flush() {

@@ -199,12 +199,13 @@ struct MqPlaneEnds {
 
 // One block per lane of a warp pair (mq_enc.cuh): warp 0 runs the interval part and puts four
 // symbols' additions and shifts into a ring in shared memory, warp 1 takes them through the code
-// part a chunk of 16 symbols behind.  The two parts are serial chains of their own, so a symbol
-// costs the longer one instead of both.  Bound by the interval chain: 34 instructions and 85 cycles
-// a symbol for a block alone in its pair, about 145 with 32 blocks.  One warp with both parts takes
-// 104 and 165 cycles: whole encodes of a 512 x 512 gray image 1.9 ms against 1.58 with pairs, of a
-// 4096 x 4096 colour image 4.1 against 3.7.  An integer coder with a leading-zero count and a branch
-// to the byte output in every symbol's chain took over 200 cycles (2.8 and 6.0 ms).
+// part eight at a time, a chunk of 16 symbols behind.  The two parts are serial chains of their own,
+// so a symbol costs the longer one instead of both.  Bound by the interval chain: 34 instructions and
+// 78 cycles a symbol for a block alone in its pair, about 100 with 32 blocks (taking the bytes out
+// four symbols at a time made the code warp the slower one there, 145).  One warp with both parts
+// took 104 and 165 cycles; an integer coder with a leading-zero count and a branch to the byte output
+// in every symbol's chain over 200.  4096 blocks of a 4096 x 4096 gray image, 32 to a pair: 1.57 ms,
+// 2.32 with the bytes taken out by fours, 2.44 with one warp.
 // RATE: also record the plane ends (MqPlaneEnds) into plane_bytes[job * 32 + k].
 template <bool RATE>
 __global__ void __launch_bounds__(2 * kMqThreads)
@@ -281,16 +282,23 @@ t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jo
         ends.start();
         while (ends.next() == 0u) ends.at(e);  // passes with no symbols at all
     }
-    MqNoEnds none;
     for (int k = 0; k < chunks; ++k) {
         __syncthreads();  // chunk k is in the ring; the interval warp goes on with chunk k + 1
 #pragma unroll 1
-        for (int q = 0; q < 4 && 16 * k + 4 * q < n; ++q) {
+        for (int q = 0; q < 4 && 16 * k + 4 * q < n; q += 2) {
+            const int at = 16 * k + 4 * q;
             const uint4 r = ring[k & 1][q][lane];
-            const uint32_t a[4] = {r.x & 0xFFFFu, r.y & 0xFFFFu, r.z & 0xFFFFu, r.w & 0xFFFFu};
-            const int s[4] = {(int)(r.x >> 16), (int)(r.y >> 16), (int)(r.z >> 16), (int)(r.w >> 16)};
-            if (RATE) mq_code_group(e, a, s, (uint32_t)(16 * k + 4 * q), ends);
-            else mq_code_group(e, a, s, (uint32_t)(16 * k + 4 * q), none);
+            uint4 t = ring[k & 1][q + 1][lane];
+            if (at + 4 >= n) t = make_uint4(0, 0, 0, 0);  // not written: the block has ended
+            const uint32_t ev[8] = {r.x, r.y, r.z, r.w, t.x, t.y, t.z, t.w};
+            if ((!RATE || ends.next() > (uint32_t)at + 8u) && e.code8(ev)) continue;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                e.C += ev[j] & 0xFFFFu;
+                e.shift((int)(ev[j] >> 16));
+                if (RATE)
+                    while (ends.next() == (uint32_t)(at + j + 1)) ends.at(e);
+            }
         }
     }
     if (!live) return;
@@ -820,11 +828,11 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
         left -= std::min(left, wk * l);
         warps += wk;
     }
-    // blocks per pair after the tiers: two more pairs per SM hold the rest, up to full warps.  Whole
-    // encodes on B200 after a tier of one block per SM, by blocks per pair: 777 blocks 1 2.68, 2 2.12,
-    // 4 2.08 ms; 3072 blocks 4 3.26, 8 2.85, 12 2.77; 12288 blocks 8 6.8, 16 5.6, 24 and 32 4.8 (before
-    // the context modelling took a third of that)
-    const size_t per = 2 * (size_t)ctx->sm_count;
+    // blocks per pair after the tiers: one more pair per SM holds the rest (a scheduler for each of
+    // the warps of two pairs per SM), up to full warps.  Whole encodes on B200 after a tier of one
+    // block per SM: 777 blocks with 2 a pair 1.84, with 16 or 32 1.57 ms; 3072 blocks with 10 2.03,
+    // with 32 1.82; 12288 blocks with 16 4.1, with 32 2.94
+    const size_t per = (size_t)ctx->sm_count;
     const int lanes = ctx->mq_lanes ? ctx->mq_lanes : (int)std::min<size_t>(std::max<size_t>((left + per - 1) / per, 1), 32);
     warps += (left + lanes - 1) / lanes;
     const auto mq = rate ? t1_mq_kernel<true> : t1_mq_kernel<false>;
