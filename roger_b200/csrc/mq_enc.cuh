@@ -1,4 +1,4 @@
-// The MQ encoder of one lane (T.800 C.2), in two parts that meet every four symbols.
+// The MQ encoder of one lane (T.800 C.2), in two parts that meet every eight symbols.
 //
 // Interval part.  A, Qe and the comparisons of the conditional exchange are kept as floats: A is
 // the float whose value is the 16-bit register (0x8000 <= A < 0x10000, so its exponent field is
@@ -12,7 +12,7 @@
 // The sign rides along in Qe's sign bit.  The chain from symbol to symbol is then three
 // operations: restore the exponent, multiply-add, maximum.
 //
-// Code part.  The four pairs (value added to C, shifts) of a group are folded into C in one go, and
+// Code part.  The eight pairs (value added to C, shifts) of a group are folded into C in one go, and
 // the bytes that became due are taken from a 64-bit C afterwards.  A byte taken late already holds
 // the carry of the additions after it, which T.800 would add to it one byte later; the result is
 // the same unless the byte was 0xFF when it was due (then the carry stays in the next byte's stuffed
@@ -150,30 +150,6 @@ struct MqCoder {
         CT = ct;
         return true;
     }
-    // code part of four symbols: values a added, shifts s
-    MQ_HD void code4(const uint32_t (&a)[4], const int (&s)[4]) {
-        const int S = s[0] + s[1] + s[2] + s[3];
-        if (S < CT) {  // no byte is due
-            C = ((((((C + a[0]) << s[0]) + a[1]) << s[1]) + a[2]) << s[2]) + a[3];
-            C <<= s[3];
-            CT -= S;
-            return;
-        }
-        if (S <= 32) {
-            uint64_t c = ((uint64_t)(C + a[0]) << s[0]) + a[1];
-            c = (c << s[1]) + a[2];
-            c = (c << s[2]) + a[3];
-            c <<= s[3];
-            if (bytes_late(c, CT - S)) return;
-        }
-#ifdef __CUDA_ARCH__
-#pragma unroll 1
-#endif
-        for (int j = 0; j < 4; ++j) {
-            C += j == 0 ? a[0] : (j == 1 ? a[1] : (j == 2 ? a[2] : a[3]));
-            shift(j == 0 ? s[0] : (j == 1 ? s[1] : (j == 2 ? s[2] : s[3])));
-        }
-    }
     // code part of eight symbols, each an addition | shifts << 16; each half's additions are summed
     // by themselves (32 bits hold them up to 15 shifts) before C comes in.  False where the symbols
     // have to be coded one by one.
@@ -201,6 +177,16 @@ struct MqCoder {
         if (S[0] > 15 || S[1] > 15) return false;
         return bytes_late(((uint64_t)C << both) + ((uint64_t)P[0] << S[1]) + P[1], CT - both);
     }
+    // the same one by one
+    MQ_HD void code_each(const uint32_t (&e)[8]) {
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+        for (int j = 0; j < 8; ++j) {
+            C += e[j] & 0xFFFFu;
+            shift((int)(e[j] >> 16));
+        }
+    }
     // FLUSH (C.2.9); a last byte of 0xFF is dropped.  Returns the codeword's length.
     MQ_HD int flush() {
         const uint32_t a = ((mq_bits(A) & 0x7FFFFFu) | 0x800000u) >> 8;
@@ -220,11 +206,6 @@ struct MqCoder {
         }
         return cnt - (B == 0xFFu ? 1 : 0);
     }
-};
-
-struct MqNoEnds {
-    MQ_HD uint32_t next() const { return 0xFFFFFFFFu; }
-    MQ_HD void at(const MqCoder&) {}
 };
 
 #ifdef __CUDA_ARCH__
@@ -325,68 +306,35 @@ struct MqSymbols {
             cx = ncx;
         }
     }
-    // all symbols in order: each(w, wnext, left, number of the first) for every four
-    template <class Group>
-    MQ_HD void walk(Group each) {
-        int k = 0;
-        for (; 16 * k + 16 <= n; ++k) {
-            const uint4 c = next(k);
-            uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w;
-#ifdef __CUDA_ARCH__
-#pragma unroll 1
-#endif
-            for (int q = 0; q < 4; ++q) {
-                each(wa, wb, 4, 16 * k + 4 * q);
-                wa = wb;
-                wb = wc;
-                wc = wd;
-                wd = c0.x;
-            }
-        }
-        uint32_t wa = c0.x, wb = c0.y, wc = c0.z, wd = c0.w;
-#ifdef __CUDA_ARCH__
-#pragma unroll 1
-#endif
-        for (int i = 16 * k; i < n; i += 4) {
-            each(wa, wb, n - i, i);
-            wa = wb;
-            wb = wc;
-            wc = wd;
-        }
-    }
 };
 
-// The code part of four symbols that follow symbol `done`; ends.at() is called after symbol i - 1
-// wherever ends.next() == i.
-template <class Ends>
-MQ_HD void mq_code_group(MqCoder& e, const uint32_t (&a)[4], const int (&s)[4], uint32_t done, Ends& ends) {
-    if (ends.next() > done + 4u) {
-        e.code4(a, s);
-    } else {  // a plane ends in this group: symbol by symbol
+// Both parts by one lane
+template <int SHIFT>
+MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, MqMem<SHIFT> mem) {
+    MqSymbols<SHIFT> src(syms, n, mem);
+    for (int k = 0; k < src.nchunks; ++k) {
+        const uint4 c = src.next(k);
+        uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w, ev[8];
+        const auto put = [&](int j, uint32_t add, uint32_t moved) { ev[j] = add | (moved >> 7); };
+        const auto put4 = [&](int j, uint32_t add, uint32_t moved) { ev[4 + j] = add | (moved >> 7); };
 #ifdef __CUDA_ARCH__
-#pragma unroll
+#pragma unroll 1
 #endif
-        for (int j = 0; j < 4; ++j) {
-            e.C += a[j];
-            e.shift(s[j]);
-            while (ends.next() == done + j + 1u) ends.at(e);
+        for (int i = 16 * k; i < 16 * k + 16 && i < n; i += 8) {
+            if (n - i >= 8) {
+                src.group(e, wa, wb, 4, put);
+                src.group(e, wb, wc, 4, put4);
+            } else {
+                ev[4] = ev[5] = ev[6] = ev[7] = 0;
+                src.group(e, wa, wb, n - i, put);
+                if (n - i > 4) src.group(e, wb, wc, n - i - 4, put4);
+            }
+            if (!e.code8(ev)) e.code_each(ev);
+            wa = wc;
+            wb = wd;
+            wc = src.c0.x;
         }
     }
-}
-
-// Both parts by one lane
-template <int SHIFT, class Ends>
-MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, MqMem<SHIFT> mem, Ends& ends) {
-    MqSymbols<SHIFT> src(syms, n, mem);
-    src.walk([&](uint32_t w, uint32_t wnext, int left, int done) {
-        uint32_t a[4];
-        int s[4];
-        src.group(e, w, wnext, left, [&](int j, uint32_t add, uint32_t moved) {
-            a[j] = add;
-            s[j] = (int)(moved >> 23);
-        });
-        mq_code_group(e, a, s, (uint32_t)done, ends);
-    });
 }
 
 MQ_HD MqState mq_table_entry(uint32_t qe, uint32_t nmps, uint32_t nlps, uint32_t sw, uint32_t mps) {

@@ -593,8 +593,7 @@ t1_mq_pass_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict
         reset_mq_states(st, kPassThreads, tab);
         MqCoder e;
         e.init(reinterpret_cast<uint32_t*>(segs + base), (int)(lim - base));
-        MqNoEnds ends;
-        mq_encode(e, syms + J.sym_off + s0, n, MqMem<7>(st, tab), ends);
+        mq_encode(e, syms + J.sym_off + s0, n, MqMem<7>(st, tab));
         len = (uint32_t)e.flush();
         ovf = e.ovf;
     }

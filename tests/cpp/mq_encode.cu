@@ -112,8 +112,7 @@ int main(int argc, char** argv) {
         st[18] = tab[92];
         MqCoder e;
         e.init(out.data(), (int)out.size() * 4);
-        MqNoEnds ends;
-        mq_encode(e, sym, n, MqMem<0>(st, tab), ends);
+        mq_encode(e, sym, n, MqMem<0>(st, tab));
         const int len = n ? e.flush() : 0;
         if (e.ovf || len != (int)f.b.size() || std::memcmp(out.data(), f.b.data(), (size_t)len) != 0) {
             std::printf("stream %d of %d symbols differs\n", it, n);
@@ -130,16 +129,16 @@ int main(int argc, char** argv) {
         std::fill(out.begin(), out.begin() + f.b.size() / 4 + 1, 0u);
         std::vector<uint32_t> ev(n + 16, 0);
         MqSymbols<0> src(sym, n, MqMem<0>(st, tab));
-        src.walk([&](uint32_t w, uint32_t wnext, int left, int done) {
-            src.group(iv, w, wnext, left, [&](int j, uint32_t add, uint32_t moved) { ev[done + j] = add | (moved >> 7); });
-        });
+        for (int k = 0; k < src.nchunks; ++k) {
+            const uint4 c = src.next(k);
+            const uint32_t w[5] = {c.x, c.y, c.z, c.w, src.c0.x};
+            for (int q = 0; q < 4 && 16 * k + 4 * q < n; ++q)
+                src.group(iv, w[q], w[q + 1], std::min(4, n - 16 * k - 4 * q),
+                          [&](int j, uint32_t add, uint32_t moved) { ev[16 * k + 4 * q + j] = add | (moved >> 7); });
+        }
         for (int i = 0; i < n; i += 8) {
             const uint32_t e8[8] = {ev[i], ev[i + 1], ev[i + 2], ev[i + 3], ev[i + 4], ev[i + 5], ev[i + 6], ev[i + 7]};
-            if (cd.code8(e8)) continue;
-            for (uint32_t v : e8) {
-                cd.C += v & 0xFFFFu;
-                cd.shift((int)(v >> 16));
-            }
+            if (!cd.code8(e8)) cd.code_each(e8);
         }
         cd.A = iv.A;
         const int len2 = n ? cd.flush() : 0;
