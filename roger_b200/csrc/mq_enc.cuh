@@ -101,7 +101,8 @@ struct MqCoder {
     }
     // interval part of one symbol in state e: the decision in bit 31 of d31, the value added to C
     // in *add; returns the shift count << 23.  *next: table entry of the state after a shift.
-    MQ_HD uint32_t interval(MqState e, uint32_t d31, uint32_t* add, uint32_t* next) {
+    // *width: the new A before the shifts, with either sign (the state changes iff it is below 0x8000).
+    MQ_HD uint32_t interval(MqState e, uint32_t d31, uint32_t* add, uint32_t* next, float* width) {
         const uint32_t qs = e.x ^ (d31 & 0x80000000u);
         const float q = mq_float(qs), s = mq_float((qs & 0x80000000u) | 0x3F800000u);
 #ifdef __CUDA_ARCH__
@@ -115,6 +116,7 @@ struct MqCoder {
 #endif
         *add = a1 > low ? e.y & 0xFFFFu : 0u;
         A = mq_float((m & 0x7FFFFFu) | kMqExp);
+        *width = mq_float(m);
         return kMqExp - (m & 0x7F800000u);
     }
     // Takes the bytes out of c, a C that has been shifted -ct times since the first of them was due;
@@ -228,9 +230,12 @@ struct MqMem {
     // cx8: the context << (SHIFT + 3)
     __device__ __forceinline__ MqState state(uint32_t cx8) const { return load(st + cx8); }
     __device__ __forceinline__ MqState entry(uint32_t i) const { return load(tab + 8 * i); }
-    __device__ __forceinline__ void store_if(uint32_t cond, uint32_t cx8, MqState v) const {
-        asm volatile("{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n @p st.shared.v2.u32 [%0], {%1, %2};\n}" ::"r"(st + cx8),
-                     "r"(v.x), "r"(v.y), "r"(cond)
+    // stores v when |width| is below 0x8000 (compared as it comes out of the maximum: the shift count
+    // takes three operations more)
+    __device__ __forceinline__ void store_if_below(float width, uint32_t cx8, MqState v) const {
+        asm volatile("{\n .reg .pred p;\n .reg .f32 t;\n abs.f32 t, %3;\n setp.lt.f32 p, t, 0f47000000;\n"
+                     " @p st.shared.v2.u32 [%0], {%1, %2};\n}" ::"r"(st + cx8),
+                     "r"(v.x), "r"(v.y), "f"(width)
                      : "memory");
     }
     __device__ __forceinline__ static MqState load(uint32_t at) {
@@ -244,8 +249,8 @@ struct MqMem {
     MqMem(MqState* s, const MqState* t) : st(s), tab(t) {}
     MqState state(uint32_t cx8) const { return st[cx8 / 8]; }
     MqState entry(uint32_t i) const { return tab[i]; }
-    void store_if(uint32_t cond, uint32_t cx8, MqState v) const {
-        if (cond) st[cx8 / 8] = v;
+    void store_if_below(float width, uint32_t cx8, MqState v) const {
+        if (fabsf(width) < 32768.0f) st[cx8 / 8] = v;
     }
 #endif
     // byte j of a symbol word as cx8 (j = 4: the first byte of the next word)
@@ -296,12 +301,13 @@ struct MqSymbols {
             const uint32_t ncx = j < 3 ? mem.context(w, j + 1) : mem.context(wnext, 0);
             const MqState nx = mem.state(ncx);
             uint32_t to, add;
-            const uint32_t moved = e.interval(cur, w << (24 - 8 * j), &add, &to);
+            float width;
+            const uint32_t moved = e.interval(cur, w << (24 - 8 * j), &add, &to, &width);
             put(j, add, moved);
             const MqState up = mem.entry(to);
-            mem.store_if(moved, cx, up);
+            mem.store_if_below(width, cx, up);
             // the next symbol's state: the one loaded ahead, unless this symbol has changed it
-            const bool changed = ncx == cx && moved != 0;
+            const bool changed = ncx == cx && fabsf(width) < 32768.0f;
             cur = MqState{changed ? up.x : nx.x, changed ? up.y : nx.y};
             cx = ncx;
         }

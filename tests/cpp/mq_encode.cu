@@ -3,6 +3,7 @@
 // 20000 symbols (all remainders of a group of four).  Byte 0xFF followed by a late carry, which the
 // group coder codes again, is met thousands of times.  Prints "streams N symbols M" and exits 0.
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
