@@ -16,8 +16,8 @@
 // the bytes that became due are taken from a 64-bit C afterwards.  A byte taken late already holds
 // the carry of the additions after it, which T.800 would add to it one byte later; the result is
 // the same unless the byte was 0xFF when it was due (then the carry stays in the next byte's stuffed
-// bit).  That byte reads as 0, so whenever a late byte does, or the shifts are too many for 64 bits,
-// the group is coded again byte by byte in T.800's order.
+// bit).  That byte reads as 0 with a carry out of it, so whenever one may be such a byte, or the
+// shifts are too many, the group is coded again byte by byte in T.800's order.
 //
 // Host-callable: the same code runs on the CPU in the tests.
 
@@ -125,21 +125,23 @@ struct MqCoder {
         const uint32_t B0 = B, w0 = wacc;
         const int cnt0 = cnt;
         const bool ovf0 = ovf;
-        bool doubt = false;
+        bool doubt = (c >> (28 - ct)) != 0, again = false;
+        // the due byte at bits 62..55, its carry at 63 (each byte taken moves the next one up)
+        uint64_t t = c << (36 + ct);
         do {
-            const int k = -ct;  // shifts since the byte was due (additions without a shift may follow)
-            const uint32_t ck = (uint32_t)(c >> k);
-            const bool carry = B != 0xFFu && (ck >> 27) != 0;
+            const uint32_t top = (uint32_t)(t >> 32);
+            const bool carry = B != 0xFFu && (top >> 31) != 0;
             B += carry ? 1u : 0u;
             const bool ff = B == 0xFFu;
-            const int low = ff ? 20 : 19;
-            const uint32_t v = (carry ? ck & 0x7FFFFFFu : ck) >> low;
-            doubt |= v == 0 || (ck >> 28) != 0;
+            const uint32_t v = ((carry ? top & 0x7FFFFFFFu : top) >> (ff ? 24 : 23)) & 0xFFu;
+            // a 0 that a carry came out of, into B now or into the byte taken before it
+            doubt |= v == 0 && (carry || again);
             push();
             ++cnt;
-            B = v & 0xFFu;
-            c &= ((uint64_t)1 << (low + k)) - 1;
+            B = v;
+            t = (t << (ff ? 8 : 9)) >> 1;
             ct += ff ? 7 : 8;
+            again = true;
         } while (ct <= 0);
         if (doubt) {
             B = B0;
@@ -148,7 +150,7 @@ struct MqCoder {
             ovf = ovf0;
             return false;
         }
-        C = (uint32_t)c;
+        C = (uint32_t)(t >> (36 + ct));
         CT = ct;
         return true;
     }
@@ -219,7 +221,9 @@ struct MqCoder {
 // One lane's 32 context states, 8 << SHIFT bytes apart, and the state table.  On the device both
 // are 32-bit shared-memory addresses that the compiler cannot see through: it computes the address
 // of a shared array anew for every access otherwise, with a special-register read in it.
-template <int SHIFT>
+// COPIES: the table holds each entry that many times side by side, and lane l reads copy l % COPIES
+// (the lanes' entries then fall in distinct banks but for pairs of them).
+template <int SHIFT, int COPIES = 1>
 struct MqMem {
 #ifdef __CUDA_ARCH__
     uint32_t st, tab;
@@ -229,7 +233,7 @@ struct MqMem {
     }
     // cx8: the context << (SHIFT + 3)
     __device__ __forceinline__ MqState state(uint32_t cx8) const { return load(st + cx8); }
-    __device__ __forceinline__ MqState entry(uint32_t i) const { return load(tab + 8 * i); }
+    __device__ __forceinline__ MqState entry(uint32_t i) const { return load(tab + 8 * COPIES * i); }
     // stores v when |width| is below 0x8000 (compared as it comes out of the maximum: the shift count
     // takes three operations more)
     __device__ __forceinline__ void store_if_below(float width, uint32_t cx8, MqState v) const {
@@ -248,7 +252,7 @@ struct MqMem {
     const MqState* tab;
     MqMem(MqState* s, const MqState* t) : st(s), tab(t) {}
     MqState state(uint32_t cx8) const { return st[cx8 / 8]; }
-    MqState entry(uint32_t i) const { return tab[i]; }
+    MqState entry(uint32_t i) const { return tab[COPIES * i]; }
     void store_if_below(float width, uint32_t cx8, MqState v) const {
         if (fabsf(width) < 32768.0f) st[cx8 / 8] = v;
     }
@@ -263,15 +267,15 @@ struct MqMem {
 // The interval part's walk over a symbol stream: n symbols at syms (16-byte aligned; bits 0-4
 // context, bit 7 decision) in 16-byte chunks, two in flight; the state of the next symbol's context
 // is loaded a symbol ahead and replaced when this symbol changes the same context.
-template <int SHIFT>
+template <class Mem>
 struct MqSymbols {
-    const MqMem<SHIFT> mem;
+    const Mem mem;
     const uint4* sp;
     int n, nchunks;
     uint4 c0, c1;
     uint32_t cx;
     MqState cur;
-    MQ_HD MqSymbols(const uint8_t* syms, int count, MqMem<SHIFT> m)
+    MQ_HD MqSymbols(const uint8_t* syms, int count, Mem m)
         : mem(m), sp(reinterpret_cast<const uint4*>(syms)), n(count), nchunks((count + 15) >> 4) {
         const uint4 z = make_uint4(0, 0, 0, 0);
         c0 = nchunks > 0 ? MQ_LOAD16(sp) : z;
@@ -315,9 +319,9 @@ struct MqSymbols {
 };
 
 // Both parts by one lane
-template <int SHIFT>
-MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, MqMem<SHIFT> mem) {
-    MqSymbols<SHIFT> src(syms, n, mem);
+template <class Mem>
+MQ_HD void mq_encode(MqCoder& e, const uint8_t* syms, int n, Mem mem) {
+    MqSymbols<Mem> src(syms, n, mem);
     for (int k = 0; k < src.nchunks; ++k) {
         const uint4 c = src.next(k);
         uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w, ev[8];

@@ -98,20 +98,29 @@ __constant__ uint8_t c_nlps[47] = {1,  6,  9,  12, 29, 33, 6,  14, 14, 14, 17, 1
 
 constexpr int kMqThreads = 32;  // one warp per CTA: the longest blocks' warps spread one per SM
 
-// the 94-entry state table (state * 2 + MPS), filled by the threads of a CTA
+constexpr int kMqCopies = 8;
+constexpr int kMqTable = 94 * kMqCopies;
+
+// the 94-entry state table (state * 2 + MPS), each entry kMqCopies times, filled by the threads of
+// a CTA
 __device__ __forceinline__ void fill_mq_table(MqState* tab) {
-    for (int i = threadIdx.x; i < 94; i += blockDim.x) {
-        const int k = i >> 1;
-        tab[i] = mq_table_entry(c_qe[k], c_nmps[k], c_nlps[k], k == 0 || k == 6 || k == 14, (uint32_t)(i & 1));
+    for (int i = threadIdx.x; i < kMqTable; i += blockDim.x) {
+        const int k = i / kMqCopies >> 1;
+        tab[i] = mq_table_entry(c_qe[k], c_nmps[k], c_nlps[k], k == 0 || k == 6 || k == 14,
+                                (uint32_t)(i / kMqCopies & 1));
     }
+}
+template <int SHIFT>
+__device__ __forceinline__ MqMem<SHIFT, kMqCopies> mq_mem(MqState* st, const MqState* tab) {
+    return MqMem<SHIFT, kMqCopies>(st, tab + threadIdx.x % kMqCopies);
 }
 // T.800 Table D.7: the initial states (context k at st[k * stride]; 32 of them, so that a 5-bit
 // index needs no clamp)
 __device__ __forceinline__ void reset_mq_states(MqState* st, int stride, const MqState* tab) {
     for (int k = 0; k < 32; ++k) st[k * stride] = tab[0];
-    st[0] = tab[4 * 2];
-    st[17 * stride] = tab[3 * 2];
-    st[18 * stride] = tab[46 * 2];
+    st[0] = tab[4 * 2 * kMqCopies];
+    st[17 * stride] = tab[3 * 2 * kMqCopies];
+    st[18 * stride] = tab[46 * 2 * kMqCopies];
 }
 
 // The byte-by-byte MQ encoder registers of the general styled coder, and the byte writer of raw
@@ -200,11 +209,12 @@ struct MqPlaneEnds {
 // One block per lane of a warp pair (mq_enc.cuh): warp 0 runs the interval part and puts four
 // symbols' additions and shifts into a ring in shared memory, warp 1 takes them through the code
 // part eight at a time, a chunk of 16 symbols behind.  The two parts are serial chains of their own,
-// so a symbol costs the longer one instead of both.  Bound by the interval chain: 34 instructions and
-// 78 cycles a symbol for a block alone in its pair, about 100 with 32 blocks (taking the bytes out
-// four symbols at a time made the code warp the slower one there, 145).  One warp with both parts
+// so a symbol costs the longer one instead of both.  Bound by the interval chain: 33 instructions and
+// 67 cycles a symbol for a block alone in its pair (16 symbols unrolled; with four 76), about 90 with
+// 32 blocks (145 with the bytes taken out four symbols at a time, when the code warp was the slower
+// one; 94 with one copy of the state table, whose banks the lanes shared).  One warp with both parts
 // took 104 and 165 cycles; an integer coder with a leading-zero count and a branch to the byte output
-// in every symbol's chain over 200.  4096 blocks of a 4096 x 4096 gray image, 32 to a pair: 1.57 ms,
+// in every symbol's chain over 200.  4096 blocks of a 4096 x 4096 gray image, 32 to a pair: 1.45 ms,
 // 2.32 with the bytes taken out by fours, 2.44 with one warp.
 // RATE: also record the plane ends (MqPlaneEnds) into plane_bytes[job * 32 + k].
 template <bool RATE>
@@ -213,7 +223,7 @@ t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jo
              const uint32_t* __restrict__ order, int njobs, uint8_t* __restrict__ bytes,
              j2k_cb_desc* __restrict__ descs, uint32_t* __restrict__ err, const uint32_t* __restrict__ pend,
              uint32_t* __restrict__ plane_bytes, MqSchedule sched, int lanes) {
-    __shared__ MqState tab[94];
+    __shared__ MqState tab[kMqTable];
     __shared__ MqState cst[32 * kMqThreads];
     __shared__ uint4 ring[2][4][kMqThreads];  // [chunk parity][group][lane]
     __shared__ float last_a[kMqThreads];
@@ -245,13 +255,13 @@ t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jo
     if (threadIdx.x < 32) {
         MqState* st = cst + lane;
         reset_mq_states(st, kMqThreads, tab);
-        MqSymbols<5> src(syms + J.sym_off, n, MqMem<5>(st, tab));
+        MqSymbols<MqMem<5, kMqCopies>> src(syms + J.sym_off, n, mq_mem<5>(st, tab));
         for (int k = 0; k < chunks; ++k) {
             const uint4 c = src.next(k);
             uint32_t wa = c.x, wb = c.y, wc = c.z, wd = c.w, ev[4];
             const auto put = [&](int j, uint32_t add, uint32_t moved) { ev[j] = add | (moved >> 7); };
             if (16 * k + 16 <= n) {
-#pragma unroll 1
+#pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     src.group(e, wa, wb, 4, put);
                     ring[k & 1][q][lane] = make_uint4(ev[0], ev[1], ev[2], ev[3]);
@@ -565,7 +575,7 @@ t1_mq_pass_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict
                   const uint32_t* __restrict__ order, const uint32_t* __restrict__ keys, int nslots, int style,
                   int fac, uint8_t* __restrict__ segs, uint32_t* __restrict__ ulen, uint32_t* __restrict__ ends,
                   uint32_t* __restrict__ err) {
-    __shared__ MqState tab[94];
+    __shared__ MqState tab[kMqTable];
     __shared__ MqState cst[32 * kPassThreads];
     fill_mq_table(tab);
     __syncthreads();
@@ -593,7 +603,7 @@ t1_mq_pass_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict
         reset_mq_states(st, kPassThreads, tab);
         MqCoder e;
         e.init(reinterpret_cast<uint32_t*>(segs + base), (int)(lim - base));
-        mq_encode(e, syms + J.sym_off + s0, n, MqMem<7>(st, tab));
+        mq_encode(e, syms + J.sym_off + s0, n, mq_mem<7>(st, tab));
         len = (uint32_t)e.flush();
         ovf = e.ovf;
     }

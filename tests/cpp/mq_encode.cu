@@ -129,7 +129,7 @@ int main(int argc, char** argv) {
         cd.init(out.data(), (int)out.size() * 4);
         std::fill(out.begin(), out.begin() + f.b.size() / 4 + 1, 0u);
         std::vector<uint32_t> ev(n + 16, 0);
-        MqSymbols<0> src(sym, n, MqMem<0>(st, tab));
+        MqSymbols<MqMem<0>> src(sym, n, MqMem<0>(st, tab));
         for (int k = 0; k < src.nchunks; ++k) {
             const uint4 c = src.next(k);
             const uint32_t w[5] = {c.x, c.y, c.z, c.w, src.c0.x};
