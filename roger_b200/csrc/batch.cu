@@ -18,6 +18,7 @@
 #include <numeric>
 
 #include <cub/cub.cuh>
+#include <cuda.h>  // pointer attributes (the call is reached through the runtime's entry points)
 
 #include "j2k_internal.cuh"
 
@@ -99,6 +100,40 @@ struct j2k_batch {
 };
 
 namespace {
+// Up to 128 images copied by one launch: CTA c takes 32 KB of the image whose chunks hold c.  Bound
+// by the copies' number, not their bytes: 256 images of 64 to 2048 pixels a side one by one
+// took 1.2 of the encode's 10.4 ms, and two launches leave it at 9.3 ms.
+constexpr int kGatherImages = 128, kGatherChunk = 32768;
+struct GatherList {
+    const uint8_t* src[kGatherImages];
+    uint8_t* dst[kGatherImages];       // 16-byte aligned
+    uint32_t bytes[kGatherImages];
+    uint32_t chunk0[kGatherImages + 1];  // first chunk of each image, then their total
+    int n;
+};
+__global__ void __launch_bounds__(256) batch_gather_kernel(const __grid_constant__ GatherList g) {
+    int lo = 0, hi = g.n - 1;  // the last image that starts at or before this chunk
+    while (lo < hi) {
+        const int m = (lo + hi + 1) / 2;
+        if (g.chunk0[m] <= blockIdx.x) lo = m;
+        else hi = m - 1;
+    }
+    const uint32_t at = (blockIdx.x - g.chunk0[lo]) * kGatherChunk;
+    const uint32_t len = min((uint32_t)kGatherChunk, g.bytes[lo] - at);
+    const uint8_t* src = g.src[lo] + at;
+    uint8_t* dst = g.dst[lo] + at;
+    uint32_t done = 0;
+    if (((uintptr_t)src & 15) == 0) {
+        const uint32_t v = len / 16;
+        const uint4* s4 = reinterpret_cast<const uint4*>(src);
+        uint4* d4 = reinterpret_cast<uint4*>(dst);
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < v; i += 256) d4[i] = __ldg(s4 + i);
+        done = 16 * v;
+    }
+    for (uint32_t i = done + threadIdx.x; i < len; i += 256) dst[i] = __ldg(src + i);
+}
+
 __global__ void batch_lengths_kernel(const j2k_cb_desc* __restrict__ d, uint32_t* __restrict__ len, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) len[i] = (uint32_t)max(d[i].length, 0);
@@ -501,6 +536,34 @@ j2k_status j2k_batch_get_option(j2k_batch* b, int key, int* value) {
     J2K_API_END
 }
 
+// [p, p + bytes) lies in one allocation of the context's own device, which its kernels can read.
+// What does not is left to the copy call, which refuses a range that runs past its allocation.
+static bool own_memory(const j2k_ctx* ctx, const void* p, size_t bytes) {
+    using GetAttributes = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const GetAttributes get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<GetAttributes>(f);
+    }();
+    if (!get) return false;
+    CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                  CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    int device = -1;
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    void* value[] = {&type, &managed, &device, &start, &size};
+    const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+    return get(5, what, value, at) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !(managed & 0xff) &&
+           device == ctx->device && start <= at && bytes <= size && at - start <= size - bytes;
+}
+
 j2k_status j2k_batch_upload(j2k_batch* b, const uint8_t* const* pixels, int on_device) {
     J2K_API_BEGIN
     if (!b || !pixels) return J2K_ERR_INVALID_ARG;
@@ -508,12 +571,32 @@ j2k_status j2k_batch_upload(j2k_batch* b, const uint8_t* const* pixels, int on_d
     cudaSetDevice(ctx->device);
     for (size_t i = 0; i < b->img.size(); ++i)
         if (!pixels[i]) return j2k_fail(ctx, J2K_ERR_INVALID_ARG, "pixel pointer is NULL");
+    // images in this device's own memory are gathered by a kernel, any others copied one by one
+    GatherList g;
+    g.n = 0;
+    g.chunk0[0] = 0;
+    const auto gather = [&]() {
+        if (g.n == 0) return J2K_OK;
+        batch_gather_kernel<<<g.chunk0[g.n], 256, 0, ctx->stream>>>(g);
+        g.n = 0;
+        return j2k_cuda_check(ctx, cudaGetLastError(), "batch gather");
+    };
     for (size_t i = 0; i < b->img.size(); ++i) {
         const ImgPlan& im = b->img[i];
-        J2K_CUDA(ctx, cudaMemcpyAsync((uint8_t*)b->in.p + im.in_off, pixels[i], im.n * im.d.ncomp,
-                                      on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, ctx->stream));
+        const size_t bytes = im.n * im.d.ncomp;
+        uint8_t* dst = (uint8_t*)b->in.p + im.in_off;
+        if (on_device && bytes < ((size_t)1 << 31) && own_memory(ctx, pixels[i], bytes)) {
+            g.src[g.n] = pixels[i];
+            g.dst[g.n] = dst;
+            g.bytes[g.n] = (uint32_t)bytes;
+            g.chunk0[g.n + 1] = g.chunk0[g.n] + (uint32_t)((bytes + kGatherChunk - 1) / kGatherChunk);
+            if (++g.n == kGatherImages) J2K_TRY(gather());
+            continue;
+        }
+        J2K_CUDA(ctx, cudaMemcpyAsync(dst, pixels[i], bytes, on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                                      ctx->stream));
     }
-    return J2K_OK;
+    return gather();
     J2K_API_END
 }
 
