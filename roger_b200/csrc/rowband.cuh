@@ -97,6 +97,22 @@ __device__ __forceinline__ void rb_gstore(float* p, const float (&v)[N]) {
     }
 }
 
+// A row between Mallat order (its low half, then its high half) and the lanes' segments, through
+// the row's own shared memory.  A lane's segment of a half is SPL/2 samples; read or written in
+// place, 16 bytes a lane at a stride of SPL * 2 bytes, each access fills half of every 32-byte
+// sector it touches and every sector moves twice.  The lanes instead take the 16-byte chunks
+// lane, lane + 32, ... of each half and change them over in shared memory, chunk c at
+// c ^ (c / 8 % 8): both sides are free of bank conflicts.  Narrower rows (one chunk a lane or less)
+// are contiguous as they are.  Bound by those sectors, not by occupancy (twice the warps per SM
+// left the times as they were).  The four finest levels of 16 images of 1024 x 1024 (forward,
+// inverse with the residual, and the two transposes), lanes' segments -> chunks: 63.5, 65.9, 62.8,
+// 54.1 -> 51.2, 53.9, 53.2, 48.8 us; the whole step 443 -> 380 us.
+template <int SPL>
+constexpr bool rb_staged = SPL >= 16;
+template <int SPL>
+constexpr int rb_chunks = SPL >= 8 ? SPL / 8 : 1;  // chunks of a half per lane
+__device__ __forceinline__ int rb_stage(int c) { return 4 * (c ^ ((c >> 3) & 7)); }
+
 // Horizontal steps of one full row (lane l holds x = SPL*l .. SPL*l + SPL-1, the row is W wide).
 // MODE 3: forward; 0: inverse; 1: transpose of the forward; 2: transpose of the inverse.
 template <int MODE, int SPL>
@@ -336,7 +352,6 @@ rb_ana(const float* __restrict__ in, size_t ipitch, size_t iz, int h, float* __r
         lamG = __fmul_rn(s, q.lam);
     }
     const int bt = 1 + 3 * (q.levels - (q.level + 1));  // this level's HL; LH = bt + 1, HH = bt + 2
-    const int bx = H2 * lane;
     float acc_lo = 0.0f, acc_hi = 0.0f;
 #pragma unroll 1
     for (int r = wp; r < BH; r += G::NW) {
@@ -346,37 +361,69 @@ rb_ana(const float* __restrict__ in, size_t ipitch, size_t iz, int h, float* __r
         rb_row_load<SPL>(rbs + r * W, lane, v);
         const int qy = y & 1, sy = (y >> 1) + (qy ? hl : 0);
         const size_t so = (size_t)sy * dpitch;
+        // runs of N samples at K places of each half: the lane's segment, or its chunks when staged
+        constexpr bool STAGED = rb_staged<SPL>;
+        constexpr int N = STAGED ? 4 : H2, K = STAGED ? rb_chunks<SPL> : 1;
+        const int at = N * lane;
         // QB 2: the row's coefficients and noise, loaded before the lifting hides their latency
-        constexpr int NQ = QB == 2 ? H2 : 1;
-        float ylo[NQ], ulo[NQ], yhi[NQ], uhi[NQ];
+        constexpr int KQ = QB == 2 ? K : 1;
+        float ylo[KQ][N], ulo[KQ][N], yhi[KQ][N], uhi[KQ][N];
         if constexpr (QB == 2) {
-            rb_gload<H2>(q.y + so + wl + bx, yhi);
-            rb_gload<H2>(q.u + so + wl + bx, uhi);
-            if (qy || last) {
-                rb_gload<H2>(q.y + so + bx, ylo);
-                rb_gload<H2>(q.u + so + bx, ulo);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const size_t o = so + at + 128 * k;
+                rb_gload<N>(q.y + o + wl, yhi[k]);
+                rb_gload<N>(q.u + o + wl, uhi[k]);
+                if (qy || last) {
+                    rb_gload<N>(q.y + o, ylo[k]);
+                    rb_gload<N>(q.u + o, ulo[k]);
+                }
             }
         }
         rb_hlift<MODE, SPL>(v, lane);
-        float lo[H2], hi[H2];
+        float lo[K][N], hi[K][N];
+        if constexpr (STAGED) {
+            float* row = rbs + r * W;
+            __syncwarp();
 #pragma unroll
-        for (int i = 0; i < H2; ++i) {
-            lo[i] = v[2 * i];
-            hi[i] = v[2 * i + 1];
-        }
-        if (qy) {
-            rb_put<QB, H2>(dst + so + bx, so + bx, lo, sy, bx, bt + 1, q, stp, rstp, key, G2, lamG, acc_lo, ylo,
-                           ulo);
-            rb_put<QB, H2>(dst + so + wl + bx, so + wl + bx, hi, sy, wl + bx, bt + 2, q, stp, rstp, key, G2, lamG,
-                           acc_hi, yhi, uhi);
+            for (int k = 0; k < K; ++k) {
+                const int p = rb_stage(K * lane + k);
+                *reinterpret_cast<float4*>(row + p) = make_float4(v[8 * k], v[8 * k + 2], v[8 * k + 4], v[8 * k + 6]);
+                *reinterpret_cast<float4*>(row + wl + p) =
+                    make_float4(v[8 * k + 1], v[8 * k + 3], v[8 * k + 5], v[8 * k + 7]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int p = rb_stage(lane + 32 * k);
+                *reinterpret_cast<float4*>(lo[k]) = *reinterpret_cast<const float4*>(row + p);
+                *reinterpret_cast<float4*>(hi[k]) = *reinterpret_cast<const float4*>(row + wl + p);
+            }
         } else {
-            if (QB != 0 && last)
-                rb_put<QB, H2>(dst + so + bx, so + bx, lo, sy, bx, 0, q, stp, rstp, key, G2, lamG, acc_lo, ylo, ulo);
-            else
-                rb_put<0, H2>(lld + (size_t)(y >> 1) * llpitch + bx, 0, lo, 0, 0, 0, q, stp, rstp, key, G2, lamG,
-                              acc_lo, lo, lo);
-            rb_put<QB, H2>(dst + so + wl + bx, so + wl + bx, hi, sy, wl + bx, bt, q, stp, rstp, key, G2, lamG,
-                           acc_hi, yhi, uhi);
+#pragma unroll
+            for (int i = 0; i < H2; ++i) {
+                lo[0][i] = v[2 * i];
+                hi[0][i] = v[2 * i + 1];
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int x = at + 128 * k, kq = QB == 2 ? k : 0;
+            if (qy) {
+                rb_put<QB, N>(dst + so + x, so + x, lo[k], sy, x, bt + 1, q, stp, rstp, key, G2, lamG, acc_lo,
+                              ylo[kq], ulo[kq]);
+                rb_put<QB, N>(dst + so + wl + x, so + wl + x, hi[k], sy, wl + x, bt + 2, q, stp, rstp, key, G2, lamG,
+                              acc_hi, yhi[kq], uhi[kq]);
+            } else {
+                if (QB != 0 && last)
+                    rb_put<QB, N>(dst + so + x, so + x, lo[k], sy, x, 0, q, stp, rstp, key, G2, lamG, acc_lo, ylo[kq],
+                                  ulo[kq]);
+                else
+                    rb_put<0, N>(lld + (size_t)(y >> 1) * llpitch + x, 0, lo[k], 0, 0, 0, q, stp, rstp, key, G2, lamG,
+                                 acc_lo, lo[k], lo[k]);
+                rb_put<QB, N>(dst + so + wl + x, so + wl + x, hi[k], sy, wl + x, bt, q, stp, rstp, key, G2, lamG,
+                              acc_hi, yhi[kq], uhi[kq]);
+            }
         }
     }
     if constexpr (QB != 0) {
@@ -432,15 +479,18 @@ rb_syn(const float* __restrict__ src, size_t spitch, size_t sz, const float* __r
     const float* up = LQ ? q.u + img * sz : nullptr;
     const int wl = W / 2, hl = (h + 1) >> 1;
     const int bt = 1 + 3 * (q.levels - (q.level + 1));
-    const int bx = H2 * lane;
     // 1. the band's rows and 4 halo rows per side (mirrored, or zero outside for MODE 1),
     //    lifted horizontally in registers, natural order into shared memory
+    constexpr bool STAGED = rb_staged<SPL>;
+    constexpr int N = STAGED ? 4 : H2, K = STAGED ? rb_chunks<SPL> : 1;
+    const int at = N * lane;
 #pragma unroll
     for (int r = wp; r < NY; r += G::NW) {
         int gy = y0 - RB_HV + r;
         bool zero = false;
         if (MODE == 0) gy = mirror(gy, h);
         else zero = gy < 0 || gy >= h;
+        float* row = rbs + r * W;
         float v[SPL];
         if (zero) {
 #pragma unroll
@@ -448,33 +498,62 @@ rb_syn(const float* __restrict__ src, size_t spitch, size_t sz, const float* __r
         } else {
             const int qy = gy & 1;
             const size_t so = (size_t)((gy >> 1) + (qy ? hl : 0)) * spitch;
-            float lo[H2], hi[H2];
-            if (qy) rb_gload<H2>(src + so + bx, lo);
-            else rb_gload<H2>(lls + (size_t)(gy >> 1) * llpitch + bx, lo);
-            rb_gload<H2>(src + so + wl + bx, hi);
+            float lo[K][N], hi[K][N];
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const int x = at + 128 * k;
+                if (qy) rb_gload<N>(src + so + x, lo[k]);
+                else rb_gload<N>(lls + (size_t)(gy >> 1) * llpitch + x, lo[k]);
+                rb_gload<N>(src + so + wl + x, hi[k]);
+            }
             if constexpr (LQ) {
-                float u[H2];
-                rb_gload<H2>(up + so + wl + bx, u);
+                float u[K][N];
                 const int bh = qy ? bt + 2 : bt;
 #pragma unroll
-                for (int i = 0; i < H2; ++i)
-                    hi[i] = __fmul_rn(__fadd_rn(__fmul_rn(hi[i], rstp[bh]), u[i]), stp[bh]);
+                for (int k = 0; k < K; ++k) rb_gload<N>(up + so + wl + at + 128 * k, u[k]);
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+#pragma unroll
+                    for (int i = 0; i < N; ++i)
+                        hi[k][i] = __fmul_rn(__fadd_rn(__fmul_rn(hi[k][i], rstp[bh]), u[k][i]), stp[bh]);
                 if (qy || deepest) {
-                    rb_gload<H2>(up + so + bx, u);
                     const int bl = qy ? bt + 1 : 0;
 #pragma unroll
-                    for (int i = 0; i < H2; ++i)
-                        lo[i] = __fmul_rn(__fadd_rn(__fmul_rn(lo[i], rstp[bl]), u[i]), stp[bl]);
+                    for (int k = 0; k < K; ++k) rb_gload<N>(up + so + at + 128 * k, u[k]);
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+#pragma unroll
+                        for (int i = 0; i < N; ++i)
+                            lo[k][i] = __fmul_rn(__fadd_rn(__fmul_rn(lo[k][i], rstp[bl]), u[k][i]), stp[bl]);
                 }
             }
+            if constexpr (STAGED) {
 #pragma unroll
-            for (int i = 0; i < H2; ++i) {
-                v[2 * i] = lo[i];
-                v[2 * i + 1] = hi[i];
+                for (int k = 0; k < K; ++k) {
+                    const int p = rb_stage(lane + 32 * k);
+                    *reinterpret_cast<float4*>(row + p) = *reinterpret_cast<const float4*>(lo[k]);
+                    *reinterpret_cast<float4*>(row + wl + p) = *reinterpret_cast<const float4*>(hi[k]);
+                }
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const int p = rb_stage(K * lane + k);
+                    const float4 a = *reinterpret_cast<const float4*>(row + p);
+                    const float4 b = *reinterpret_cast<const float4*>(row + wl + p);
+                    v[8 * k] = a.x, v[8 * k + 2] = a.y, v[8 * k + 4] = a.z, v[8 * k + 6] = a.w;
+                    v[8 * k + 1] = b.x, v[8 * k + 3] = b.y, v[8 * k + 5] = b.z, v[8 * k + 7] = b.w;
+                }
+                __syncwarp();
+            } else {
+#pragma unroll
+                for (int i = 0; i < H2; ++i) {
+                    v[2 * i] = lo[0][i];
+                    v[2 * i + 1] = hi[0][i];
+                }
             }
             rb_hlift<MODE, SPL>(v, lane);
         }
-        rb_row_store<SPL>(rbs + r * W, lane, v);
+        rb_row_store<SPL>(row, lane, v);
     }
     __syncthreads();
     // 2. columns: vertical steps in registers, natural-order writes
