@@ -209,13 +209,13 @@ dwt_fwd_batched(const j2k_dwt_level_desc* __restrict__ descs, const uint32_t* __
 //   * the vertical lifting runs in registers, one thread per column, the whole column unrolled;
 //   * the horizontal lifting runs in registers, 8 samples per lane, neighbours exchanged with
 //     warp shuffles (the 4-column halo absorbs the missing neighbours at the warp ends);
-//   * subbands are written straight from registers (8-byte vectors when aligned).
+//   * the subbands' rows are put in order in shared memory and written by consecutive samples
+//     (8-byte vectors when aligned).
 // Same arithmetic, operation order and rounding as dwt_fwd_level, so the outputs are identical.
 
 // Step 3 of the fast forward level: horizontal lifting of the FTH vertically lifted rows held in
 // shared memory (strip row r at s[r - RO]), 8 samples per lane (tile columns 8*lane ..
-// 8*lane+7), and the writes of the four subbands (dead-zone indices when QUANT) straight from
-// registers.  Shared by the register-load and the TMA-staged forms of the level kernel.
+// 8*lane+7), and the writes of the four subbands (dead-zone indices when QUANT).  Shared by the register-load and the TMA-staged forms of the level kernel.
 template <int KERN, typename TD, bool QUANT, bool QLL, int FTH, int RO>
 __device__ __forceinline__ void fwd_fast_rows(typename KT<KERN>::T (*s)[FNX], int x0, int y0, int w, int h,
                                               typename KT<KERN>::T* __restrict__ ll_dst, size_t llpitch,
@@ -258,46 +258,51 @@ __device__ __forceinline__ void fwd_fast_rows(typename KT<KERN>::T (*s)[FNX], in
         // subband rows: even y -> LL / HL, odd y -> LH / HH
         const int qy = y & 1;
         const int sy = (y >> 1) + (qy ? hl : 0);
-        const int xs = x0 - 4 + 8 * lane;  // absolute x of v[0] (even)
+        // the row back to its own place in shared memory, low samples first: the lanes then write
+        // consecutive pairs (or single samples) of a band, whole sectors at a time
+        T* row = &s[r - RO][0];
+        __syncwarp();
+        {
+            T lo[4] = {v[0], v[2], v[4], v[6]}, hi[4] = {v[1], v[3], v[5], v[7]};
+            *reinterpret_cast<uint4*>(row + 4 * lane) = *reinterpret_cast<uint4*>(lo);
+            *reinterpret_cast<uint4*>(row + 128 + 4 * lane) = *reinterpret_cast<uint4*>(hi);
+        }
+        __syncwarp();
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {  // samples v[4*half .. 4*half+3]
-            const int e0 = 8 * lane + 4 * half;  // tile column of the first sample
-            const int xa = xs + 4 * half;
-            if (e0 + 4 <= 4 || e0 >= 252) continue;  // halo columns
-            for (int qx = 0; qx < 2; ++qx) {
-                const bool isll = (qx == 0 && qy == 0);
-                T a = v[4 * half + qx], b = v[4 * half + 2 + qx];
-                const int sx = (xa >> 1) + (qx ? wl : 0);  // band index of a (b is sx+1)
-                const bool va = xa + qx < w, vb = xa + 2 + qx < w;
-                if (isll && !QLL) {
-                    T* p = ll_dst + (size_t)sy * llpitch + sx;
-                    if (vec_out && va && vb) {
-                        T pr[2] = {a, b};
-                        *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(pr);
-                    } else {
-                        if (va) p[0] = a;
-                        if (vb) p[1] = b;
+        for (int qx = 0; qx < 2; ++qx) {
+            const bool isll = (qx == 0 && qy == 0);
+            const float step = isll ? st.ll : (qx && qy ? st.hh : (qx ? st.hl : st.lh));
+            // samples 2 .. 125 of the strip's 128 are the tile's; n of them lie inside the level
+            const int n = min(FTW / 2, (w - x0 - qx + 1) >> 1);
+            const int sx = (x0 >> 1) + (qx ? wl : 0);
+            const T* b = row + 128 * qx + 2;
+            const auto put = [&](auto* p, auto conv) {
+                using P = decltype(conv(T()));
+                if (vec_out && (sx & 1) == 0) {
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const int i = 2 * lane + 64 * k;
+                        T pr[2];
+                        *reinterpret_cast<uint2*>(pr) = *reinterpret_cast<const uint2*>(b + min(i, FTW / 2 - 2));
+                        P o[2] = {conv(pr[0]), conv(pr[1])};
+                        if (i + 1 < n) *reinterpret_cast<uint2*>(p + i) = *reinterpret_cast<uint2*>(o);
+                        else if (i < n) p[i] = o[0];
                     }
                 } else {
-                    const float step = isll ? st.ll : (qx && qy ? st.hh : (qx ? st.hl : st.lh));
-                    TD oa, ob;
-                    if (QUANT) {
-                        oa = (TD)quantize((float)a, step);
-                        ob = (TD)quantize((float)b, step);
-                    } else {
-                        oa = (TD)a;
-                        ob = (TD)b;
-                    }
-                    TD* p = dst + (size_t)sy * dpitch + sx;
-                    if (vec_out && va && vb && ((sx & 1) == 0)) {
-                        TD pr[2] = {oa, ob};
-                        *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(pr);
-                    } else {
-                        if (va) p[0] = oa;
-                        if (vb) p[1] = ob;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const int i = lane + 32 * k;
+                        if (i < n) p[i] = conv(b[i]);
                     }
                 }
-            }
+            };
+            if (isll && !QLL)
+                put(ll_dst + (size_t)sy * llpitch + sx, [](T a) { return a; });
+            else
+                put(dst + (size_t)sy * dpitch + sx, [&](T a) {
+                    if constexpr (QUANT) return (TD)quantize((float)a, step);
+                    else return (TD)a;
+                });
         }
     }
 }

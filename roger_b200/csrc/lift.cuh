@@ -309,12 +309,15 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
             sb[j] = (colok && y0 + j < h) ? __ldcg(sub + (size_t)(y0 + j) * ex.sub_pitch + x) : 0.0f;
     }
     // 1. the strip's rows y0 - HV + r (mirrored, or zero outside the level for MODE 1), warp w
-    //    taking rows w, w + 8, ...: lane l loads the band samples of natural columns
-    //    x0 - 4 + 8l .. + 7 straight into registers (low band: LL or LH row, high band: HL or
-    //    HH row), raw; all rows' loads are issued before any is used
+    //    taking rows w, w + 8, ...: 128 samples of the low band (LL or LH row) and of the high
+    //    band (HL or HH row), raw; all rows' loads are issued before any is used.  The lanes take
+    //    consecutive pairs (single samples where the rows do not allow pairs), so that whole
+    //    sectors move; a lane's own four, 16 bytes apart, would touch every sector two or four
+    //    times (with the forward levels written the same way: three 4096 x 4096 planes there and
+    //    back by 5/3 279 -> 267 us, three odd-sized planes by 9/7 186 -> 167 us)
     constexpr int RI = (NY + 7) / 8;
     uint32_t rl[RI][4], rh[RI][4];
-    const int lx = ((x0 - 4) >> 1) + 4 * lane;  // band index of this lane's first low sample
+    const int lx = (x0 - 4) >> 1;  // band index of the strip's first low sample
 #pragma unroll
     for (int i = 0; i < RI; ++i) {
         const int r = warp + 8 * i;
@@ -332,16 +335,16 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
         if (inner_x && vec_in) {
             // (L2 only, as in the forward levels: a level launched as a dependent may start while the
             // previous one runs, so an SM's L1 could still hold lines of its input buffer)
-            const uint2 l0 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx));
-            const uint2 l1 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx + 2));
-            const uint2 h0 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx));
-            const uint2 h1 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx + 2));
+            const uint2 l0 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx) + lane);
+            const uint2 l1 = __ldcg(reinterpret_cast<const uint2*>(lsrc + lx) + lane + 32);
+            const uint2 h0 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx) + lane);
+            const uint2 h1 = __ldcg(reinterpret_cast<const uint2*>(srow + wl + lx) + lane + 32);
             rl[i][0] = l0.x; rl[i][1] = l0.y; rl[i][2] = l1.x; rl[i][3] = l1.y;
             rh[i][0] = h0.x; rh[i][1] = h0.y; rh[i][2] = h1.x; rh[i][3] = h1.y;
         } else {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                int ge = x0 - 4 + 8 * lane + 2 * k, go = ge + 1;
+                int ge = x0 - 4 + 2 * (lane + 32 * k), go = ge + 1;
                 if (MODE == 0) {
                     ge = mirror(ge, w);
                     go = mirror(go, w);
@@ -360,6 +363,25 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
         for (int i = 0; i < RI; ++i) {
             const int r = warp + 8 * i;
             if (r >= NY) break;
+            // the row's samples to their lanes: lane l lifts natural columns x0 - 4 + 8l .. + 7
+            if (inner_x && vec_in) {
+#pragma unroll
+                for (int k = 0; k < 2; ++k) {
+                    reinterpret_cast<uint2*>(&s[r][0])[lane + 32 * k] = make_uint2(rl[i][2 * k], rl[i][2 * k + 1]);
+                    reinterpret_cast<uint2*>(&s[r][128])[lane + 32 * k] = make_uint2(rh[i][2 * k], rh[i][2 * k + 1]);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    s[r][lane + 32 * k] = bits_as<T>(rl[i][k]);
+                    s[r][128 + lane + 32 * k] = bits_as<T>(rh[i][k]);
+                }
+            }
+            __syncwarp();
+            const uint4 ql = *reinterpret_cast<const uint4*>(&s[r][4 * lane]);
+            const uint4 qh = *reinterpret_cast<const uint4*>(&s[r][128 + 4 * lane]);
+            const uint32_t vl[4] = {ql.x, ql.y, ql.z, ql.w}, vh[4] = {qh.x, qh.y, qh.z, qh.w};
+            __syncwarp();
             T v[8];
             const int qy = r & 1;  // mirroring keeps the parity of y0 - HV + r
             const float sl = qy ? st.lh : st.ll, sh = qy ? st.hh : st.hl;
@@ -367,11 +389,11 @@ dwt_syn_fast(const TS* __restrict__ src, size_t spitch, const typename KT<KERN>:
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 if constexpr (DEQ) {
-                    v[2 * k] = lo_raw ? (T)dequantize((int32_t)rl[i][k], sl) : bits_as<T>(rl[i][k]);
-                    v[2 * k + 1] = (T)dequantize((int32_t)rh[i][k], sh);
+                    v[2 * k] = lo_raw ? (T)dequantize((int32_t)vl[k], sl) : bits_as<T>(vl[k]);
+                    v[2 * k + 1] = (T)dequantize((int32_t)vh[k], sh);
                 } else {
-                    v[2 * k] = bits_as<T>(rl[i][k]);
-                    v[2 * k + 1] = bits_as<T>(rh[i][k]);
+                    v[2 * k] = bits_as<T>(vl[k]);
+                    v[2 * k + 1] = bits_as<T>(vh[k]);
                 }
             }
             if (w > 1) {
