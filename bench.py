@@ -668,7 +668,7 @@ def bench_c1(flush, hbm, peak_src, clocks):
         planar_gbs=round(n * 15 / (t_planar * 1e-3) / 1e9, 1),
         planar_frac=round(n * 15 / (t_planar * 1e-3) / 1e9 / hbm, 4),
         tier1_issue=tier1_issue("tier1_instructions_lossless_4096.txt",
-                                "t1_symbols_kernel + t1_mq_kernel<16> (tiered warp schedule)", t1_ms, clocks),
+                                "t1_symbols_kernel + t1_mq_kernel (warp pairs, tiered schedule)", t1_ms, clocks),
         tier1={"codeblocks": int(len(descs)), "sample_passes": samples,
                "gsample_passes_per_s": round(samples / (t1_ms * 1e-3) / 1e9, 3),
                "codeword_bytes": int(res[1].size)},
