@@ -282,6 +282,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
         ++npass;
         if (pad) {  // the next pass starts on a 16-byte boundary (a coding unit of its own)
             if (!ovf) write_rest();
+            __syncwarp();  // before another lane writes the stage's first bytes again
             pos = (pos + 15) & ~15;
             ovf |= pos > cap;
         }
