@@ -206,6 +206,13 @@ struct MqPlaneEnds {
     }
 };
 
+// Where the two warps of a pair meet, once per chunk in each one's loop.  A numbered barrier, not
+// __syncthreads: the meeting places of the two roles are different ones.
+__device__ __forceinline__ void mq_pair_barrier() {
+    static_assert(kMqThreads == 32, "a pair is 64 threads");
+    asm volatile("bar.sync 1, 64;" ::: "memory");
+}
+
 // One block per lane of a warp pair (mq_enc.cuh): warp 0 runs the interval part and puts four
 // symbols' additions and shifts into a ring in shared memory, warp 1 takes them through the code
 // part eight at a time, a chunk of 16 symbols behind.  The two parts are serial chains of their own,
@@ -281,7 +288,7 @@ t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jo
                 }
             }
             if (16 * k + 16 >= n) last_a[lane] = e.A;  // (again in every chunk after the last symbol)
-            __syncthreads();
+            mq_pair_barrier();
         }
         return;
     }
@@ -293,7 +300,7 @@ t1_mq_kernel(const uint8_t* __restrict__ syms, const j2k_cb_job* __restrict__ jo
         while (ends.next() == 0u) ends.at(e);  // passes with no symbols at all
     }
     for (int k = 0; k < chunks; ++k) {
-        __syncthreads();  // chunk k is in the ring; the interval warp goes on with chunk k + 1
+        mq_pair_barrier();  // chunk k is in the ring; the interval warp goes on with chunk k + 1
 #pragma unroll 1
         for (int q = 0; q < 4 && 16 * k + 4 * q < n; q += 2) {
             const int at = 16 * k + 4 * q;
