@@ -713,6 +713,8 @@ struct TmaStrip {
     static constexpr int SMEM = 2 * BYTES + 16;  // two strips, two barriers
 };
 
+// orders this thread's shared-memory accesses before tensor copies issued after the next barrier
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 template <int KERN, typename TD, bool QUANT, bool QLL>
@@ -811,7 +813,10 @@ dwt_fwd_tma(const __grid_constant__ CUtensorMap tmap, int w, int h, int nz, int 
         // 3. horizontal lifting and the subband writes, from the strip's rows HV .. HV+15
         fwd_fast_rows<KERN, TD, QUANT, QLL, kTmaTh, 0>(stg[stage], x0, y0, w, h, ll_dst + tz * z.ll, llpitch,
                                                        dst + tz * z.dst, dpitch, st, vec_out);
-        __syncthreads();  // the strip is free for the copy issued at the top of the next tile
+        // the strip is free for the copy issued at the top of the next tile, which comes after
+        // every thread's own writes to it (the lifted rows, and the rows put in order)
+        fence_proxy_async();
+        __syncthreads();
     }
 }
 

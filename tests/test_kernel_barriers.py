@@ -35,3 +35,16 @@ def test_no_block_barrier_where_the_warps_part():
                 rest = src[end:src.index("\n}\n", end)]
                 assert "__syncthreads" not in rest, name
     assert roles > 0
+
+
+def test_strips_that_tensor_copies_refill_are_fenced():
+    """A thread that has written shared memory which a tensor copy then overwrites puts a proxy fence
+    before the barrier after which the copy is issued: a barrier alone does not order the two."""
+    loops = 0
+    for name, src in _code():
+        for m in re.finditer(r"cp\.async\.bulk\.tensor", src):
+            start = src.rindex("__global__", 0, m.start())
+            body = src[start:_end_of_block(src, src.index("{", src.index(")", start)))]
+            assert re.search(r"fence_proxy_async\(\);\s*__syncthreads\(\);\s*\}\s*\}$", body), name
+            loops += 1
+    assert loops > 0
