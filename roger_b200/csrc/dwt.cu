@@ -1284,10 +1284,12 @@ j2k_status fwd_levels(j2k_ctx* ctx, const void* in, size_t in_pitch, void* out, 
         // 286 us with level 0 in the tile kernel (146 us) and take 192 us this way.
         const bool aligned = ((uintptr_t)src & 15) == 0 && (spitch & 3) == 0 && (n == 1 || (src_z & 3) == 0);
         const bool loads_samples = !ctx || (ctx->dwt_reg && !ctx->dwt_pipe && !ctx->dwt_tma);
-        const bool fast_ok = ORDER == J2K_ORDER_T800 && (aligned || loads_samples) && cw >= 8 && chh >= 2 &&
-                             (!ctx || ctx->dwt_fast_th != 0);
+        // A grid has at most 65535 rows of tiles: a level of more takes the tile kernel, whose tiles
+        // are higher.
+        const int fth = ctx ? ctx->dwt_fast_th : 32;
+        const bool fast_ok = ORDER == J2K_ORDER_T800 && (aligned || loads_samples) && cw >= 8 && chh >= 2 && fth != 0 &&
+                             (chh - 1) / fth < 65535;
         if (fast_ok) {
-            const int fth = ctx ? ctx->dwt_fast_th : 32;
             dim3 fg((cw + FTW - 1) / FTW, (chh + fth - 1) / fth, n);
             const int vec = (((uintptr_t)out & 7) == 0) && ((out_pitch & 1) == 0) &&
                             (((uintptr_t)lld & 7) == 0) && ((llp & 1) == 0) &&
