@@ -67,12 +67,7 @@ t1_symbols_kernel(const int32_t* __restrict__ coeff, const j2k_cb_job* __restric
         }
         continue;
     }
-    if (J.cw > 32)
-        symbols_of_block<4, 2, uint64_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
-    else if (J.ch > 32)
-        symbols_of_block<2, 2, uint32_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
-    else
-        symbols_of_block<1, 4, uint32_t>(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
+    symbols_of_shape(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad);
     }  // queue loop
 }
 

@@ -96,9 +96,7 @@ __device__ __forceinline__ SignSlices sign_slices(const Near& a, uint32_t own, u
     return r;
 }
 
-// NW words per lane, LPS lanes per stripe, RT row masks of 8 * NW * LPS columns: <4, 2, uint64_t>
-// for blocks wider than 32, <2, 2, uint32_t> for narrower ones and <1, 4, uint32_t> where they are
-// at most 32 high (all 32 lanes busy on a 32 x 32 block).
+// NW words per lane, LPS lanes per stripe, RT row masks of 8 * NW * LPS columns or more.
 template <int NW, int LPS, typename RT>
 __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J, int jid, int lane,
                                                  const int32_t* __restrict__ coeff, uint8_t* __restrict__ syms,
@@ -106,9 +104,16 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                                                  uint64_t* __restrict__ planes, j2k_cb_desc* __restrict__ descs,
                                                  uint32_t* __restrict__ err, int pad) {
     constexpr unsigned FULL = 0xffffffffu;
+    // kOne: the block is one word.  Every lane holds it, and writes the symbols of sample `lane`.
+    // kNarrow: one word per stripe.  Such blocks are small: what counts is not their symbols but what
+    // every plane and pass costs whatever it holds, so the empty passes and exchanges are left out (at
+    // most 8 x 64 samples, whose symbols of a pass fit the stage).
+    constexpr bool kOne = LPS == 32, kNarrow = kOne || LPS == 1;
+    static_assert(!kNarrow || NW == 1, "");
     const int cw = J.cw, ch = J.ch, orient = J.orient;
     const int32_t* blk = coeff + J.off;
-    const int s0 = 4 * (lane / LPS), part = lane % LPS;  // first row of the lane's stripe, place in it
+    const uint32_t me = 1u << lane, before_me = me - 1u;  // (kOne)
+    const int s0 = 4 * (lane / LPS), part = kOne ? 0 : lane % LPS;  // first row of the lane's stripe, place in it
 
     // ---- bit-plane slicing: lane p ends up holding plane p of each row and stores it
     uint32_t mor = 0;
@@ -167,10 +172,26 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
     __syncwarp();
 
     // a word from the lane of the stripe above / below or of the words before / after (0 outside)
-    auto above = [&](uint32_t x) { const uint32_t t = __shfl_up_sync(FULL, x, LPS); return lane < LPS ? 0u : t; };
-    auto below = [&](uint32_t x) { const uint32_t t = __shfl_down_sync(FULL, x, LPS); return lane >= 32 - LPS ? 0u : t; };
-    auto before = [&](uint32_t x) { const uint32_t t = __shfl_up_sync(FULL, x, 1); return part == 0 ? 0u : t; };
-    auto after = [&](uint32_t x) { const uint32_t t = __shfl_down_sync(FULL, x, 1); return part == LPS - 1 ? 0u : t; };
+    auto above = [&](uint32_t x) {
+        if constexpr (kOne) return 0u;
+        const uint32_t t = __shfl_up_sync(FULL, x, LPS);
+        return lane < LPS ? 0u : t;
+    };
+    auto below = [&](uint32_t x) {
+        if constexpr (kOne) return 0u;
+        const uint32_t t = __shfl_down_sync(FULL, x, LPS);
+        return lane >= 32 - LPS ? 0u : t;
+    };
+    auto before = [&](uint32_t x) {
+        if constexpr (kNarrow) return 0u;
+        const uint32_t t = __shfl_up_sync(FULL, x, 1);
+        return part == 0 ? 0u : t;
+    };
+    auto after = [&](uint32_t x) {
+        if constexpr (kNarrow) return 0u;
+        const uint32_t t = __shfl_down_sync(FULL, x, 1);
+        return part == LPS - 1 ? 0u : t;
+    };
     // the lane's words of four row masks
     auto nibbles = [&](const RT (&row)[4], uint32_t (&x)[NW]) {
         uint32_t h[4];
@@ -248,8 +269,8 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
     // One pass's symbols: each lane has cnt of them, which emit(at) writes from stage[at] on.  The
     // stage holds the bytes from the last 16-byte boundary of the output on.
     auto write_pass = [&](int cnt, auto emit) {
-        int tot;
-        const int off = warp_excl(cnt, lane, &tot);
+        int tot = cnt, off = 0;
+        if (!kOne) off = warp_excl(cnt, lane, &tot);
         if (pos + tot > cap) {
             ovf = true;
             return;
@@ -258,16 +279,18 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
             const bool mine = off >= base && off + cnt <= base + kStage && cnt > 0;
             const int lead = pos & 15;
             if (mine) emit(lead + off - base);
-            const unsigned left = __ballot_sync(FULL, cnt > 0 && off + cnt > base + kStage);
+            const unsigned left = kNarrow ? 0u : __ballot_sync(FULL, cnt > 0 && off + cnt > base + kStage);
             const int next = left ? __shfl_sync(FULL, off, __ffs(left) - 1) : tot;
             __syncwarp();
             const int fill = lead + next - base, full = fill >> 4;
-            uint4* dst = reinterpret_cast<uint4*>(out + (pos - lead));
-            for (int i = lane; i < full; i += 32) dst[i] = S.stage[i];
-            const uint4 rest = S.stage[full];
-            __syncwarp();
-            if (lane == 0) S.stage[0] = rest;
-            __syncwarp();
+            if (!kNarrow || full > 0) {
+                uint4* dst = reinterpret_cast<uint4*>(out + (pos - lead));
+                for (int i = lane; i < full; i += 32) dst[i] = S.stage[i];
+                const uint4 rest = S.stage[full];
+                __syncwarp();
+                if (lane == 0) S.stage[0] = rest;
+                __syncwarp();
+            }
             pos += next - base;
             base = next;
         }
@@ -288,6 +311,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
         }
     };
 
+    bool all = false;  // every sample is significant: the propagation and cleanup passes are empty
     for (int p = numbps - 1; p >= 0 && !ovf; --p) {
         RT Br[4];
         uint32_t B[NW], K[NW], now[NW];  // this plane, samples the propagation pass codes, significance
@@ -301,63 +325,68 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
         }
         if (p != numbps - 1) {
             // ------------------------- significance propagation pass
-            RT N[4] = {0, 0, 0, 0};
-            {
-                RT up = __shfl_up_sync(FULL, O[3], LPS), dw = __shfl_down_sync(FULL, O[0], LPS);
-                if (lane < LPS) up = 0;
-                if (lane >= 32 - LPS) dw = 0;
-                RT E[4], M[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const RT u = j ? O[j ? j - 1 : 0] : up, w = j < 3 ? O[j < 3 ? j + 1 : 3] : dw;
-                    M[j] = Vr[j] & ~O[j] & Br[j];
-                    E[j] = M[j] & dil((RT)(u | O[j] | w));
-                }
-                bool more;
-                do {
-                    RT ab = __shfl_up_sync(FULL, N[3], LPS);
-                    if (lane < LPS) ab = 0;
-                    RT was = 0;
+            Near a[NW];
+            int cnt = 0;
+            if (!all) {
+                RT N[4] = {0, 0, 0, 0};
+                {
+                    RT up = 0, dw = 0;
+                    if (!kOne) up = __shfl_up_sync(FULL, O[3], LPS), dw = __shfl_down_sync(FULL, O[0], LPS);
+                    if (lane < LPS) up = 0;
+                    if (lane >= 32 - LPS) dw = 0;
+                    RT E[4], M[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const RT u = j ? N[j ? j - 1 : 0] : (RT)0, w = j < 3 ? N[j < 3 ? j + 1 : 3] : (RT)0;
-                        const RT seeds = (E[j] | (M[j] & ((RT)((u | w) << 1) | u | (j == 0 ? dil(ab) : (RT)0))));
-                        const RT f = M[j] & ((RT) ~(RT)(M[j] + seeds) | seeds);
-                        was |= f ^ N[j];
-                        N[j] = f;
+                        const RT u = j ? O[j ? j - 1 : 0] : up, w = j < 3 ? O[j < 3 ? j + 1 : 3] : dw;
+                        M[j] = Vr[j] & ~O[j] & Br[j];
+                        E[j] = M[j] & dil((RT)(u | O[j] | w));
                     }
-                    more = __any_sync(FULL, was != 0);
-                } while (more);
-            }
-            uint32_t Nn[NW];
-            nibbles(N, Nn);
-            Near a[NW];
+                    bool more;
+                    do {
+                        RT ab = 0;
+                        if (!kOne) ab = __shfl_up_sync(FULL, N[3], LPS);
+                        if (lane < LPS) ab = 0;
+                        RT was = 0;
 #pragma unroll
-            for (int k = 0; k < NW; ++k) now[k] = sig[k] | Nn[k];
-            neighbours(sig, now, a);
-            int cnt = 0;
+                        for (int j = 0; j < 4; ++j) {
+                            const RT u = j ? N[j ? j - 1 : 0] : (RT)0, w = j < 3 ? N[j < 3 ? j + 1 : 3] : (RT)0;
+                            const RT seeds = (E[j] | (M[j] & ((RT)((u | w) << 1) | u | (j == 0 ? dil(ab) : (RT)0))));
+                            const RT f = M[j] & ((RT) ~(RT)(M[j] + seeds) | seeds);
+                            was |= f ^ N[j];
+                            N[j] = f;
+                        }
+                        more = __any_sync(FULL, was != 0);
+                    } while (more);
+                }
+                uint32_t Nn[NW];
+                nibbles(N, Nn);
 #pragma unroll
-            for (int k = 0; k < NW; ++k) {
-                K[k] = V[k] & ~sig[k] & a[k].any();
-                cnt += __popc(K[k]) + __popc(Nn[k]);
-            }
-            write_pass(cnt, [&](int at) {
+                for (int k = 0; k < NW; ++k) now[k] = sig[k] | Nn[k];
+                neighbours(sig, now, a);
 #pragma unroll
                 for (int k = 0; k < NW; ++k) {
-                    uint32_t L[4], m = K[k];
-                    if (!m) continue;
-                    zc_slices(a[k], orient, L);
-                    const SignSlices g = signs(a[k], k);
-                    while (m) {
-                        const int i = __ffs((int)m) - 1;
-                        m &= m - 1;
-                        const uint32_t b = bit_of(B[k], i);
-                        stage[at++] = (uint8_t)(bit_of(L[0], i) | (bit_of(L[1], i) << 1) | (bit_of(L[2], i) << 2) |
-                                                (bit_of(L[3], i) << 3) | (b << 7));
-                        if (b) stage[at++] = (uint8_t)g.symbol(i);
-                    }
+                    K[k] = V[k] & ~sig[k] & a[k].any();
+                    cnt += __popc(K[k]) + __popc(Nn[k]);
                 }
-            });
+                write_pass(cnt, [&](int at) {
+#pragma unroll
+                    for (int k = 0; k < NW; ++k) {
+                        uint32_t L[4], m = K[k];
+                        if (!m) continue;
+                        if (kOne) at += __popc(m & before_me) + __popc(m & B[k] & before_me), m &= me;
+                        zc_slices(a[k], orient, L);
+                        const SignSlices g = signs(a[k], k);
+                        while (m) {
+                            const int i = __ffs((int)m) - 1;
+                            m &= m - 1;
+                            const uint32_t b = bit_of(B[k], i);
+                            stage[at++] = (uint8_t)(bit_of(L[0], i) | (bit_of(L[1], i) << 1) | (bit_of(L[2], i) << 2) |
+                                                    (bit_of(L[3], i) << 3) | (b << 7));
+                            if (b) stage[at++] = (uint8_t)g.symbol(i);
+                        }
+                    }
+                });
+            }
             end_pass();
             if (ovf) break;
             // ------------------------- magnitude refinement pass
@@ -370,6 +399,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                 for (int k = 0; k < NW; ++k) {
                     const uint32_t nb = a[k].any();
                     uint32_t m = sig[k];
+                    if (kOne) at += __popc(m & before_me), m &= me;
                     while (m) {
                         const int i = __ffs((int)m) - 1;
                         m &= m - 1;
@@ -383,7 +413,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
             if (ovf) break;
         }
         // ------------------------- cleanup pass
-        {
+        if (!all) {
             uint32_t C[NW], fin[NW];
             Near a[NW];
 #pragma unroll
@@ -416,6 +446,9 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                 for (int k = 0; k < NW; ++k) {
                     uint32_t L[4], m = ev[k];
                     if (!m) continue;
+                    if (kOne)
+                        at += __popc(m & before_me) + __popc(m & B[k] & before_me) + 2 * __popc(run[k] & B[k] & before_me),
+                            m &= me;
                     zc_slices(a[k], orient, L);
                     const SignSlices g = signs(a[k], k);
                     while (m) {
@@ -434,12 +467,17 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                     }
                 }
             });
+            uint32_t none = 0;
 #pragma unroll
-            for (int k = 0; k < NW; ++k) sig[k] = fin[k];
+            for (int k = 0; k < NW; ++k) {
+                sig[k] = fin[k];
+                none |= V[k] & ~sig[k];
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) O[j] |= Br[j] & Vr[j];
-            end_pass();
+            if (kNarrow) all = !__any_sync(FULL, none != 0);
         }
+        end_pass();
     }
     if (ovf) {
         if (lane == 0) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_SYM_CAPACITY);
@@ -453,3 +491,32 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
     }
     __syncwarp();
 }
+
+#define SYMBOLS_ARGS                                                                                                    \
+    SymSmem &S, const j2k_cb_job &J, int jid, int lane, const int32_t *__restrict__ coeff, uint8_t *__restrict__ syms, \
+        uint32_t *__restrict__ nsyms, uint32_t *__restrict__ pass_end, uint64_t *__restrict__ planes,                  \
+        j2k_cb_desc *__restrict__ descs, uint32_t *__restrict__ err, int pad
+#define SYMBOLS(...) __VA_ARGS__(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad)
+
+// a call of its own, so that the common forms' code is what it would be without this one
+template <int NW, int LPS, typename RT>
+__device__ __noinline__ void symbols_of_rare_block(SYMBOLS_ARGS) {
+    SYMBOLS(symbols_of_block<NW, LPS, RT>);
+}
+
+// The form that keeps most lanes busy: 32 / LPS stripes of 8 * NW * LPS columns, or for the narrow ones
+// one word per lane, or one in all lanes.  Bound by issue.  Whole encodes of 2048 x 2048 colour with
+// three forms only (wider than 32, narrower, at most 32 x 32) -> with these: blocks of 64 x 4 2.80 -> 1.24
+// ms, 64 x 8 1.84 -> 0.98, 8 x 8 2.92 -> 2.89, 4 x 4 6.62 -> 3.92; 32 x 32 and 64 x 64 as before.
+__device__ __forceinline__ void symbols_of_shape(SYMBOLS_ARGS) {
+    const int w = J.cw, h = J.ch;
+    if (w <= 8 && h <= 4) SYMBOLS(symbols_of_rare_block<1, 32, uint32_t>);
+    else if (w <= 8) SYMBOLS(symbols_of_rare_block<1, 1, uint32_t>);
+    else if (w <= 32 && h <= 32) SYMBOLS(symbols_of_block<1, 4, uint32_t>);
+    else if (w <= 32) SYMBOLS(symbols_of_block<2, 2, uint32_t>);
+    else if (h <= 16) SYMBOLS(symbols_of_rare_block<1, 8, uint64_t>);
+    else if (h <= 32) SYMBOLS(symbols_of_rare_block<2, 4, uint64_t>);
+    else SYMBOLS(symbols_of_block<4, 2, uint64_t>);
+}
+#undef SYMBOLS
+#undef SYMBOLS_ARGS

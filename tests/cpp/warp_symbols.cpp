@@ -19,6 +19,10 @@
 
 #include "j2k_internal.cuh"
 
+#ifndef __noinline__
+#define __noinline__ __attribute__((noinline))
+#endif
+
 namespace {
 
 struct Meeting {  // of 32 threads
@@ -126,16 +130,8 @@ int main() {
         for (int lane = 0; lane < 32; ++lane)
             lanes.emplace_back([&, lane] {
                 my_lane = lane;
-                // the kernel's choice of a form
-                if (cw > 32)
-                    symbols_of_block<4, 2, uint64_t>(*smem, J, 0, lane, coeff.data(), out, &nsyms, pend.data(),
-                                                     planes.data(), &d, &err, pad);
-                else if (ch > 32)
-                    symbols_of_block<2, 2, uint32_t>(*smem, J, 0, lane, coeff.data(), out, &nsyms, pend.data(),
-                                                     planes.data(), &d, &err, pad);
-                else
-                    symbols_of_block<1, 4, uint32_t>(*smem, J, 0, lane, coeff.data(), out, &nsyms, pend.data(),
-                                                     planes.data(), &d, &err, pad);
+                symbols_of_shape(*smem, J, 0, lane, coeff.data(), out, &nsyms, pend.data(), planes.data(), &d, &err,
+                                 pad);
             });
         for (auto& t : lanes) t.join();
         if (err) return 3;
