@@ -452,7 +452,7 @@ j2k_status j2k_bpc_decode(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t*
     if (!dj) return J2K_ERR_OUT_OF_MEMORY;
     J2K_CUDA(ctx, cudaMemcpyAsync(dj, jobs.data(), jobs.size() * sizeof(j2k_cb_job), cudaMemcpyHostToDevice, ctx->stream));
     J2K_TRY(j2k_clear_device_error(ctx));
-    J2K_TRY(j2k_t1_decode_jobs(ctx, descs, bytes, dj, jobs.size(), w * h, coeff, ctx->stream));
+    J2K_TRY(j2k_t1_decode_jobs(ctx, descs, bytes, dj, jobs.size(), w * h, cbw, cbh, coeff, ctx->stream));
     return j2k_read_device_error(ctx);
     J2K_API_END
 }
@@ -911,8 +911,9 @@ j2k_status j2k_decoder_run_batch(j2k_decoder* d, const j2k_decode_item* items, i
     }
     // tier-1 of every block of every image in one launch
     J2K_TRY(j2k_t1_decode_jobs(ctx, (const j2k_cb_desc*)d->descs.p, (const uint8_t*)d->bytes.p,
-                               (const j2k_cb_job*)d->jobs.p, jobs.size(), coef_total, (int32_t*)d->coef.p, ctx->stream, 0, dpe,
-                               djs));
+                               (const j2k_cb_job*)d->jobs.p, jobs.size(), coef_total,
+                               *std::max_element(cbw.begin(), cbw.end()), *std::max_element(cbh.begin(), cbh.end()),
+                               (int32_t*)d->coef.p, ctx->stream, 0, dpe, djs));
     void* ll0 = j2k_scratch(ctx, SCR_LL0, max_ll0);
     void* ll1 = j2k_scratch(ctx, SCR_LL1, max_ll1);
     if (!ll0 || !ll1) return J2K_ERR_OUT_OF_MEMORY;
@@ -1033,8 +1034,8 @@ j2k_status j2k_decoder_run_codeblocks(j2k_decoder* d, const j2k_cb_desc* descs, 
     J2K_TRY(d->coef.ensure(ctx, n * 4 * ncomp));
     J2K_TRY(d->planes.ensure(ctx, n * 4 * ncomp));
     J2K_TRY(j2k_clear_device_error(ctx));
-    J2K_TRY(j2k_t1_decode_jobs(ctx, dd, db, (const j2k_cb_job*)d->jobs.p, njobs, n * ncomp, (int32_t*)d->coef.p, ctx->stream,
-                               style, dpe));
+    J2K_TRY(j2k_t1_decode_jobs(ctx, dd, db, (const j2k_cb_job*)d->jobs.p, njobs, n * ncomp, cbw, cbh,
+                               (int32_t*)d->coef.p, ctx->stream, style, dpe));
     std::vector<float> steps;
     if (d->lossy) {
         if (p && p->steps) steps.assign(p->steps, p->steps + 3 * levels + 1);

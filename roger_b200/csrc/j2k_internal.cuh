@@ -262,9 +262,10 @@ constexpr int J2K_TRUNC_EXTRA = 4;  // bytes kept beyond those produced at a pla
 // style / pass_ends (device, J2K_PASS_STRIDE per job) locate the codeword segments of styled
 // blocks; style 0 decodes one segment of descs[i].length bytes.  job_style (device, one byte per
 // job, optional) gives each job its own style (pass ends then needed for every job).  samples: the
-// samples of all jobs together (the kernel's launch shape follows from it).
+// samples of all jobs together, cbw x cbh: no job's block is wider or higher (the kernel's form and
+// launch shape follow from them).
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
-                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int32_t* coeff,
+                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int cbw, int cbh, int32_t* coeff,
                               cudaStream_t st, int style = 0, const uint32_t* pass_ends = nullptr,
                               const uint8_t* job_style = nullptr);
 

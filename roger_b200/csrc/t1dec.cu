@@ -897,21 +897,24 @@ static j2k_status launch_steps(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc*
     return J2K_OK;
 }
 
-// Blocks per warp by the work there is, as a number of full blocks of 4096 samples: one while those
-// would be resident at once that way (16 an SM), two up to 40 an SM, four for more (the long blocks
-// get warps of their own as far as all still fit).  A block runs fastest alone; sharing a warp saves
-// instructions, which counts once the ALU pipes are full.  Host to host on B200, 1 / 2 / 4 / 8 blocks
-// per warp: 70 blocks of a 512 x 512 gray image 5.5 ms, with two 7.6, four 10.2; 777 of 1024 x 1024
-// colour 6.7, 8.4, 10.4; 24 images of mixed sizes and block sizes (5071 blocks, the work of 1590)
-// 11.0 / 11.2 / 13.6 / 17.5; 3072 blocks of 2048 x 2048 colour 12.4 / 10.0 / 11.1 / 13.9; 12288 blocks
-// of 4096 x 4096 colour 42 / 32 / 20.0 / 21.6.
-static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t samples) {
-    const size_t full = samples / 4096, sms = (size_t)ctx->sm_count;
-    return full <= 16 * sms ? 1 : (full <= 40 * sms ? 2 : 4);
+// Blocks per warp by the work there is, as a number of blocks of the largest one's size: one while
+// those would be resident at once that way (16 an SM), two up to 40 an SM, four for more (the long
+// blocks get warps of their own as far as all still fit).  A block runs fastest alone; sharing a warp
+// saves instructions, which counts once the ALU pipes are full, and that is a matter of how many
+// blocks wait behind one another, not of how large they are.  Host to host on B200, 1 / 2 / 4 / 8
+// blocks per warp: 70 blocks of a 512 x 512 gray image 5.5 ms, with two 7.6, four 10.2; 777 of
+// 1024 x 1024 colour 6.7, 8.4, 10.4; 24 images of mixed sizes and block sizes (the work of 1590 largest
+// blocks) 11.0 / 11.2 / 13.6 / 17.5; 3072 blocks of 2048 x 2048 colour 12.4 / 10.0 / 11.1 / 13.9; 12288
+// blocks of 4096 x 4096 colour 42 / 32 / 20.0 / 21.6.  Smaller blocks, 1 / 2 / 4 / 8: 3072 of 32 x 32
+// (1024 x 1024 colour) 4.0 / 3.5 / 3.8 / 4.7; 12288 of 32 x 32 (2048 x 2048) 14.9 / 11.8 / 8.5 / 9.7; 4096
+// of 16 x 16 (1024 x 1024 gray) 1.45 / 1.24 / 1.36 / 1.57; 12288 of 16 x 16 4.1 / 3.2 / 2.2 / 2.5.
+static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t samples, int cbw, int cbh) {
+    const size_t n = samples / ((size_t)cbw * cbh), sms = (size_t)ctx->sm_count;
+    return n <= 16 * sms ? 1 : (n <= 40 * sms ? 2 : 4);
 }
 
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
-                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int32_t* coeff,
+                              const j2k_cb_job* d_jobs, size_t njobs, size_t samples, int cbw, int cbh, int32_t* coeff,
                               cudaStream_t st, int style, const uint32_t* pass_ends, const uint8_t* job_style) {
     if (njobs == 0) return J2K_OK;
     if ((style || job_style) && !pass_ends)
@@ -926,7 +929,7 @@ j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint
         default: break;
         }
     }
-    const int L = forced < 0 ? stripe_blocks_per_warp(ctx, samples)
+    const int L = forced < 0 ? stripe_blocks_per_warp(ctx, samples, cbw, cbh)
                              : (forced <= 1 ? 1 : (forced == 2 ? 2 : (forced <= 4 ? 4 : (forced <= 8 ? 8 : 16))));
     const uint32_t *ord = nullptr, *keys = nullptr;
     if (ctx->t1d_order && njobs > (size_t)L) {

@@ -8,6 +8,7 @@ import torch
 from oracle import oracle as O
 from roger_b200 import codec as C
 from roger_b200 import synth
+from roger_b200._lib import lib
 
 from test_gpu_t1_symbols import _contents
 
@@ -52,3 +53,23 @@ def test_no_shape_encodes_much_slower(picture, shape, other, most):
     enc = C.OCLEncoder(ctx=C.Context(0))
     t = [_time(lambda: enc.run_rgb(picture, levels=5, cbw=cw, cbh=ch)) for cw, ch in (shape, other)]
     assert t[0] < most * t[1], t
+
+
+def _decoding(img, cbw, cbh, lanes=None, lossy=False):
+    """A call that decodes img coded with blocks of cbw x cbh, with the tuned number of blocks per warp."""
+    h, w, n = img.shape
+    enc = C.OCLEncoder(ctx=C.Context(0), lossy=lossy).run_rgb(img, levels=5, cbw=cbw, cbh=cbh)
+    d, b = [np.array(v) for v in enc.get_codeblocks()]
+    ctx = C.Context(0)
+    if lanes is not None:
+        assert lib().j2k_ctx_set_tuning(ctx.h, 10, lanes) == 0
+    dec, out = C.OCLDecoder(ctx=ctx, lossy=lossy), torch.empty((h, w, n), dtype=torch.uint8, pin_memory=True).numpy()
+    return lambda: dec.run(d, b, w, h, n, levels=5, cbw=cbw, cbh=cbh, out=out)
+
+
+# with the work counted in blocks of 64 x 64: 2.0 and 1.5; in blocks of the largest one's size 1.0
+@pytest.mark.parametrize("size,cb", [(1024, 16), (2048, 32)])
+def test_blocks_per_warp_fit_small_blocks(size, cb):
+    img = torch.from_numpy(synth.rgb(size, size, (1, 2, 3, 4))).cuda()
+    t = [_time(_decoding(img, cb, cb, lanes)) for lanes in (None, 2, 4)]
+    assert t[0] < 1.2 * min(t[1:]), t
