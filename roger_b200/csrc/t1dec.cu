@@ -2,7 +2,7 @@
 //
 // The reference has no decoder for this stage (src/OCLDecoder.cpp:35-38 runs only the "reverse"
 // DWT).  Decoding is serial per code-block: every context depends on the bits decoded before it.
-// The kernel runs one code-block per lane, 1, 2 or 4 (8, 16 by tuning) in a warp, and takes all
+// The kernel runs one code-block per lane, 1 to 16 in a warp, and takes all
 // work that is not a block's own serial chain out of the lanes' loops (t1dec_stripe.cuh).  What
 // bounds it: the chain of dependent instructions per symbol (about 91 warp instructions and 360
 // cycles a symbol with one block per warp), and with 4 blocks per warp the ALU pipe, since the lanes
@@ -287,25 +287,25 @@ __host__ __device__ __forceinline__ int32_t cut_half(int numbps, int npasses) {
     return 0;
 }
 
-// Warps per CTA of the stripe decoder: with 4 or 8 blocks per warp one CTA's state fills an SM's
-// shared memory (84 or 88 blocks; the 12288 blocks of a 4096 x 4096 colour image are then resident
-// at once on 148 SMs).
-template <int L>
+// Warps per CTA of the stripe decoder for L blocks per warp of Q words a stripe: with 4 or 8 blocks of
+// 8 words one CTA's state fills an SM's shared memory (84 or 88 blocks; the 12288 blocks of a
+// 4096 x 4096 colour image are then resident at once on 148 SMs).
+template <int L, int Q>
 __host__ __device__ constexpr int stripe_warps() {
-    return L == 1 ? 16 : (L == 2 ? 20 : (L == 4 ? 21 : (L == 8 ? 11 : 5)));
+    return Q == 1 ? 24 : L == 1 ? 16 : (L == 2 ? 20 : (L == 4 ? 21 : (L == 8 ? 11 : 5)));
 }
 constexpr size_t kStripeTablesBytes = (sizeof(StripeTables) + 15) & ~(size_t)15;
-template <int L>
+template <int L, int Q>
 __host__ __device__ constexpr size_t stripe_smem_bytes(int warps) {
-    return kStripeTablesBytes + (size_t)warps * stripe_state_words<L>() * 4;
+    return kStripeTablesBytes + (size_t)warps * stripe_state_words<L, Q>() * 4;
 }
 
-// L code-blocks per warp, one per lane (t1dec_stripe.cuh).  Groups of L consecutive blocks of
+// L code-blocks per warp, one per lane, of at most 8 * Q columns (t1dec_stripe.cuh).  Groups of L consecutive blocks of
 // `order` (longest codewords first) go to the warps of all CTAs in turn, then from a queue.  Blocks
 // of more than half the longest codeword (keys: the lengths in that order) get a warp of their own,
 // at most `alone` of them: a block runs fastest alone, and the others end before it anyway.
-template <bool STYLED, int L>
-__global__ void __launch_bounds__(32 * stripe_warps<L>(), 1)
+template <bool STYLED, int L, int Q>
+__global__ void __launch_bounds__(32 * stripe_warps<L, Q>(), 1)
 t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __restrict__ bytes,
                         const j2k_cb_job* __restrict__ jobs, int njobs, int32_t* __restrict__ coeff,
                         uint32_t* __restrict__ err, int style, const uint32_t* __restrict__ pass_ends,
@@ -316,8 +316,9 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
     for (int i = threadIdx.x; i < 4 * 512; i += blockDim.x) fill_stripe_tables_entry(tabs, i);
     __syncthreads();
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const StripeState<L> S{reinterpret_cast<uint32_t*>(dsm + kStripeTablesBytes) + wid * stripe_state_words<L>()};
-    constexpr int R = (8 * L + 31) / 32;  // rounds of 32 (block, word) items per stripe
+    const StripeState<L, Q> S{reinterpret_cast<uint32_t*>(dsm + kStripeTablesBytes) + wid * stripe_state_words<L, Q>()};
+    constexpr int R = (Q * L + 31) / 32;  // rounds of 32 (block, word) items per stripe
+    constexpr int WX = Q == 1 ? 8 : 32, WY = 32 / WX;  // columns and rows of a block that the warp takes at a time
     if (L > 1 && alone > 0) {  // the number of leading keys above half the first one
         const uint32_t half = keys[0] / 2;
         int lo = 0, hi = alone;  // it is in lo..hi
@@ -342,35 +343,38 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
         if (lane < nb) {
             J = jobs[jid];
             D = descs[jid];
-            ok = dec_job_ok(J, D, STYLED);
+            ok = dec_job_ok(J, D, STYLED) && J.cw <= 8 * Q;
             if (!ok) atomicCAS(err, 0u, (uint32_t)J2K_DEVERR_BAD_JOB);
         }
         const unsigned okmask = __ballot_sync(~0u, ok);
-        for (int i = lane; i < kStripeBitmapWords * L; i += 32) S.w[i] = 0;
+        for (int i = lane; i < S.kCols * L; i += 32) S.w[i] = 0;
+        if (Q < 8)  // (only the bytes of words that there are get written below)
+            for (int i = lane; i < 2 * L; i += 32) S.colset(i & 1, i >> 1) = 0;
         for (int b = 0; b < nb; ++b) {
             if (!((okmask >> b) & 1)) continue;
             const int cw = __shfl_sync(~0u, (int)J.cw, b), ch = __shfl_sync(~0u, (int)J.ch, b);
             const size_t pitch = __shfl_sync(~0u, J.pitch, b);
             int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
-            for (int r = 0; r < ch; ++r)
-                for (int x = lane; x < cw; x += 32) blk[(size_t)r * pitch + x] = 0;
+            for (int r = lane / WX; r < ch; r += WY)
+                for (int x = lane % WX; x < cw; x += WX) blk[(size_t)r * pitch + x] = 0;
         }
         // this lane's block, and the sizes and pass counts of the blocks of its items
         const int np = ok && D.numbps > 0 ? min((int)D.npasses, 3 * (int)D.numbps - 2) : 0;
-        StripeLane<L> me{S, LaneMem<L>(S, tabs, J.orient & 3, lane < L ? lane : 0), lane, J.cw, J.ch, {}, {}, false};
+        StripeLane<L, Q> me{S,    LaneMem<L, Q>(S, tabs, J.orient & 3, lane < L ? lane : 0),
+                            lane, J.cw, J.ch, {}, {}, false};
         int icw[R], ich[R], inp[R], inb[R];
         uint32_t ipitch[R];
         int32_t* iblk[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int i = lane + 32 * r, b = (i >> 3) & 31;
+            const int i = lane + 32 * r, b = (i / Q) & 31;
             icw[r] = __shfl_sync(~0u, (int)J.cw, b);
             ich[r] = __shfl_sync(~0u, (int)J.ch, b);
             inp[r] = __shfl_sync(~0u, np, b);
             inb[r] = __shfl_sync(~0u, (int)D.numbps, b);
             ipitch[r] = __shfl_sync(~0u, J.pitch, b);
             iblk[r] = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
-            if (i >= 8 * L) inp[r] = 0;
+            if (i >= Q * L) inp[r] = 0;
         }
         const int pmax = __reduce_max_sync(~0u, np > 0 ? (int)D.numbps : 0);
         const int smax = (__reduce_max_sync(~0u, np > 0 ? (int)J.ch : 0) + 3) >> 2;
@@ -395,11 +399,13 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
                 for (int r = 0; r < R; ++r) {
                     const int i = lane + 32 * r;
                     if (ion[r] && 4 * s < ich[r]) {
-                        if (kind == kPassMR) stripe_prepare_mr<L>(S, s, i & 7, i >> 3, icw[r]);
-                        else stripe_prepare_zc<L>(S, kind, s, i & 7, i >> 3, icw[r], stripe_rows(ich[r], s));
+                        if (kind == kPassMR) stripe_prepare_mr(S, s, i % Q, i / Q, icw[r]);
+                        else stripe_prepare_zc(S, kind, s, i % Q, i / Q, icw[r], stripe_rows(ich[r], s));
                     }
                 }
                 __syncwarp();
+                // (with one word a stripe, preparing and finishing it costs as much as its symbols)
+                if (Q == 1 && !__any_sync(~0u, on && 4 * s < me.ch && S.colset(0, lane) != 0)) continue;
                 if (on && 4 * s < me.ch) {
                     const uint32_t rv = stripe_rows(me.ch, s);
                     if (kind == kPassSP) me.template decode_zc<STYLED, kPassSP>(rv);
@@ -412,9 +418,9 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
                     const int i = lane + 32 * r;
                     if (ion[r] && 4 * s < ich[r]) {
                         const uint32_t ones = kind == kPassMR
-                                                  ? stripe_finish_mr<L>(S, s, i & 7, i >> 3, icw[r])
-                                                  : stripe_finish_zc<L>(S, kind, s, i & 7, i >> 3, icw[r]);
-                        stripe_add_bits(ones, iblk[r], ipitch[r], s, i & 7, p);
+                                                  ? stripe_finish_mr(S, s, i % Q, i / Q, icw[r])
+                                                  : stripe_finish_zc(S, kind, s, i % Q, i / Q, icw[r]);
+                        stripe_add_bits(ones, iblk[r], ipitch[r], s, i % Q, p);
                     }
                 }
                 __syncwarp();
@@ -428,8 +434,8 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
             const size_t pitch = __shfl_sync(~0u, J.pitch, b);
             int32_t* blk = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
             const int32_t half = __shfl_sync(~0u, my_half, b);
-            for (int r = 0; r < ch; ++r)
-                for (int x = lane; x < cw; x += 32) {
+            for (int r = lane / WX; r < ch; r += WY)
+                for (int x = lane % WX; x < cw; x += WX) {
                     const int sh = 4 * (x & 7) + (r & 3);
                     int32_t v = __ldcg(blk + (size_t)r * pitch + x);
                     if ((S.sig(r >> 2, x >> 3, b) >> sh) & 1) v += half;
@@ -726,7 +732,7 @@ t1_decode_steps_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __r
 // Host execution of the device decoder logic for one block (used by the test suite): the stripe
 // decoder that the default kernel runs, its warp-wide parts one item after another, or (steps) the
 // one-symbol-per-step loop of J2K_TUNE_T1D_STEPS.
-template <bool STYLED>
+template <bool STYLED, int Q>
 static void decode_stripes_host(const uint8_t* data, int len, int numbps, int npasses, int orient, int cw, int ch,
                                 int32_t* out, size_t pitch, int style, const uint32_t* pe) {
     static const StripeTables T = [] {  // built once, thread-safely
@@ -734,25 +740,25 @@ static void decode_stripes_host(const uint8_t* data, int len, int numbps, int np
         for (int i = 0; i < 4 * 512; ++i) fill_stripe_tables_entry(t, i);
         return t;
     }();
-    uint32_t words[stripe_state_words<1>()] = {};
-    const StripeState<1> S{words};
-    StripeLane<1> me{S, LaneMem<1>(S, T, orient, 0), 0, cw, ch, {}, {}, false};
+    uint32_t words[stripe_state_words<1, Q>()] = {};
+    const StripeState<1, Q> S{words};
+    StripeLane<1, Q> me{S, LaneMem<1, Q>(S, T, orient, 0), 0, cw, ch, {}, {}, false};
     const int np = std::min(npasses, 3 * numbps - 2), ns = (ch + 3) / 4;
     for (int q = 0; q < np; ++q) {
         const int kind = q == 0 ? kPassCU : (q + 2) % 3, p = numbps - 1 - (q + 2) / 3;
         me.template begin<STYLED>(q, npasses, data, len, style, pe);
         for (int s = 0; s < ns; ++s) {
             const uint32_t rv = stripe_rows(ch, s);
-            for (int i = 0; i < 8; ++i) {
-                if (kind == kPassMR) stripe_prepare_mr<1>(S, s, i, 0, cw);
-                else stripe_prepare_zc<1>(S, kind, s, i, 0, cw, rv);
+            for (int i = 0; i < Q; ++i) {
+                if (kind == kPassMR) stripe_prepare_mr(S, s, i, 0, cw);
+                else stripe_prepare_zc(S, kind, s, i, 0, cw, rv);
             }
             if (kind == kPassSP) me.template decode_zc<STYLED, kPassSP>(rv);
             else if (kind == kPassMR) me.template decode_mr<STYLED>();
             else me.template decode_zc<STYLED, kPassCU>(rv);
-            for (int i = 0; i < 8; ++i) {
-                const uint32_t ones = kind == kPassMR ? stripe_finish_mr<1>(S, s, i, 0, cw)
-                                                      : stripe_finish_zc<1>(S, kind, s, i, 0, cw);
+            for (int i = 0; i < Q; ++i) {
+                const uint32_t ones = kind == kPassMR ? stripe_finish_mr(S, s, i, 0, cw)
+                                                      : stripe_finish_zc(S, kind, s, i, 0, cw);
                 stripe_add_bits(ones, out, pitch, s, i, p);
             }
         }
@@ -772,7 +778,8 @@ static int decode_block_host(const uint8_t* data, int len, int numbps, int npass
         for (int x = 0; x < cw; ++x) out[(size_t)y * pitch + x] = 0;
     if (numbps == 0 || npasses == 0) return 0;
     if (!steps) {
-        decode_stripes_host<false>(data, len, numbps, npasses, orient, cw, ch, out, pitch, 0, nullptr);
+        const auto decode = cw <= 8 ? decode_stripes_host<false, 1> : decode_stripes_host<false, 8>;
+        decode(data, len, numbps, npasses, orient, cw, ch, out, pitch, 0, nullptr);
         return 0;
     }
     DecSmem S;
@@ -811,12 +818,13 @@ extern "C" int j2k_t1_decode_block_styled_host(const uint8_t* data, int len, con
         return -1;
     for (int y = 0; y < ch; ++y)
         for (int x = 0; x < cw; ++x) out[(size_t)y * pitch + x] = 0;
+    const auto decode = cw <= 8 ? decode_stripes_host<true, 1> : decode_stripes_host<true, 8>;
     if (numbps > 0 && npasses > 0)
-        decode_stripes_host<true>(data, len, numbps, npasses, orient, cw, ch, out, pitch, style, pass_ends);
+        decode(data, len, numbps, npasses, orient, cw, ch, out, pitch, style, pass_ends);
     return 0;
 }
 
-template <bool STYLED, int L>
+template <bool STYLED, int L, int Q>
 static j2k_status launch_stripe(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc* descs, const uint8_t* bytes,
                                 const j2k_cb_job* d_jobs, size_t njobs, int32_t* coeff, int style,
                                 const uint32_t* pass_ends, const uint8_t* job_style, const uint32_t* order,
@@ -824,22 +832,22 @@ static j2k_status launch_stripe(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc
     static std::atomic<uint64_t> attr_set{0};  // devices whose attribute is set, per instantiation
     const uint64_t bit = 1ull << (ctx->device & 63);
     if (!(attr_set.load() & bit)) {
-        J2K_CUDA(ctx, cudaFuncSetAttribute(t1_decode_stripe_kernel<STYLED, L>,
+        J2K_CUDA(ctx, cudaFuncSetAttribute(t1_decode_stripe_kernel<STYLED, L, Q>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)stripe_smem_bytes<L>(stripe_warps<L>())));
+                                           (int)stripe_smem_bytes<L, Q>(stripe_warps<L, Q>())));
         attr_set.fetch_or(bit);
     }
     uint32_t* queue = (uint32_t*)j2k_scratch(ctx, SCR_DECQ, 4);
     if (!queue) return J2K_ERR_OUT_OF_MEMORY;
     J2K_CUDA(ctx, cudaMemsetAsync(queue, 0, 4, st));
     // the groups spread over the SMs first, then over the warps of a CTA
-    const size_t sms = (size_t)ctx->sm_count, resident = sms * stripe_warps<L>();
+    const size_t sms = (size_t)ctx->sm_count, resident = sms * stripe_warps<L, Q>();
     // blocks that can have a warp alone with all blocks still resident at once
     const size_t alone = L > 1 && keys && resident * L > njobs ? std::min(njobs, (resident * L - njobs) / (L - 1)) : 0;
     const size_t groups = alone + (njobs - alone + L - 1) / L;
     const unsigned grid = (unsigned)std::min(groups, sms);
-    const int warps = (int)std::min<size_t>((groups + grid - 1) / grid, (size_t)stripe_warps<L>());
-    t1_decode_stripe_kernel<STYLED, L><<<grid, 32 * warps, stripe_smem_bytes<L>(warps), st>>>(
+    const int warps = (int)std::min<size_t>((groups + grid - 1) / grid, (size_t)stripe_warps<L, Q>());
+    t1_decode_stripe_kernel<STYLED, L, Q><<<grid, 32 * warps, stripe_smem_bytes<L, Q>(warps), st>>>(
         descs, bytes, d_jobs, (int)njobs, coeff, ctx->d_err, style, pass_ends, job_style, order, keys, (int)alone, queue);
     J2K_CUDA(ctx, cudaGetLastError());
     return J2K_OK;
@@ -908,9 +916,26 @@ static j2k_status launch_steps(j2k_ctx* ctx, cudaStream_t st, const j2k_cb_desc*
 // blocks of 4096 x 4096 colour 42 / 32 / 20.0 / 21.6.  Smaller blocks, 1 / 2 / 4 / 8: 3072 of 32 x 32
 // (1024 x 1024 colour) 4.0 / 3.5 / 3.8 / 4.7; 12288 of 32 x 32 (2048 x 2048) 14.9 / 11.8 / 8.5 / 9.7; 4096
 // of 16 x 16 (1024 x 1024 gray) 1.45 / 1.24 / 1.36 / 1.57; 12288 of 16 x 16 4.1 / 3.2 / 2.2 / 2.5.
+// Blocks up to 8 wide are one word a stripe, with little state, few symbols at a time and the more so
+// as they are many: up to 16 a warp.  Host to host, 1 / 2 / 4 / 8 / 16: 4096 of 8 x 32 (1024 x 1024 gray)
+// 1.59 / 1.41 / 1.43 / 1.56 / 1.71; 6168 of 8 x 64 (1024 x 1024 colour) 4.0 / 3.3 / 3.6 / 3.6 / 4.1; 12336
+// of 4 x 64 4.3 / 3.2 / 2.6 / 2.6 / 2.8; 24576 of 8 x 64 (2048 x 2048 colour) 16.6 / 13.0 / 9.4 / 7.1 / 7.3;
+// 49152 of 8 x 32 16.5 / 13.0 / 10.2 / 7.4 / 6.4; 196608 of 8 x 8 16.5 / 12.2 / 9.6 / 7.5 / 6.1.
 static int stripe_blocks_per_warp(const j2k_ctx* ctx, size_t samples, int cbw, int cbh) {
     const size_t n = samples / ((size_t)cbw * cbh), sms = (size_t)ctx->sm_count;
-    return n <= 16 * sms ? 1 : (n <= 40 * sms ? 2 : 4);
+    if (cbw > 8) return n <= 16 * sms ? 1 : (n <= 40 * sms ? 2 : 4);
+    return n <= 16 * sms ? 1 : (n <= 48 * sms ? 2 : (n <= 96 * sms ? 4 : (n <= 256 * sms ? 8 : 16)));
+}
+
+template <bool STYLED, int Q, class... Args>
+static j2k_status launch_stripe_lanes(int lanes, Args... args) {
+    switch (lanes) {
+    case 1: return launch_stripe<STYLED, 1, Q>(args...);
+    case 2: return launch_stripe<STYLED, 2, Q>(args...);
+    case 4: return launch_stripe<STYLED, 4, Q>(args...);
+    case 8: return launch_stripe<STYLED, 8, Q>(args...);
+    default: return launch_stripe<STYLED, 16, Q>(args...);
+    }
 }
 
 j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint8_t* bytes,
@@ -936,16 +961,9 @@ j2k_status j2k_t1_decode_jobs(j2k_ctx* ctx, const j2k_cb_desc* descs, const uint
         ord = decode_order(ctx, st, descs, njobs, &keys);
         if (!ord) return J2K_ERR_OUT_OF_MEMORY;
     }
-    switch ((styled ? 100 : 0) + L) {
-    case 1: return launch_stripe<false, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
-    case 2: return launch_stripe<false, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
-    case 4: return launch_stripe<false, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
-    case 8: return launch_stripe<false, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
-    case 16: return launch_stripe<false, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, 0, nullptr, nullptr, ord, keys);
-    case 101: return launch_stripe<true, 1>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
-    case 102: return launch_stripe<true, 2>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
-    case 104: return launch_stripe<true, 4>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
-    case 108: return launch_stripe<true, 8>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
-    default: return launch_stripe<true, 16>(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
-    }
+    const auto go = [&](auto... a) {
+        return styled ? (cbw <= 8 ? launch_stripe_lanes<true, 1>(L, a...) : launch_stripe_lanes<true, 8>(L, a...))
+                      : (cbw <= 8 ? launch_stripe_lanes<false, 1>(L, a...) : launch_stripe_lanes<false, 8>(L, a...));
+    };
+    return go(ctx, st, descs, bytes, d_jobs, njobs, coeff, style, pass_ends, job_style, ord, keys);
 }

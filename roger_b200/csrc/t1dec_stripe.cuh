@@ -12,7 +12,10 @@
 //            registers (a sample that turns significant reaches the next column as a carry);
 //   finish   turns the column words back into the bitmaps.
 // The lanes of a warp go through the bit-planes, passes and stripes together, so that they meet on
-// the same instructions.
+// the same instructions.  A stripe of a block is Q words of 8 columns: 8, or 1 for blocks that are no
+// wider.  Those in the form for 64 columns left seven eighths of the lanes idle while a stripe was
+// prepared and finished: host to host on B200, 4096 x 4096 colour with blocks of 4 x 64 42.7 -> 15.4 ms,
+// 8 x 8 38.7 -> 16.5, 2048 x 2048 with 4 x 64 12.0 -> 6.3, 1024 x 1024 with 8 x 64 3.6 -> 3.2.
 //
 // Bitmaps: one word per 8 columns of a stripe, a nibble per column (bit j = stripe row j).
 // Column word of the propagation and cleanup passes:
@@ -62,26 +65,26 @@ struct alignas(8) MqdState {
 };
 
 // Words of a warp's L blocks, interleaved by block so that the lanes' accesses fall in distinct
-// banks: four bitmaps of 16 stripes x 8 words, 64 column words, 19 context states of 2 words, 2
-// words of column sets.
-template <int L>
+// banks: four bitmaps of 16 stripes x Q words (blocks of up to 8 * Q columns), 8 * Q column words, 19
+// context states of 2 words, 2 words of column sets.
+template <int L, int Q>
 struct StripeState {
+    static constexpr int kMap = 16 * Q, kCols = 4 * kMap, kCtx = kCols + 8 * Q, kSets = kCtx + 38, kWords = kSets + 2;
     uint32_t* w;
-    T1D_HD uint32_t& sig(int s, int q, int b) const { return w[(s * 8 + q) * L + b]; }
-    T1D_HD uint32_t& neg(int s, int q, int b) const { return w[(128 + s * 8 + q) * L + b]; }
-    T1D_HD uint32_t& vis(int s, int q, int b) const { return w[(256 + s * 8 + q) * L + b]; }
-    T1D_HD uint32_t& ref(int s, int q, int b) const { return w[(384 + s * 8 + q) * L + b]; }
-    T1D_HD uint32_t& col(int x, int b) const { return w[(512 + x) * L + b]; }
-    T1D_HD MqdState& ctx(int k, int b) const { return reinterpret_cast<MqdState*>(w + 576 * L)[k * L + b]; }
+    T1D_HD uint32_t& sig(int s, int q, int b) const { return w[(s * Q + q) * L + b]; }
+    T1D_HD uint32_t& neg(int s, int q, int b) const { return w[(kMap + s * Q + q) * L + b]; }
+    T1D_HD uint32_t& vis(int s, int q, int b) const { return w[(2 * kMap + s * Q + q) * L + b]; }
+    T1D_HD uint32_t& ref(int s, int q, int b) const { return w[(3 * kMap + s * Q + q) * L + b]; }
+    T1D_HD uint32_t& col(int x, int b) const { return w[(kCols + x) * L + b]; }
+    T1D_HD MqdState& ctx(int k, int b) const { return reinterpret_cast<MqdState*>(w + kCtx * L)[k * L + b]; }
     // column set of block b, a byte per 8 columns (the bytes of one block are contiguous)
-    T1D_HD uint8_t* cols(int b) const { return reinterpret_cast<uint8_t*>(w + 614 * L) + 8 * b; }
-    T1D_HD uint32_t& colset(int h, int b) const { return (w + 614 * L)[2 * b + h]; }
+    T1D_HD uint8_t* cols(int b) const { return reinterpret_cast<uint8_t*>(w + kSets * L) + 8 * b; }
+    T1D_HD uint32_t& colset(int h, int b) const { return (w + kSets * L)[2 * b + h]; }
 };
-template <int L>
+template <int L, int Q>
 __host__ __device__ constexpr int stripe_state_words() {
-    return 616 * L;
+    return StripeState<L, Q>::kWords * L;
 }
-constexpr int kStripeBitmapWords = 512;  // per block, cleared at the start
 
 enum : int { kPassSP = 0, kPassMR = 1, kPassCU = 2 };
 
@@ -94,8 +97,8 @@ T1D_HD uint32_t near_rows(uint32_t W) {
 
 // prepare: word q (8 columns) of stripe s of block b, whose rows below the block are outside rv (the
 // stripe's valid rows at 3k) and whose width is cw
-template <int L>
-T1D_HD void stripe_prepare_zc(const StripeState<L>& S, int kind, int s, int q, int b, int cw, uint32_t rv) {
+template <int L, int Q>
+T1D_HD void stripe_prepare_zc(const StripeState<L, Q>& S, int kind, int s, int q, int b, int cw, uint32_t rv) {
     if (8 * q >= cw) {
         S.cols(b)[q] = 0;
         return;
@@ -105,7 +108,7 @@ T1D_HD void stripe_prepare_zc(const StripeState<L>& S, int kind, int s, int q, i
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            const bool in = s + i >= 1 && s + i <= 16 && q + j >= 1 && q + j <= 8;
+            const bool in = s + i >= 1 && s + i <= 16 && (Q > 1 ? q + j >= 1 && q + j <= Q : j == 1);
             sg[i][j] = in ? S.sig(s + i - 1, q + j - 1, b) : 0u;
             ng[i][j] = in ? S.neg(s + i - 1, q + j - 1, b) : 0u;
         }
@@ -124,6 +127,7 @@ T1D_HD void stripe_prepare_zc(const StripeState<L>& S, int kind, int s, int q, i
     uint32_t v0 = sig_col(0), v1 = sig_col(1), n0 = neg_col(0), n1 = neg_col(1), set = 0;
 #pragma unroll
     for (int i = 1; i <= 8; ++i) {
+        if (Q == 1 && i > cw) break;
         const uint32_t v2 = sig_col(i + 1), n2 = neg_col(i + 1);
         const int sh = 4 * (i - 1);
         const uint32_t vert = ((ng[0][1] >> (sh + 3)) & 1u) | (((own_ng >> sh) & 15u) << 1) |
@@ -141,12 +145,13 @@ T1D_HD void stripe_prepare_zc(const StripeState<L>& S, int kind, int s, int q, i
     }
     if (cw - 8 * q < 8) set &= (1u << (cw - 8 * q)) - 1u;
     S.cols(b)[q] = (uint8_t)set;
+    if (Q == 1 && kind == kPassSP) S.vis(s, q, b) = 0;  // a stripe without symbols is not finished
 }
 
 // samples of word q that the refinement pass codes (significant before this plane), and the number
 // of those in the words before it: within a word the bits are in coding order already
-template <int L>
-T1D_HD uint32_t stripe_mr_symbols(const StripeState<L>& S, int s, int q, int b, int* before) {
+template <int L, int Q>
+T1D_HD uint32_t stripe_mr_symbols(const StripeState<L, Q>& S, int s, int q, int b, int* before) {
     int n = 0;
     for (int i = 0; i < q; ++i) n += popc32(S.sig(s, i, b) & ~S.vis(s, i, b));
     *before = n;
@@ -156,13 +161,13 @@ T1D_HD uint32_t stripe_mr_symbols(const StripeState<L>& S, int s, int q, int b, 
 // prepare of a refinement stripe: no decision changes another one's context here, so the stripe's
 // labels are listed in coding order (a byte each, in the column words) and their number put in
 // column set word 0
-template <int L>
-T1D_HD void stripe_prepare_mr(const StripeState<L>& S, int s, int q, int b, int cw) {
+template <int L, int Q>
+T1D_HD void stripe_prepare_mr(const StripeState<L, Q>& S, int s, int q, int b, int cw) {
     if (8 * q >= cw) return;
     uint32_t vert = 0, h3[3];
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-        const bool in = q + j >= 1 && q + j <= 8;
+        const bool in = Q > 1 ? q + j >= 1 && q + j <= Q : j == 1;
         const uint32_t m = in ? S.sig(s, q + j - 1, b) : 0u;
         const uint32_t a = in && s > 0 ? S.sig(s - 1, q + j - 1, b) : 0u;
         const uint32_t e = in && s < 15 ? S.sig(s + 1, q + j - 1, b) : 0u;
@@ -187,8 +192,8 @@ T1D_HD void stripe_prepare_mr(const StripeState<L>& S, int s, int q, int b, int 
 }
 
 // finish: the decisions of a refinement stripe (32 to a word, in coding order) back to their samples
-template <int L>
-T1D_HD uint32_t stripe_finish_mr(const StripeState<L>& S, int s, int q, int b, int cw) {
+template <int L, int Q>
+T1D_HD uint32_t stripe_finish_mr(const StripeState<L, Q>& S, int s, int q, int b, int cw) {
     if (8 * q >= cw) return 0;
     int at = 0;
     uint32_t ones = 0;
@@ -199,13 +204,14 @@ T1D_HD uint32_t stripe_finish_mr(const StripeState<L>& S, int s, int q, int b, i
 
 // finish: the column words of a propagation or cleanup stripe back into the bitmaps; returns the
 // samples that turned significant
-template <int L>
-T1D_HD uint32_t stripe_finish_zc(const StripeState<L>& S, int kind, int s, int q, int b, int cw) {
+template <int L, int Q>
+T1D_HD uint32_t stripe_finish_zc(const StripeState<L, Q>& S, int kind, int s, int q, int b, int cw) {
     if (8 * q >= cw) return 0;
     const uint32_t seen = S.cols(b)[q];  // the columns whose word holds visits (stripe_decode)
     uint32_t sg = 0, ng = 0, vs = 0;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
+        if (Q == 1 && i >= cw) break;
         const uint32_t W = S.col(8 * q + i, b);
         sg |= gather4(W >> 4) << (4 * i);
         ng |= ((W >> 23) & 15u) << (4 * i);
@@ -343,11 +349,11 @@ __host__ __device__ inline void fill_stripe_tables_entry(StripeTables& T, int i)
 // What a lane's symbol loops touch: its block's column words and context states and the tables.  On
 // the device 32-bit shared-memory addresses that the compiler cannot see through (it computes the
 // address of a shared array anew for every access otherwise, special-register read included).
-template <int L>
+template <int L, int Q>
 struct LaneMem {
 #ifdef __CUDA_ARCH__
     uint32_t cols, ctxs, zcs, scs, mqs;
-    __device__ __forceinline__ LaneMem(const StripeState<L>& S, const StripeTables& T, int orient, int b)
+    __device__ __forceinline__ LaneMem(const StripeState<L, Q>& S, const StripeTables& T, int orient, int b)
         : cols(addr(&S.col(0, b))), ctxs(addr(&S.ctx(0, b))), zcs(addr(T.zc[orient])), scs(addr(T.sc)), mqs(addr(T.mq)) {
         asm volatile("" : "+r"(cols), "+r"(ctxs), "+r"(zcs), "+r"(scs), "+r"(mqs));
     }
@@ -381,10 +387,10 @@ struct LaneMem {
         return v;
     }
 #else
-    const StripeState<L>& S;
+    const StripeState<L, Q>& S;
     const StripeTables& T;
     int o, b;
-    LaneMem(const StripeState<L>& s, const StripeTables& t, int orient, int blk) : S(s), T(t), o(orient), b(blk) {}
+    LaneMem(const StripeState<L, Q>& s, const StripeTables& t, int orient, int blk) : S(s), T(t), o(orient), b(blk) {}
     uint32_t col(int x) const { return S.col(x, b); }
     void col_set(int x, uint32_t v) const { S.col(x, b) = v; }
     MqdState ctx(uint32_t k) const { return S.ctx((int)k, b); }
@@ -398,10 +404,10 @@ struct LaneMem {
 };
 
 // One lane's block and its coder.
-template <int L>
+template <int L, int Q>
 struct StripeLane {
-    StripeState<L> S;
-    LaneMem<L> mem;
+    StripeState<L, Q> S;
+    LaneMem<L, Q> mem;
     int b, cw, ch;
     MqReg m;
     RawD rd;
@@ -471,7 +477,7 @@ struct StripeLane {
         uint32_t next_set = S.colset(1, b);
         const uint32_t wide_hi = cw >= 64 ? ~0u : (cw > 32 ? (1u << (cw - 32)) - 1u : 0u);
         uint32_t carry = 0;  // what the column before leaves to the next one
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < (Q > 4 ? 2 : 1); ++h) {
             const int x0 = 32 * h;
             uint32_t set = h ? next_set : S.colset(0, b), all = set;
             const uint32_t wide = h ? wide_hi : (cw >= 32 ? ~0u : (1u << cw) - 1u);
@@ -500,7 +506,7 @@ struct StripeLane {
                 for (;;) {
                     // the symbol after a 0: the column's next row, or the next column
                     const uint32_t c2 = run ? 0u : c & (c - 1);
-                    const int nx = ctz32(set) & 31;
+                    const int nx = ctz32(set) & (Q > 4 ? 31 : 8 * Q - 1);
                     const uint32_t Wn = mem.col(x0 + nx) | (nx == x + 1 ? carry : 0u);
                     const uint32_t W2 = c2 ? W : Wn, d2 = c2 ? c2 : candidates<KIND>(Wn, rv);
                     const int k32 = ctz32(d2) & 15;
@@ -595,7 +601,7 @@ struct StripeLane {
         MqdState e = mem.ctx(cx);
         for (int i = 0; i < n; ++i) {
             labels >>= 8;
-            if ((i & 3) == 3) labels = mem.col(((i + 1) >> 2) & 63);
+            if ((i & 3) == 3) labels = mem.col(((i + 1) >> 2) & (8 * Q - 1));
             const uint32_t ncx = min(labels & 31u, 18u);  // (past the last label: any context)
             const MqdState ne = mem.ctx(ncx);
             MqdState up;
