@@ -131,3 +131,19 @@ def test_narrow_blocks_cut_after_any_pass(lanes):
         assert lib().j2k_ctx_set_tuning(ctx.h, 10, lanes) == 0
     got = C.bpc_decode(descs, torch.from_numpy(data).cuda(), 176, 64, 0, cbw=8, cbh=64, ctx=ctx).cpu().numpy()
     assert np.array_equal(got, want)
+
+
+def test_one_large_block_among_many_small_ones():
+    """The blocks per warp follow the many."""
+    imgs = [(synth.gray(512, 512, k), 16) for k in range(30)] + [(synth.gray(64, 64, 99), 64)]
+    streams = [C.OCLEncoder(ctx=C.Context(0)).run_rgb(im, levels=1, cbw=cb, cbh=cb).codestream() for im, cb in imgs]
+    t = []
+    for lanes in (None, 4):
+        ctx = C.Context(0)
+        if lanes is not None:
+            assert lib().j2k_ctx_set_tuning(ctx.h, 10, lanes) == 0
+        dec = C.OCLDecoder(ctx=ctx)
+        t.append(_time(lambda: C.decode_codestreams(streams, decoder=dec)))
+        for (im, _), out in zip(imgs, C.decode_codestreams(streams, decoder=dec)):
+            assert np.array_equal(np.array(out).reshape(im.shape), im)
+    assert t[0] < 1.2 * t[1], t
