@@ -61,8 +61,9 @@ const char* j2k_last_error(const j2k_ctx* ctx);
  * the reference fixed its OpenCL work-group shapes in -D build strings (src/OCLEncoder.cpp:27-29). */
 enum {
     J2K_TUNE_MQ_LANES = 1,   /* MQ kernel: blocks per warp pair (8, 16, 32) after the tiers of
-                                J2K_TUNE_MQ_TIER; left alone, 1 to 32 by the number of blocks */
-    J2K_TUNE_MQ_VARIANT = 2, /* 0 or 1; both run the pair of an interval warp and a code warp */
+                                J2K_TUNE_MQ_TIER; 0 (default): 1 to 32 by the number of blocks */
+    J2K_TUNE_MQ_VARIANT = 2, /* 0 or 1: kept for callers that set it; there is one form, a pair of an
+                                interval warp and a code warp */
     J2K_TUNE_DWT_FAST_TH = 3, /* register-lifting forward DWT tile height: 16 (default), 32, 0 = off */
     J2K_TUNE_DWT_PIPE = 4,    /* 1: that kernel streams bands with cp.async double buffering (default 0) */
     J2K_TUNE_DWT_REG = 5,     /* 1 (default): that kernel loads its columns straight into registers;
@@ -77,8 +78,8 @@ enum {
                                  tiles per plane, one thread-block cluster of 16, 16, 8, 16 CTAs per
                                  plane with the cluster barrier between levels.  0 (default): off */
     J2K_TUNE_T1D_LANES = 10,  /* tier-1 decoder: code-blocks decoded side by side in one warp, one per lane:
-                                 0 (one), 2, 4, 8, 16; 3, 6 and 32 run as 4, 8 and 16.  Left alone, it is 1,
-                                 2 or 4 by the number of samples */
+                                 0 (one), 2, 4, 8, 16; 3, 6 and 32 run as 4, 8 and 16.  -1 (default): 1 to
+                                 16 by the number and size of the blocks */
     J2K_TUNE_T1D_STEPS = 11,  /* 1: with 8, 16 or 32 lanes, unstyled blocks are decoded in a loop of one
                                  symbol per step over 64-bit row masks; 0 (default): stripe by stripe */
     J2K_TUNE_PLANAR = 12,     /* interleaved-to-planar split of contiguous images: 0: 16 pixels per thread;
@@ -259,7 +260,8 @@ j2k_status j2k_encoder_get_codeblocks(j2k_encoder* enc, j2k_cb_desc* descs, size
                                       uint8_t* bytes, size_t cap, size_t* used);
 /* Times the tier-1 MQ schedules (J2K_TUNE_MQ_TIER / _LANES) on the last run's coefficients and
  * keeps the fastest in the encoder's context; the result stays that of the last run.
- * report (optional, 4 ints): tier-0 warps, tier-1 warps, tier-1 blocks per warp, blocks per warp. */
+ * report (optional, 4 ints): tier-0 and tier-1 warp pairs, tier-1 blocks per pair, most blocks per pair
+ * after them (32 for a new context's schedule, 1 to 32 by their number, which is a candidate too). */
 j2k_status j2k_encoder_autotune(j2k_encoder* enc, int reps, int* report);
 /* T.800 codestream (SOC..EOC, one tile, LRCP; one quality layer, or the layers asked for) of the
  * last run.  out NULL: size only. */
@@ -462,7 +464,7 @@ enum {
     J2K_BATCH_TILE97 = 3,        /* same for 9/7 images */
     J2K_BATCH_PHASE_A_ORDER = 4, /* 1: context modelling takes the largest code-blocks first */
     J2K_BATCH_MQ_VARIANT = 5,    /* read-only here; set with j2k_ctx_set_tuning */
-    J2K_BATCH_MQ_LANES = 6,
+    J2K_BATCH_MQ_LANES = 6,      /* the same */
     J2K_BATCH_MQ_TIERS = 7,      /* read-only: 1 when the MQ coder runs the tiered warp schedule */
     J2K_BATCH_GRAPH_KERNELS = 8, /* read-only: kernel launches of one replay of the captured
                                     sequence, this library's own (library sort/scan kernels are
@@ -492,7 +494,8 @@ j2k_status j2k_batch_upload(j2k_batch* b, const uint8_t* const* pixels, int on_d
 j2k_status j2k_batch_set_option(j2k_batch* b, int key, int value);
 j2k_status j2k_batch_get_option(j2k_batch* b, int key, int* value);
 /* Times the tile shapes and code-block-to-warp schedules on this batch and keeps the fastest;
- * report (optional, 5 ints): tile53, tile97, phase-A order, MQ variant, MQ blocks per warp. */
+ * report (optional, 5 ints): tile53, tile97, phase-A order, MQ variant, MQ blocks per warp pair (0: by
+ * their number, a new context's schedule). */
 j2k_status j2k_batch_autotune(j2k_batch* b, int reps, int* report);
 /* Per-image results of the last encode: code-blocks (layout of j2k_encoder_get_codeblocks) and
  * the T.800 codestream. */

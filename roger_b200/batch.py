@@ -129,9 +129,9 @@ class BatchEncoder:
         check(lib().j2k_batch_autotune(self.h, reps, rep), hh)
         tiers = C.c_int()
         check(lib().j2k_batch_get_option(self.h, 7, C.byref(tiers)), hh)
-        mq = "state+code warp pair" if rep[3] else f"one lane per block, {rep[4]} per warp"
-        if tiers.value and not rep[3]:
-            mq += " after the tiers (longest blocks: 1 per warp, then 4 per warp)"
+        mq = f"{rep[4] or '1 to 32, by their number,'} blocks per warp pair"
+        if tiers.value:
+            mq += " after the longest ones, alone in theirs"
         return {"tile53": TILE_NAMES[rep[0]], "tile97": TILE_NAMES[rep[1]],
                 "phase_a_order": "largest-first" if rep[2] else "natural", "mq": mq,
                 "phase_a_ctas_per_sm": self.get_option(10)}

@@ -287,7 +287,9 @@ class OCLEncoder(OCLEncodeDecode):
 
     def autotune(self, reps=2):
         """Times the tier-1 MQ warp schedules on the last run's coefficients and keeps the fastest
-        in this encoder's context (shared with every object on that context)."""
+        in this encoder's context (shared with every object on that context).  A new context's
+        schedule (by the number of blocks, reported as 32 blocks per warp pair, its most) is among
+        them; J2K_TUNE_MQ_LANES 0 returns to it."""
         rep = (C.c_int * 4)()
         hh = self.ctx._bind()
         check(lib().j2k_encoder_autotune(self.h, reps, rep), hh)

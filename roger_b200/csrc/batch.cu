@@ -693,9 +693,10 @@ j2k_status j2k_batch_autotune(j2k_batch* b, int reps, int* report) {
         b->tile_code[f] = best_code;
         if (s == J2K_OK) s = plan_dwt(b);
     }
-    // MQ candidates: {variant, blocks per warp pair, tiered schedule on}; the tiers are the context's
-    // (by default one pair per SM with one block)
-    const int cand[5][3] = {{0, 8, 1}, {0, 16, 1}, {0, 32, 1}, {0, 16, 0}, {0, 32, 0}};
+    // MQ candidates: {blocks per warp pair (0: by their number), tiered schedule on}; the tiers are the
+    // context's (by default one pair per SM with one block).  The first is a new context's.
+    constexpr int kCand = 6;
+    const int cand[kCand][2] = {{0, 1}, {8, 1}, {16, 1}, {32, 1}, {16, 0}, {32, 0}};
     int tw[J2K_MQ_TIERS], tl[J2K_MQ_TIERS];
     std::copy(ctx->mq_tier_warps, ctx->mq_tier_warps + J2K_MQ_TIERS, tw);
     std::copy(ctx->mq_tier_lanes, ctx->mq_tier_lanes + J2K_MQ_TIERS, tl);
@@ -708,18 +709,16 @@ j2k_status j2k_batch_autotune(j2k_batch* b, int reps, int* report) {
     int best_order = 1, best_c = 0;
     float best_t = 1e30f;
     for (int ord = 0; ord < 2 && s == J2K_OK; ++ord)
-        for (int c = 0; c < 5 && s == J2K_OK; ++c) {
+        for (int c = 0; c < kCand && s == J2K_OK; ++c) {
             b->phase_a_order = ord;
-            ctx->mq_variant = cand[c][0];
-            ctx->mq_lanes = cand[c][1];
-            set_tiers(cand[c][2] != 0);
+            ctx->mq_lanes = cand[c][0];
+            set_tiers(cand[c][1] != 0);
             s = time_stage(false, false, true, &t);
             if (s == J2K_OK && t < best_t) { best_t = t; best_order = ord; best_c = c; }
         }
     b->phase_a_order = best_order;
-    ctx->mq_variant = cand[best_c][0];
-    ctx->mq_lanes = cand[best_c][1];
-    set_tiers(cand[best_c][2] != 0);
+    ctx->mq_lanes = cand[best_c][0];
+    set_tiers(cand[best_c][1] != 0);
     // phase A's register budget: 2 or 3 resident CTAs per SM
     {
         int best_occ = ctx->t1a_ctas;

@@ -663,15 +663,14 @@ j2k_status j2k_encoder_autotune(j2k_encoder* e, int reps, int* report) {
         return j2k_fail(ctx, J2K_ERR_INVALID_ARG, "autotune needs the tier-1 result of a run");
     cudaSetDevice(ctx->device);
     reps = std::max(reps, 1);
-    // candidates: {tier-0 warps per SM, tier-1 warps per SM, tier-1 blocks per warp, blocks per
-    // warp after the tiers}; 0 warps: no tier
-    const int cand[8][4] = {{1, 0, 0, 8}, {1, 0, 0, 16}, {1, 0, 0, 32}, {1, 1, 4, 16},
+    // candidates: {tier-0 pairs per SM, tier-1 pairs per SM, tier-1 blocks per pair, blocks per
+    // pair after the tiers (0: by their number)}; 0 pairs: no tier.  The first is a new context's.
+    constexpr int kCand = 9;
+    const int cand[kCand][4] = {{1, 0, 0, 0}, {1, 0, 0, 8}, {1, 0, 0, 16}, {1, 0, 0, 32}, {1, 1, 4, 16},
                             {1, 1, 4, 32}, {1, 2, 4, 16}, {0, 0, 0, 16}, {0, 0, 0, 32}};
     cudaEvent_t e0, e1;
     J2K_CUDA(ctx, cudaEventCreate(&e0));
     J2K_CUDA(ctx, cudaEventCreate(&e1));
-    const int variant = ctx->mq_variant;
-    ctx->mq_variant = 0;
     auto apply = [&](const int* c) {
         for (int k = 0; k < J2K_MQ_TIERS; ++k) ctx->mq_tier_warps[k] = 0, ctx->mq_tier_lanes[k] = 0;
         if (c[0]) ctx->mq_tier_warps[0] = c[0] * ctx->sm_count, ctx->mq_tier_lanes[0] = 1;
@@ -681,7 +680,7 @@ j2k_status j2k_encoder_autotune(j2k_encoder* e, int reps, int* report) {
     j2k_status s = J2K_OK;
     int best = 0;
     float best_t = 1e30f;
-    for (int c = 0; c < 8 && s == J2K_OK; ++c) {
+    for (int c = 0; c < kCand && s == J2K_OK; ++c) {
         apply(cand[c]);
         float tmin = 1e30f;
         for (int r = 0; r <= reps && s == J2K_OK; ++r) {  // the first run warms up
@@ -699,12 +698,11 @@ j2k_status j2k_encoder_autotune(j2k_encoder* e, int reps, int* report) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     apply(cand[best]);
-    ctx->mq_variant = variant;
     if (report) {
         report[0] = ctx->mq_tier_warps[0];
         report[1] = ctx->mq_tier_warps[1];
         report[2] = ctx->mq_tier_lanes[1];
-        report[3] = ctx->mq_lanes;
+        report[3] = ctx->mq_lanes ? ctx->mq_lanes : 32;
     }
     // the result again, as the encoder left it (rate control included)
     e->packed_ok = false;

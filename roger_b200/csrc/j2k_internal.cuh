@@ -76,7 +76,7 @@ struct j2k_ctx {
     size_t h_pinned_size = 0;
     int sm_count = 148;
     int mq_lanes = 0;            // tier-1 MQ: code-blocks per warp pair after the tiers (0: by their number)
-    int mq_variant = 0;          // tier-1 MQ form asked for (one form is left)
+    int mq_variant = 0;          // J2K_TUNE_MQ_VARIANT as set (there is one form)
     int dwt_fast_th = 16;        // fast level-0 DWT tile height (16, 32; 0 = off)
     int dwt_pipe = 0;            // fast level-0 DWT: persistent cp.async double-buffered variant
     // MQ schedule: tiers of warps with fewer blocks each for the longest blocks (lanes 0 ends)
