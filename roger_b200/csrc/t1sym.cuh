@@ -97,28 +97,38 @@ __device__ __forceinline__ SignSlices sign_slices(const Near& a, uint32_t own, u
 }
 
 // NW words per lane, LPS lanes per stripe, RT row masks of 8 * NW * LPS columns or more.
-template <int NW, int LPS, typename RT>
+// NARROW: a stripe is one word, which all its lanes hold; each writes the symbols of 32 / LPS samples.
+// Such blocks are small: what counts is not their symbols but what every plane and pass costs whatever
+// it holds, so the empty passes and exchanges are left out (at most 8 x 64 samples, whose symbols of a
+// pass fit the stage).
+template <int NW, int LPS, typename RT, bool NARROW = false>
 __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J, int jid, int lane,
                                                  const int32_t* __restrict__ coeff, uint8_t* __restrict__ syms,
                                                  uint32_t* __restrict__ nsyms, uint32_t* __restrict__ pass_end,
                                                  uint64_t* __restrict__ planes, j2k_cb_desc* __restrict__ descs,
                                                  uint32_t* __restrict__ err, int pad) {
     constexpr unsigned FULL = 0xffffffffu;
-    // kOne: the block is one word.  Every lane holds it, and writes the symbols of sample `lane`.
-    // kNarrow: one word per stripe.  Such blocks are small: what counts is not their symbols but what
-    // every plane and pass costs whatever it holds, so the empty passes and exchanges are left out (at
-    // most 8 x 64 samples, whose symbols of a pass fit the stage).
-    constexpr bool kOne = LPS == 32, kNarrow = kOne || LPS == 1;
-    static_assert(!kNarrow || NW == 1, "");
+    static_assert(!NARROW || NW == 1, "");
+    constexpr bool kOne = LPS == 32;  // one stripe
     const int cw = J.cw, ch = J.ch, orient = J.orient;
     const int32_t* blk = coeff + J.off;
-    const uint32_t me = 1u << lane, before_me = me - 1u;  // (kOne)
-    const int s0 = 4 * (lane / LPS), part = kOne ? 0 : lane % LPS;  // first row of the lane's stripe, place in it
+    constexpr int SEG = 32 / LPS;  // the lane's samples of a narrow word, and those before them
+    const uint32_t before_me = (1u << (SEG * (lane % LPS))) - 1u;
+    const uint32_t me = (SEG == 32 ? ~0u : (1u << (SEG & 31)) - 1u) << (SEG * (lane % LPS));
+    const int s0 = 4 * (lane / LPS), part = NARROW ? 0 : lane % LPS;  // first row of the lane's stripe, place in it
 
-    // ---- bit-plane slicing: lane p ends up holding plane p of each row and stores it
-    uint32_t mor = 0;
+    // ---- bit-plane slicing: lane p ends up holding plane p of each row and stores it (one word: lane i
+    // holds sample i, and a plane is one vote)
+    uint32_t mor = 0, mine_abs = 0;
+    bool mine_neg = false;
+    const bool mine_in = (lane & 3) < ch && lane >> 2 < cw;
+    if constexpr (kOne) {
+        const int32_t v = mine_in ? blk[(size_t)(lane & 3) * J.pitch + (lane >> 2)] : 0;
+        mine_neg = v < 0;
+        mor = mine_abs = v < 0 ? (uint32_t)(-(int64_t)v) : (uint32_t)v;
+    }
     constexpr int G = 4;  // rows whose loads are in flight together
-    for (int r0 = 0; r0 < ch; r0 += G) {
+    for (int r0 = 0; r0 < ch && !kOne; r0 += G) {
         int32_t a0[G], a1[G];
 #pragma unroll
         for (int g = 0; g < G; ++g) {
@@ -183,12 +193,12 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
         return lane >= 32 - LPS ? 0u : t;
     };
     auto before = [&](uint32_t x) {
-        if constexpr (kNarrow) return 0u;
+        if constexpr (NARROW) return 0u;
         const uint32_t t = __shfl_up_sync(FULL, x, 1);
         return part == 0 ? 0u : t;
     };
     auto after = [&](uint32_t x) {
-        if constexpr (kNarrow) return 0u;
+        if constexpr (NARROW) return 0u;
         const uint32_t t = __shfl_down_sync(FULL, x, 1);
         return part == LPS - 1 ? 0u : t;
     };
@@ -213,10 +223,15 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
     for (int j = 0; j < 4; ++j) {
         Vr[j] = s0 + j < ch ? colmask : (RT)0;
         O[j] = 0;
-        negrow[j] = s0 + j < ch ? (RT)planes[(s0 + j) * 32 + 31] : (RT)0;
+        negrow[j] = !kOne && s0 + j < ch ? (RT)planes[(s0 + j) * 32 + 31] : (RT)0;
     }
-    nibbles(Vr, V);
-    nibbles(negrow, neg);
+    if constexpr (kOne) {
+        V[0] = __ballot_sync(FULL, mine_in);
+        neg[0] = __ballot_sync(FULL, mine_neg);
+    } else {
+        nibbles(Vr, V);
+        nibbles(negrow, neg);
+    }
     {  // signs of the four direct neighbours
         const uint32_t pv = before(neg[NW - 1]), nx = after(neg[0]);
 #pragma unroll
@@ -270,7 +285,12 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
     // stage holds the bytes from the last 16-byte boundary of the output on.
     auto write_pass = [&](int cnt, auto emit) {
         int tot = cnt, off = 0;
-        if (!kOne) off = warp_excl(cnt, lane, &tot);
+        if (NARROW && !kOne) {  // every lane of a stripe has its count
+            off = warp_excl(lane % LPS == 0 ? cnt : 0, lane, &tot);
+            if (lane % LPS != 0) off -= cnt;
+        } else if (!kOne) {
+            off = warp_excl(cnt, lane, &tot);
+        }
         if (pos + tot > cap) {
             ovf = true;
             return;
@@ -279,11 +299,11 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
             const bool mine = off >= base && off + cnt <= base + kStage && cnt > 0;
             const int lead = pos & 15;
             if (mine) emit(lead + off - base);
-            const unsigned left = kNarrow ? 0u : __ballot_sync(FULL, cnt > 0 && off + cnt > base + kStage);
+            const unsigned left = NARROW ? 0u : __ballot_sync(FULL, cnt > 0 && off + cnt > base + kStage);
             const int next = left ? __shfl_sync(FULL, off, __ffs(left) - 1) : tot;
             __syncwarp();
             const int fill = lead + next - base, full = fill >> 4;
-            if (!kNarrow || full > 0) {
+            if (!NARROW || full > 0) {
                 uint4* dst = reinterpret_cast<uint4*>(out + (pos - lead));
                 for (int i = lane; i < full; i += 32) dst[i] = S.stage[i];
                 const uint4 rest = S.stage[full];
@@ -316,8 +336,9 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
         RT Br[4];
         uint32_t B[NW], K[NW], now[NW];  // this plane, samples the propagation pass codes, significance
 #pragma unroll
-        for (int j = 0; j < 4; ++j) Br[j] = s0 + j < ch ? (RT)planes[(s0 + j) * 32 + p] : (RT)0;
-        nibbles(Br, B);
+        for (int j = 0; j < 4; ++j) Br[j] = !kOne && s0 + j < ch ? (RT)planes[(s0 + j) * 32 + p] : (RT)0;
+        if constexpr (kOne) B[0] = __ballot_sync(FULL, (mine_abs >> p) & 1u);
+        else nibbles(Br, B);
 #pragma unroll
         for (int k = 0; k < NW; ++k) {
             K[k] = 0;
@@ -328,10 +349,20 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
             Near a[NW];
             int cnt = 0;
             if (!all) {
-                RT N[4] = {0, 0, 0, 0};
-                {
-                    RT up = 0, dw = 0;
-                    if (!kOne) up = __shfl_up_sync(FULL, O[3], LPS), dw = __shfl_down_sync(FULL, O[0], LPS);
+                uint32_t Nn[NW];
+                if constexpr (NARROW) {  // on the words themselves, a step a sample: they are short
+                    neighbours(sig, sig, a);
+                    const uint32_t M = V[0] & ~sig[0] & B[0];
+                    uint32_t N = M & a[0].any(), was;
+                    do {
+                        was = N;
+                        const uint32_t top = (above(N) >> 3) & 0x11111111u, un = ((N << 1) & 0xEEEEEEEEu) | top;
+                        N |= M & (un | (un << 4) | (top >> 4) | (N << 4) | ((N << 3) & 0x77777777u));
+                    } while (kOne ? N != was : __any_sync(FULL, N != was));
+                    Nn[0] = N;
+                } else {
+                    RT N[4] = {0, 0, 0, 0};
+                    RT up = __shfl_up_sync(FULL, O[3], LPS), dw = __shfl_down_sync(FULL, O[0], LPS);
                     if (lane < LPS) up = 0;
                     if (lane >= 32 - LPS) dw = 0;
                     RT E[4], M[4];
@@ -343,8 +374,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                     }
                     bool more;
                     do {
-                        RT ab = 0;
-                        if (!kOne) ab = __shfl_up_sync(FULL, N[3], LPS);
+                        RT ab = __shfl_up_sync(FULL, N[3], LPS);
                         if (lane < LPS) ab = 0;
                         RT was = 0;
 #pragma unroll
@@ -357,9 +387,8 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                         }
                         more = __any_sync(FULL, was != 0);
                     } while (more);
+                    nibbles(N, Nn);
                 }
-                uint32_t Nn[NW];
-                nibbles(N, Nn);
 #pragma unroll
                 for (int k = 0; k < NW; ++k) now[k] = sig[k] | Nn[k];
                 neighbours(sig, now, a);
@@ -373,7 +402,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                     for (int k = 0; k < NW; ++k) {
                         uint32_t L[4], m = K[k];
                         if (!m) continue;
-                        if (kOne) at += __popc(m & before_me) + __popc(m & B[k] & before_me), m &= me;
+                        if (NARROW) at += __popc(m & before_me) + __popc(m & B[k] & before_me), m &= me;
                         zc_slices(a[k], orient, L);
                         const SignSlices g = signs(a[k], k);
                         while (m) {
@@ -399,7 +428,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                 for (int k = 0; k < NW; ++k) {
                     const uint32_t nb = a[k].any();
                     uint32_t m = sig[k];
-                    if (kOne) at += __popc(m & before_me), m &= me;
+                    if (NARROW) at += __popc(m & before_me), m &= me;
                     while (m) {
                         const int i = __ffs((int)m) - 1;
                         m &= m - 1;
@@ -446,7 +475,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
                 for (int k = 0; k < NW; ++k) {
                     uint32_t L[4], m = ev[k];
                     if (!m) continue;
-                    if (kOne)
+                    if (NARROW)
                         at += __popc(m & before_me) + __popc(m & B[k] & before_me) + 2 * __popc(run[k] & B[k] & before_me),
                             m &= me;
                     zc_slices(a[k], orient, L);
@@ -475,7 +504,7 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
             }
 #pragma unroll
             for (int j = 0; j < 4; ++j) O[j] |= Br[j] & Vr[j];
-            if (kNarrow) all = !__any_sync(FULL, none != 0);
+            if (NARROW) all = !__any_sync(FULL, none != 0);
         }
         end_pass();
     }
@@ -499,19 +528,22 @@ __device__ __forceinline__ void symbols_of_block(SymSmem& S, const j2k_cb_job& J
 #define SYMBOLS(...) __VA_ARGS__(S, J, jid, lane, coeff, syms, nsyms, pass_end, planes, descs, err, pad)
 
 // a call of its own, so that the common forms' code is what it would be without this one
-template <int NW, int LPS, typename RT>
+template <int NW, int LPS, typename RT, bool NARROW = false>
 __device__ __noinline__ void symbols_of_rare_block(SYMBOLS_ARGS) {
-    SYMBOLS(symbols_of_block<NW, LPS, RT>);
+    SYMBOLS(symbols_of_block<NW, LPS, RT, NARROW>);
 }
 
-// The form that keeps most lanes busy: 32 / LPS stripes of 8 * NW * LPS columns, or for the narrow ones
-// one word per lane, or one in all lanes.  Bound by issue.  Whole encodes of 2048 x 2048 colour with
-// three forms only (wider than 32, narrower, at most 32 x 32) -> with these: blocks of 64 x 4 2.80 -> 1.24
-// ms, 64 x 8 1.84 -> 0.98, 8 x 8 2.92 -> 2.89, 4 x 4 6.62 -> 3.92; 32 x 32 and 64 x 64 as before.
+// The form that keeps most lanes busy: 32 / LPS stripes of 8 * NW * LPS columns, or for narrow blocks of
+// one word each.  Bound by issue.  Whole encodes of 2048 x 2048 colour with three forms only (wider than
+// 32, narrower, at most 32 x 32) -> with these: blocks of 64 x 4 2.80 -> 1.24 ms, 64 x 8 1.84 -> 0.98, 8 x 8
+// 2.92 -> 1.77, 4 x 4 6.62 -> 2.88; 32 x 32 and 64 x 64 as before.
 __device__ __forceinline__ void symbols_of_shape(SYMBOLS_ARGS) {
     const int w = J.cw, h = J.ch;
-    if (w <= 8 && h <= 4) SYMBOLS(symbols_of_rare_block<1, 32, uint32_t>);
-    else if (w <= 8) SYMBOLS(symbols_of_rare_block<1, 1, uint32_t>);
+    if (w <= 8 && h <= 4) SYMBOLS(symbols_of_rare_block<1, 32, uint32_t, true>);
+    else if (w <= 8 && h <= 8) SYMBOLS(symbols_of_rare_block<1, 16, uint32_t, true>);
+    else if (w <= 8 && h <= 16) SYMBOLS(symbols_of_rare_block<1, 8, uint32_t, true>);
+    else if (w <= 8 && h <= 32) SYMBOLS(symbols_of_rare_block<1, 4, uint32_t, true>);
+    else if (w <= 8) SYMBOLS(symbols_of_rare_block<1, 2, uint32_t, true>);
     else if (w <= 32 && h <= 32) SYMBOLS(symbols_of_block<1, 4, uint32_t>);
     else if (w <= 32) SYMBOLS(symbols_of_block<2, 2, uint32_t>);
     else if (h <= 16) SYMBOLS(symbols_of_rare_block<1, 8, uint64_t>);

@@ -41,7 +41,7 @@ def _block(w, h, orient):
 @pytest.mark.parametrize("pad", [0, 1])
 def test_symbols_equal_the_oracle_without_a_race(exe, pad):
     # both sides of the forms' limits, ragged stripes, a block of one sample
-    blocks = [(w, h, o) for w, h in [(1, 1), (4, 4), (8, 3), (5, 7), (32, 32), (31, 9), (9, 33), (33, 6), (40, 13)] for o in range(4)]
+    blocks = [(w, h, o) for w, h in [(1, 1), (4, 4), (8, 3), (5, 7), (8, 16), (3, 31), (8, 61), (32, 32), (31, 9), (9, 33), (33, 6), (40, 13)] for o in range(4)]
     blocks += [(32, 64, 1), (64, 64, 3), (8, 64, 2), (9, 4, 1), (64, 16, 2), (33, 17, 1), (64, 32, 0), (40, 33, 1)]
     data = b"".join(struct.pack("<4i", w, h, o, pad) + _block(w, h, o).tobytes() for w, h, o in blocks)
     r = subprocess.run([exe], input=data, capture_output=True, env=dict(os.environ, TSAN_OPTIONS="exitcode=66"),
