@@ -376,6 +376,17 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
             iblk[r] = coeff + __shfl_sync(~0u, (unsigned long long)J.off, b);
             if (i >= Q * L) inp[r] = 0;
         }
+        // With one word a stripe and up to 4 blocks a lane per column prepares it (with 8, two columns a
+        // lane, that is no faster): the columns of block lane / 8
+        constexpr bool COLS = Q == 1 && L <= 4;
+        int xcw = 0, xch = 0, xnp = 0, xnb = 0;
+        if constexpr (COLS) {
+            xcw = __shfl_sync(~0u, (int)J.cw, lane >> 3);
+            xch = __shfl_sync(~0u, (int)J.ch, lane >> 3);
+            xnp = __shfl_sync(~0u, np, lane >> 3);
+            xnb = __shfl_sync(~0u, (int)D.numbps, lane >> 3);
+            if (lane >= 8 * L) xnp = 0;
+        }
         const int pmax = __reduce_max_sync(~0u, np > 0 ? (int)D.numbps : 0);
         const int smax = (__reduce_max_sync(~0u, np > 0 ? (int)J.ch : 0) + 3) >> 2;
         const int st = STYLED ? (job_style ? (int)job_style[jid] : style) : 0;
@@ -394,18 +405,34 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
             bool ion[R];
 #pragma unroll
             for (int r = 0; r < R; ++r) ion[r] = pass_of(inb[r]) >= 0 && pass_of(inb[r]) < inp[r];
+            const bool xon = pass_of(xnb) >= 0 && pass_of(xnb) < xnp;
             for (int s = 0; s < smax; ++s) {
+                if (COLS && kind != kPassMR) {
+                    const int b = lane >> 3, x = lane & 7;
+                    const bool mine = xon && 4 * s < xch;
+                    bool has = false;
+                    if constexpr (COLS)
+                        has = mine && x < xcw && stripe_prepare_column(S, kind, s, x, b, stripe_rows(xch, s));
+                    const unsigned set = __ballot_sync(~0u, has);
+                    if (mine && x == 0) {
+                        S.cols(b)[0] = (uint8_t)(set >> (lane & 24));
+                        if (kind == kPassSP) S.vis(s, 0, b) = 0;  // (a stripe without symbols is not finished)
+                    }
+                }
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const int i = lane + 32 * r;
-                    if (ion[r] && 4 * s < ich[r]) {
+                    if (ion[r] && 4 * s < ich[r] && (!COLS || kind == kPassMR)) {
                         if (kind == kPassMR) stripe_prepare_mr(S, s, i % Q, i / Q, icw[r]);
                         else stripe_prepare_zc(S, kind, s, i % Q, i / Q, icw[r], stripe_rows(ich[r], s));
                     }
                 }
                 __syncwarp();
                 // (with one word a stripe, preparing and finishing it costs as much as its symbols)
-                if (Q == 1 && !__any_sync(~0u, on && 4 * s < me.ch && S.colset(0, lane) != 0)) continue;
+                if (Q == 1 && !__any_sync(~0u, on && 4 * s < me.ch && S.colset(0, lane) != 0)) {
+                    __syncwarp();
+                    continue;
+                }
                 if (on && 4 * s < me.ch) {
                     const uint32_t rv = stripe_rows(me.ch, s);
                     if (kind == kPassSP) me.template decode_zc<STYLED, kPassSP>(rv);

@@ -148,6 +148,30 @@ T1D_HD void stripe_prepare_zc(const StripeState<L, Q>& S, int kind, int s, int q
     if (Q == 1 && kind == kPassSP) S.vis(s, q, b) = 0;  // a stripe without symbols is not finished
 }
 
+// The same for one column of a stripe of one word, so that a block's columns can be prepared by as many
+// lanes; returns whether the column has a symbol (the caller puts the set together).
+template <int L>
+T1D_HD bool stripe_prepare_column(const StripeState<L, 1>& S, int kind, int s, int x, int b, uint32_t rv) {
+    const uint32_t sg = S.sig(s, 0, b), ng = S.neg(s, 0, b);
+    const uint32_t sa = s > 0 ? S.sig(s - 1, 0, b) : 0u, na = s > 0 ? S.neg(s - 1, 0, b) : 0u;
+    const uint32_t se = s < 15 ? S.sig(s + 1, 0, b) : 0u, ne = s < 15 ? S.neg(s + 1, 0, b) : 0u;
+    uint32_t own_ng = ng;
+    if (kind == kPassCU) own_ng |= S.vis(s, 0, b) & ~sg;
+    // columns x - 1, x, x + 1 of a word at bits 0, 4, 8
+    const auto three = [&](uint32_t w) { return x ? (w >> (4 * x - 4)) & 0xFFFu : (w << 4) & 0xFFFu; };
+    const uint32_t m = three(sg), a = three(sa), e = three(se), n = three(ng);
+    uint32_t W = 0;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        W |= ((spread4((m >> (4 * i)) & 15u) << 3) | ((a >> (4 * i + 3)) & 1u) | (((e >> (4 * i)) & 1u) << 15)) << i;
+    const int sh = 4 * x;
+    const uint32_t vert = ((na >> (sh + 3)) & 1u) | (((own_ng >> sh) & 15u) << 1) | (((ne >> sh) & 1u) << 5);
+    W |= ((n & 15u) << 18) | (vert << 22) | ((n >> 8) << 28);
+    S.col(x, b) = W;
+    const uint32_t c = ~(W >> 4) & rv;
+    return (kind == kPassSP ? c & near_rows(W) : c & ~spread4((W >> 23) & 15u)) != 0;
+}
+
 // samples of word q that the refinement pass codes (significant before this plane), and the number
 // of those in the words before it: within a word the bits are in coding order already
 template <int L, int Q>
