@@ -65,7 +65,8 @@ enum {
     J2K_TUNE_MQ_VARIANT = 2, /* 0 or 1: kept for callers that set it; there is one form, a pair of an
                                 interval warp and a code warp */
     J2K_TUNE_DWT_FAST_TH = 3, /* register-lifting forward DWT tile height: 16 (default), 32, 0 = off */
-    J2K_TUNE_DWT_PIPE = 4,    /* 1: that kernel streams bands with cp.async double buffering (default 0) */
+    J2K_TUNE_DWT_PIPE = 4,    /* 1: that kernel streams bands with cp.async double buffering, for single
+                                 planes (default 0) */
     J2K_TUNE_DWT_REG = 5,     /* 1 (default): that kernel loads its columns straight into registers;
                                  0: it stages the strip in shared memory with cp.async */
     J2K_TUNE_DWT_TMA = 7,     /* 1: that kernel is the TMA-staged form (persistent CTAs, each strip brought in

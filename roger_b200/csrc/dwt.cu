@@ -203,19 +203,22 @@ dwt_fwd_batched(const j2k_dwt_level_desc* __restrict__ descs, const uint32_t* __
 }
 
 // ---- fast forward level (T.800 order) ------------------------------------------------------------
-// One CTA produces a 248 x 32 tile of level outputs from a 256-column x (32 + 2*HV)-row strip:
-//   * rows are loaded with 16-byte vectors (mirrored scalar loads only where the strip leaves
-//     the image), columns x0-4 .. x0+251;
+// One CTA produces a 248 x FTH tile of level outputs (16 rows by default, or 32) from a 256-column x
+// (FTH + 2*HV)-row strip:
+//   * each thread loads its column of the strip, columns x0-4 .. x0+251, into registers by single
+//     samples (mirrored where the strip leaves the image), so that any pitch will do;
 //   * the vertical lifting runs in registers, one thread per column, the whole column unrolled;
 //   * the horizontal lifting runs in registers, 8 samples per lane, neighbours exchanged with
 //     warp shuffles (the 4-column halo absorbs the missing neighbours at the warp ends);
 //   * the subbands' rows are put in order in shared memory and written by consecutive samples
 //     (8-byte vectors when aligned).
+// Other forms of the loads (cp.async, tensor copies) stage the strip in shared memory first.
 // Same arithmetic, operation order and rounding as dwt_fwd_level, so the outputs are identical.
 
 // Step 3 of the fast forward level: horizontal lifting of the FTH vertically lifted rows held in
 // shared memory (strip row r at s[r - RO]), 8 samples per lane (tile columns 8*lane ..
-// 8*lane+7), and the writes of the four subbands (dead-zone indices when QUANT).  Shared by the register-load and the TMA-staged forms of the level kernel.
+// 8*lane+7), and the writes of the four subbands (dead-zone indices when QUANT).  Shared by the
+// register-load and the TMA-staged forms of the level kernel.
 template <int KERN, typename TD, bool QUANT, bool QLL, int FTH, int RO>
 __device__ __forceinline__ void fwd_fast_rows(typename KT<KERN>::T (*s)[FNX], int x0, int y0, int w, int h,
                                               typename KT<KERN>::T* __restrict__ ll_dst, size_t llpitch,
@@ -436,8 +439,8 @@ dwt_fwd_fast(const typename KT<KERN>::T* __restrict__ src, size_t spitch, int w,
 // stored: per pixel the level reads NC bytes where the planar split wrote, and the level read
 // back, 4 NC bytes.  Component c writes dst + c * dst_z and ll_dst + c * ll_z.
 // It is an encoder option (J2K_TUNE_DWT_PX), off by default: the plane kernel is issue-bound
-// already, and this one moves a third of the bytes in 2.4x the instructions (176 us for the
-// 4096x4096 RGB level 0, against 45 + 85 us for the planar split and the level over the planes).
+// already, and this one moves a third of the bytes in 2.4x the instructions (174 us for the
+// 4096x4096 RGB level 0, against 46 + 78 us for the planar split and the level over the planes).
 // Words are read only where they hold a byte of the row's strip; such an aligned word never
 // leaves the page of that byte.
 template <int KERN, int NC, int MCT, typename TD, bool QUANT, bool QLL>
@@ -1281,7 +1284,7 @@ j2k_status fwd_levels(j2k_ctx* ctx, const void* in, size_t in_pitch, void* out, 
         // The forms that copy 16-byte chunks (cp.async, TMA) need every row and image of the batch
         // 16-byte aligned; the default form loads single samples and takes any pitch.  An odd width
         // makes every plane's pitch odd: the 9/7 transform and inverse of three 2047 x 3001 planes took
-        // 286 us with level 0 in the tile kernel (146 us) and take 192 us this way.
+        // 286 us with level 0 in the tile kernel (146 us) and take 167 us this way.
         const bool aligned = ((uintptr_t)src & 15) == 0 && (spitch & 3) == 0 && (n == 1 || (src_z & 3) == 0);
         const bool loads_samples = !ctx || (ctx->dwt_reg && !ctx->dwt_pipe && !ctx->dwt_tma);
         // A grid has at most 65535 rows of tiles: a level of more takes the tile kernel, whose tiles

@@ -478,7 +478,7 @@ t1_decode_stripe_kernel(const j2k_cb_desc* __restrict__ descs, const uint8_t* __
 }
 
 constexpr size_t kTablesBytes = (sizeof(DecTables) + 15) & ~(size_t)15;
-// warps per CTA of the lane-per-block decoders for L blocks per warp: 32 blocks per CTA for
+// warps per CTA of the one-symbol-per-step decoder for L blocks per warp: 32 blocks per CTA for
 // L >= 8, four warps for smaller L (so that a CTA's shared-memory state stays near 70 KB or less)
 template <int L>
 __host__ __device__ constexpr int cta_warps() {

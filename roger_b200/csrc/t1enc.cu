@@ -1,4 +1,5 @@
-// EBCOT tier-1 encoder: context modelling (warp per code-block) + MQ coding (lane per block).
+// EBCOT tier-1 encoder: context modelling (a warp per code-block) + MQ coding (a warp pair for 1 to 32
+// code-blocks).
 //
 // Reference: src/CL/oclbpc.cl:279-746 via src/OCLBPC.cpp:38-50.  The reference kernel computes
 // the MSB plane and sigma/neighbourhood state only (its coding actions are empty comments,
@@ -10,8 +11,9 @@
 // coder (t1sym.cuh), one byte per symbol: label in bits 0-4, decision in bit 7; sign symbols also
 // carry their context's XOR bit in bit 5, so that a raw-coded pass can recover the sign itself.
 //
-// Phase B — one lane per code-block runs the MQ encoder over its symbol stream (T.800 C.2, FLUSH of
-// C.2.9, trailing 0xFF dropped; mq_enc.cuh); codeword bytes are written as aligned 32-bit words.
+// Phase B — the MQ encoder over the symbol streams (T.800 C.2, FLUSH of C.2.9, trailing 0xFF dropped;
+// mq_enc.cuh), a block on one lane of each of two warps: the interval chain and the byte output.
+// Codeword bytes are written as aligned 32-bit words.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -38,8 +40,9 @@ __device__ __forceinline__ int warp_excl(int v, int lane, int* tot) {
 
 #include "t1sym.cuh"
 
-// MINB: resident CTAs per SM the register budget is cut for (2: no spills; 3: a few spilled
-// registers, more warps to hide the ALU chains)
+// MINB: resident CTAs per SM the register budget is cut for (2: 128 registers, no spills; 3: 80, with
+// 220 bytes of spill stores and 504 of loads in all forms together, and more warps to hide the ALU
+// chains: 256 images of mixed sizes take 3.70 ms with either)
 template <int MINB>
 __global__ void __launch_bounds__(kWarpsPerCta * 32, MINB)
 t1_symbols_kernel(const int32_t* __restrict__ coeff, const j2k_cb_job* __restrict__ jobs,
@@ -71,11 +74,11 @@ t1_symbols_kernel(const int32_t* __restrict__ coeff, const j2k_cb_job* __restric
     }  // queue loop
 }
 
-// ---- phase B: MQ encoder, one lane per code-block ------------------------------------------------
+// ---- phase B: MQ encoder ---------------------------------------------------------------------------
 //
 // The coder is serial per block, so the kernel time is (longest block's symbol count) x (time per
-// symbol).  Blocks are ordered longest-first (a radix sort of the symbol counts) so the lanes of a
-// warp finish together and the biggest blocks start first.
+// symbol).  Blocks are ordered longest-first (a radix sort of the symbol counts) so that the blocks of
+// a warp pair end together and the biggest ones start first.
 
 __constant__ uint16_t c_qe[47] = {
     0x5601, 0x3401, 0x1801, 0x0AC1, 0x0521, 0x0221, 0x5601, 0x5401, 0x4801, 0x3801, 0x3001, 0x2401,
@@ -91,7 +94,8 @@ __constant__ uint8_t c_nlps[47] = {1,  6,  9,  12, 29, 33, 6,  14, 14, 14, 17, 1
 
 #include "mq_enc.cuh"
 
-constexpr int kMqThreads = 32;  // one warp per CTA: the longest blocks' warps spread one per SM
+constexpr int kMqThreads = 32;  // blocks of a warp pair at most; one pair (64 threads) is a CTA, so that the
+                                // longest blocks' pairs spread one per SM
 
 constexpr int kMqCopies = 8;
 constexpr int kMqTable = 94 * kMqCopies;
@@ -840,9 +844,10 @@ j2k_status j2k_t1_encode_jobs(j2k_ctx* ctx, const int32_t* coeff, const j2k_cb_j
         warps += wk;
     }
     // blocks per pair after the tiers: one more pair per SM holds the rest (a scheduler for each of
-    // the warps of two pairs per SM), up to full warps.  Whole encodes on B200 after a tier of one
-    // block per SM: 777 blocks with 2 a pair 1.84, with 16 or 32 1.57 ms; 3072 blocks with 10 2.03,
-    // with 32 1.82; 12288 blocks with 16 4.1, with 32 2.94
+    // the warps of two pairs per SM), up to full warps.  Whole lossless encodes of colour images on
+    // B200 after a tier of one block per SM, by this rule / with 8 / 16 / 32 a pair: 777 blocks (5 a
+    // pair) 1.51 ms with any of them; 1749 (11) 1.56 / 1.78 / 1.56 / 1.58; 3072 (20) 1.69 / 1.95 /
+    // 1.94 / 1.73; 5511 (32) 2.17 / 2.88 / 2.23 / 2.17; 12288 (32) 2.77 / 5.18 / 3.94 / 2.78
     const size_t per = (size_t)ctx->sm_count;
     const int lanes = ctx->mq_lanes ? ctx->mq_lanes : (int)std::min<size_t>(std::max<size_t>((left + per - 1) / per, 1), 32);
     warps += (left + lanes - 1) / lanes;

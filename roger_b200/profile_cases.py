@@ -16,24 +16,24 @@ benchmark workloads but stay within a few hundred MB of device memory:
   idwt53       level-0 5/3 inverse of the same plane
   tier1        EBCOT tier-1 of one 4096x4096 RCT component (6 levels, 4096 64x64 blocks)
   encode       one whole lossless 4096x4096 RGB encode (planar, 3 x 6 DWT levels, tier-1)
-  diff-kernels one level-0 launch of every kernel of the differentiable 9/7 step on
+  diff-kernels one level-0 launch of every strip kernel of the differentiable 9/7 step on
                16 x 1024x1024 float32 (forward, quantiser, inverse+residual, inverse adjoint,
-               quantiser backward, forward adjoint+residual)
+               quantiser backward, forward adjoint+residual); levels that are not a power of two wide
+               run them (J2K_TUNE_DWT97_ROWS 0 here)
   diff-step    one fused rate-distortion step (5 levels, forward + backward)
-  batched      the 256-image mixed set (config 4) through the batched encoder: the first run
+  batched      the 256-image mixed set through the batched encoder: the first run
                captures its launch sequence in a CUDA graph, the second replays it
   decode       lossless decode of one 2048x2048 RGB image (tier-1 decode, inverse 5/3, inverse
                RCT) from code-blocks already on the host
   decode-steps / decode-lanes / decode-warp  the same with the tier-1 decoder forced to one
-               symbol per step with 32 blocks per warp, to the pass / stripe / column loops with
-               8 blocks per warp, or to one warp per block
+               symbol per step with 32 blocks per warp, or to stripes with 8 blocks per warp or one
   decode-4096  the decode case on the 4096x4096 RGB image (12288 code-blocks), default decoder
   rate         one lossless 4096x4096 RGB encode cut to 1 bit per pixel by PCRD-opt (tier-1
                rate path, distortion pass, host PCRD and header sizing, descriptor update)
   dwt53-tma    as dwt53, with the TMA-staged level kernel (tuning key J2K_TUNE_DWT_TMA)
   dwt53-all-tma  as dwt53-all, with the TMA-staged level kernel
   encode-styled  the lossless 4096x4096 RGB encode with code-block style RESET | TERMALL (every
-               pass of a block coded in its own lane)
+               pass of a block coded by a lane of its own)
 """
 import math
 import sys
@@ -106,6 +106,7 @@ def case_encode():
 
 def case_diff_kernels():
     from . import diff97 as D
+    lib().j2k_ctx_set_tuning(C.default_context(0).h, 13, 0)
     x = torch.from_numpy(synth.float_batch(16, 1024, 1024, 200)).cuda()
     L = 1
     ls = torch.full((3 * L + 1,), math.log(1 / 64.0), device="cuda")
@@ -167,7 +168,8 @@ CASES = {"planar": case_planar, "dwt53": case_dwt53, "dwt53-all": lambda: case_d
          "diff-kernels": case_diff_kernels, "diff-step": case_diff_step, "batched": case_batched,
          "decode": case_decode,
          "decode-steps": lambda: case_decode(32, 1), "decode-lanes": lambda: case_decode(8, 0),
-         "decode-warp": lambda: case_decode(0, 0), "decode-4096": lambda: case_decode(size=4096), "rate": case_rate, "dwt53-tma": case_dwt53_tma,
+         "decode-warp": lambda: case_decode(0, 0), "decode-4096": lambda: case_decode(size=4096), "rate": case_rate,
+         "dwt53-tma": case_dwt53_tma,
          "dwt53-all-tma": lambda: case_dwt53_tma(6), "encode-styled": case_encode_styled}
 
 
