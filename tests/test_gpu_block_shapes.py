@@ -47,7 +47,8 @@ def picture():
     return torch.from_numpy(synth.rgb(1024, 1024, (1, 2, 3, 4))).cuda()
 
 
-# with one lane of a warp in 16 or 32 at work: 1.8 and 2.1; with the forms by shape 1.0 and 1.3
+# with one lane of a warp in 16 or 32 at work: 1.8 and 2.1; with the forms by shape 1.0 and 1.3 (and 8 x 8
+# blocks, since then faster themselves, 1.5)
 @pytest.mark.parametrize("shape,other,most", [((64, 4), (16, 16), 1.4), ((4, 4), (8, 8), 1.7)])
 def test_no_shape_encodes_much_slower(picture, shape, other, most):
     enc = C.OCLEncoder(ctx=C.Context(0))
